@@ -8,16 +8,16 @@
 // 95-148, fragment_shader 471-506, mix_vertex 509-522), scaled and converted to AP1
 // (color.cl:3-10) and written y-flipped.
 //
-// GB300 organisation (k_raster): one CTA per T x T tile, threads own pixels (T = 32: 256
-// threads x 4 pixels). The tile's list from rf_bin_tiles holds (primitive, wavelength pair)
-// entries in increasing order. Entries are expanded in batches into shared-memory records
-// (one per sub-wavelength step): the mixed integer vertices, the five edge functions as
-// wrapping-int32 plane coefficients with the top-left bias folded in, the integer bounds
-// and the mixed attributes, set up once by one thread each. Every pixel then walks the
+// GB300 organisation (k_raster): one CTA per T x T tile; warps take the tile's blocks of pixels.
+// The tile's list from rf_bin_tiles holds (primitive, wavelength pair) entries in increasing
+// order. Entries are expanded in batches into shared-memory records (one per sub-wavelength
+// step): the mixed corners, the five edge functions as exact FP32 plane coefficients relative to
+// the tile, the integer bounds and the mixed attributes, set up once. Every pixel then walks the
 // records in order, so its sum runs in the reference's order; a pixel whose samples lie
 // outside a record's integer bounds skips it (exact: with vertex and sample coordinates
 // below 2^14 the edge functions cannot wrap, and the quad test then never accepts a
-// sample outside the bounds; records beyond that range are tested at every pixel).
+// sample outside the bounds; records beyond that range are tested at every pixel, in wrapping
+// int32).
 //
 // k_raster_masks is the literal per-pixel loop over the reference's bin masks, used for
 // parity checks of the binner and the rasteriser.
@@ -36,13 +36,12 @@ int tile_size_of(const rf_raster_args& a);
 namespace {
 
 // Tuning knobs (compile-time): records per shared-memory batch, resident blocks per SM
-// requested from the register allocator, and where the half-angle tangents use the
-// reference's exact FP32 operations (1: small angles, 0: only a_i == 0).
+// requested from the register allocator.
 #ifndef RF_RASTER_BATCH
 #define RF_RASTER_BATCH 64
 #endif
 #ifndef RF_RASTER_MIN_BLOCKS
-#define RF_RASTER_MIN_BLOCKS 3
+#define RF_RASTER_MIN_BLOCKS 4
 #endif
 #ifndef RF_RASTER_MIN_BLOCKS_S1  // the one-sample kernel needs fewer registers
 #define RF_RASTER_MIN_BLOCKS_S1 4
@@ -50,14 +49,20 @@ namespace {
 #ifndef RF_RASTER_CLASSIFY
 #define RF_RASTER_CLASSIFY 1
 #endif
-#ifndef RF_RASTER_EXACT_SMALL_ANGLES
-#define RF_RASTER_EXACT_SMALL_ANGLES 0
-#endif
 constexpr int kBatchRecords = RF_RASTER_BATCH;
+// Pixels of a column a lane of the one-sample kernels shades: two where a tile has enough blocks
+// of 8 x 8 pixels for the CTA's 8 warps (32-pixel tiles: 16; production frame 102.0 ms with one
+// pixel, 90.4 with two), one in 16-pixel tiles.
+#ifndef RF_RASTER_PIX32
+#define RF_RASTER_PIX32 2
+#endif
+#ifndef RF_RASTER_PIX16
+#define RF_RASTER_PIX16 1
+#endif
 
 #ifdef RF_RASTER_STATS
 // Work counters of the statistics build (never compiled into the product library):
-// record iterations per 8 x 4 block, those of whole-block records, fragments, fragments of
+// record iterations per block, those of whole-block records, fragments, fragments of
 // whole-block records, block visits, fragments whose smoothstep factor is 0 (rrel >= 1),
 // record iterations where that holds for every shaded pixel of the block (those two with
 // more than one sample per pixel), warp steps of the one-sample shading loop.
@@ -116,22 +121,30 @@ struct alignas(16) Rec {
     int bb[4];       // xmin, xmax, ymin, ymax
     float col[4];    // the record's XYZ weight (1, 1, 1 with one wavelength); [3]: 0 when the housing
                      // falloff is 1 and no clamp acts on any covered pixel (inside_housing), else 1
-    float xy[12];    // corner positions, exact floats: x0 x2, x1 x3, y0 y2, y1 y3, x2 x0, y2 y0
+    float xy[8];     // corner positions relative to the tile, exact floats: x0 x2, x1 x3, y0 y2, y1 y3
     float uv[8];     // ghost texel coordinates: u0 u2, u1 u3, v0 v2, v1 v3, see store_corner
     float rs[4];     // (rrel - 1) / (0.95 - 1): smoothstep(1, 0.95, rrel)'s ramp before clamping
     float inten[4], refl[4];
-    // edge functions A * y + B * x + C in samples relative to the tile (exact, see finish_record):
-    // A of edges 01 12, B 01 12, C 01 12, A 23 30, B 23 30, C 23 30, then A B C of edge 20
-    float ef[15];
-    int flags;       // 1: bounds rejection and ef are exact; 2: adds nothing (collinear, or zero_record)
-    float ext[4];    // edges 01 12 23 30: half the edge function's range over an 8 x 4 pixel block
-    int q[8];        // mixed vertex positions, sample space (x0, y0, ..., x3, y3)
+    // edge functions A y + B x + C in samples relative to the tile (exact, see finish_record):
+    float ab[8];     // A of edges 01 23, B 01 23, A 12 30, B 12 30
+    float c[4];      // C of edges 01 23 12 30
+    float cb[4];     // C with the top-left bias
+    float e20[3];    // A, B, biased C of edge 20
+    int flags;       // 1: bounds rejection and ab, cb, e20 are exact; 2: adds nothing (collinear, or zero_record)
+    float nl2[4];    // minus the squared lengths of edges 01 23 12 30; NaN: the weights take special_weights
+    float ext[4];    // edges 01 23 12 30: half the edge function's range over a block
+    float pad[4];    // the stride
+    // mixed vertex positions, sample space (x0, y0, ..., x3, y3): in ab's place while the record is
+    // built, and for good where the edge functions are not exact (flags & 1 clear)
+    __device__ __forceinline__ int* q() { return reinterpret_cast<int*>(ab); }
+    __device__ __forceinline__ const int* q() const { return reinterpret_cast<const int*>(ab); }
 };
 static_assert(sizeof(Rec) == 272 && offsetof(Rec, bb) == 0 && offsetof(Rec, col) % 16 == 0 &&
                   offsetof(Rec, xy) % 16 == 0 && offsetof(Rec, uv) % 16 == 0 && offsetof(Rec, rs) % 16 == 0 &&
-                  offsetof(Rec, inten) % 16 == 0 && offsetof(Rec, refl) % 16 == 0 &&
-                  offsetof(Rec, ef) % 16 == 0 && offsetof(Rec, flags) == offsetof(Rec, ef) + 15 * sizeof(int) &&
-                  offsetof(Rec, ext) % 16 == 0 && offsetof(Rec, q) % 16 == 0,
+                  offsetof(Rec, inten) % 16 == 0 && offsetof(Rec, refl) % 16 == 0 && offsetof(Rec, ab) % 16 == 0 &&
+                  offsetof(Rec, c) % 16 == 0 && offsetof(Rec, cb) % 16 == 0 && offsetof(Rec, e20) % 16 == 0 &&
+                  offsetof(Rec, flags) == offsetof(Rec, e20) + 12 && offsetof(Rec, nl2) % 16 == 0 &&
+                  offsetof(Rec, ext) % 16 == 0,
               "records are read with 16-byte loads");
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ int4 ld4i(const int* p) { return *reinterpret_cast<const int4*>(p); }
@@ -193,29 +206,28 @@ __device__ __forceinline__ unsigned outside_sign(unsigned n01, unsigned n12, uns
     return (~n20 & x1) | (n20 & x0);
 }
 
-// A record's edge functions in registers.
+// A record's biased edge functions in registers.
 struct Edges {
-    f2 a0, b0, c0, a1, b1, c1;  // edges (01, 12) and (23, 30)
+    f2 a0, b0, c0, a1, b1, c1;  // edges (01, 23) and (12, 30)
     float a20, b20, c20;
-    int flags;
 };
 __device__ __forceinline__ void load_edges(const Rec& r, Edges& e) {
-    ld2(r.ef, e.a0, e.b0);
-    ld2(r.ef + 4, e.c0, e.a1);
-    ld2(r.ef + 8, e.b1, e.c1);
-    const float4 d = ld4(r.ef + 12);
-    e.a20 = d.x, e.b20 = d.y, e.c20 = d.z, e.flags = __float_as_int(d.w);
+    ld2(r.ab, e.a0, e.b0);
+    ld2(r.ab + 4, e.a1, e.b1);
+    ld2(r.cb, e.c0, e.c1);
+    const float4 d = ld4(r.e20);
+    e.a20 = d.x, e.b20 = d.y, e.c20 = d.z;
 }
 // The sample at tile-relative coordinates x = (x, x), y = (y, y), for records with flags & 1: the
 // edge values are exact integers (an exact zero is +0), so their signs are the reference's.
 __device__ __forceinline__ bool inside(const Edges& e, f2 x, f2 y) {
     const f2 e0 = fma2(e.a0, y, fma2(e.b0, x, e.c0)), e1 = fma2(e.a1, y, fma2(e.b1, x, e.c1));
     const float e2 = fmaf(e.a20, lo2(y), fmaf(e.b20, lo2(x), e.c20));
-    return (int)outside_sign((unsigned)e0, (unsigned)(e0 >> 32), (unsigned)e1, (unsigned)(e1 >> 32),
+    return (int)outside_sign((unsigned)e0, (unsigned)e1, (unsigned)(e0 >> 32), (unsigned)(e1 >> 32),
                              __float_as_uint(e2)) >= 0;
 }
 
-// Coverage of an 8 x 4 pixel block's samples (centre (xc, yc) as pairs, tile-relative, half extents
+// Coverage of a block's samples (centre (xc, yc) as pairs, tile-relative, half extents
 // hx, hy) by a record with flags & 1: each edge value is linear in the sample, so its sign is
 // constant over the block when its extremes there (centre value -+ ext) agree, and then
 // inside() is constant too. Returns 0 (no sample inside), 2 (every sample inside) or 1 (mixed
@@ -234,84 +246,118 @@ __device__ __forceinline__ int rect_coverage(const Rec& r, f2 xc, f2 yc, float h
     const unsigned mixed = ((unsigned)l0 & ~(unsigned)h0) | ((unsigned)(l0 >> 32) & ~(unsigned)(h0 >> 32)) |
                            ((unsigned)l1 & ~(unsigned)h1) | ((unsigned)(l1 >> 32) & ~(unsigned)(h1 >> 32)) |
                            (l2 & ~h2);
-    const unsigned out = outside_sign((unsigned)l0, (unsigned)(l0 >> 32), (unsigned)l1, (unsigned)(l1 >> 32), l2);
+    const unsigned out = outside_sign((unsigned)l0, (unsigned)l1, (unsigned)(l0 >> 32), (unsigned)(l1 >> 32), l2);
     return (int)mixed < 0 ? 1 : ((int)out < 0 ? 0 : 2);
 }
 
-// Mean-value weights (compute_barycentric_quad, rasterizing.cl:95-148) at the integer
-// sample point (px, py). The coordinates s_i = q_i - p are exact floats; the products
-// a_i, d_i, |s_i|^2 are exact integers wherever |s| < 4096, so fused multiply-adds give
-// the reference's values there. Where a_i is 0 the reference divides the rounding residue
-// of r_i r_j - d_i by 1e-3: that tangent is evaluated with the reference's exact FP32
-// operations (correctly rounded square roots, product, difference, quotient). Elsewhere
-// the tangents and the divisions by r_i and by the weight sum use reciprocal and
-// reciprocal-square-root instructions (a few ulps).
+// Mean-value weights (compute_barycentric_quad, rasterizing.cl:95-148) at a sample point p. With
+// s_i = q_i - p, r_i = |s_i|, a_i = s_i x s_j, d_i = s_i . s_j (j the next corner), the reference's
+// weight is (t_{i-1} + t_i) / r_i, t_i = (r_i r_j - d_i) / a_i, normalised by the weights' sum.
+// Two identities save the products: a_i is minus edge ij's function at p, which is exact here
+// (integers below 2^24; records where it is not take special_weights), and
+// r_i r_j - d_i = (L^2 - (r_i - r_j)^2) / 2 with the edge's length L, which also loses fewer digits
+// than the difference of two products of the size of r^2. The common factors (-1, 2) cancel in
+// the normalisation. Reciprocals and reciprocal square roots are the approximate instructions (a
+// few ulps).
 //
-// px, py are (x, x) and (y, y). Corners 0 and 2 and corners 1 and 3 go through packed
-// operations; the cross products' second terms are formed from negated odd corners
-// (p - q instead of q - p), because a packed fused multiply-add cannot negate an operand.
-// Returns the weights of corners (0, 2) in we and (1, 3) in wo; sets `general` to 1 where they may
-// have mixed signs inside a convex quad (the rare path).
-__device__ __forceinline__ void mean_value_weights(const Rec& rec, f2 px, f2 py, f2& we, f2& wo, float& general) {
-    f2 qxe, qxo, qye, qyo, qxs, qys;
+// Positions are relative to the tile; px is (x, x), py the (y, y) of kN pixels in one column, whose
+// chains run side by side and share the terms in x. Corners 0 and 2 and corners 1 and 3 go
+// through packed operations. Returns the weights of corners (0, 2) in we and (1, 3) in wo for the
+// pixels marked in `need`, and sets `general` where they may have mixed signs inside a convex quad
+// (the special cases).
+
+// The weights where the common form failed: a vertex on the sample point, an edge's line through
+// it (that tangent in the reference's exact operations), or a weight sum of 0, infinity or NaN
+// (normalised weights would be infinite or NaN, their intensity and reflectance NaN or 0 and so
+// the clamped products 0).
+__device__ __forceinline__ void special_weights(const Rec& rec, float px, float py, f2& we, f2& wo) {
+    float sx[4], sy[4], r2[4], ir[4], t[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int k = corner_slot(i);
+        sx[i] = rec.xy[k] - px;
+        sy[i] = rec.xy[4 + k] - py;
+        r2[i] = sx[i] * sx[i] + sy[i] * sy[i];
+        ir[i] = rsqrtf(r2[i]);
+    }
+    if (r2[0] == 0.0f || r2[1] == 0.0f || r2[2] == 0.0f || r2[3] == 0.0f) {  // one-hot on the first such vertex
+        const int k = r2[0] == 0.0f ? 0 : (r2[1] == 0.0f ? 1 : (r2[2] == 0.0f ? 2 : 3));
+        we = pk(k == 0 ? 1.0f : 0.0f, k == 2 ? 1.0f : 0.0f);
+        wo = pk(k == 1 ? 1.0f : 0.0f, k == 3 ? 1.0f : 0.0f);
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int j = (i + 1) & 3;
+        const float a = sx[i] * sy[j] - sx[j] * sy[i], d = sx[i] * sx[j] + sy[i] * sy[j];
+        if (a == 0.0f)
+            t[i] = __fdiv_rn(__fsub_rn(__fmul_rn(__fsqrt_rn(r2[i]), __fsqrt_rn(r2[j])), d), 1e-3f);
+        else
+            t[i] = ((r2[i] * ir[i]) * (r2[j] * ir[j]) - d) * rcp_approx(a);
+    }
+    we = mul2(pk(t[3] + t[0], t[1] + t[2]), pk(ir[0], ir[2]));
+    wo = mul2(pk(t[0] + t[1], t[2] + t[3]), pk(ir[1], ir[3]));
+    const float sum = (lo2(we) + hi2(we)) + (lo2(wo) + hi2(wo)), inv = rcp_approx(sum);
+    const f2 inv2 = sum * inv > 0.5f ? pk(inv, inv) : 0;
+    we = inv2 ? mul2(we, inv2) : 0;
+    wo = inv2 ? mul2(wo, inv2) : 0;
+}
+
+template <int kN>
+__device__ __forceinline__ void mean_value_weights(const Rec& rec, f2 px, const f2 (&py)[kN], const bool (&need)[kN],
+                                                   f2 (&we)[kN], f2 (&wo)[kN], float& general) {
+    f2 qxe, qxo, qye, qyo, a0, b0, a1, b1, c0, c1, nl0, nl1;
     ld2(rec.xy, qxe, qxo);
     ld2(rec.xy + 4, qye, qyo);
-    ld2(rec.xy + 8, qxs, qys);
-    const f2 xe = sub2(qxe, px), ye = sub2(qye, py), xs = sub2(qxs, px), ys = sub2(qys, py), yo = sub2(qyo, py);
-    const f2 nxo = sub2(px, qxo), nyo = sub2(py, qyo);
-    const f2 a02 = fma2(xe, yo, mul2(nxo, ye));    // a0, a2
-    const f2 na13 = fma2(xs, yo, mul2(nxo, ys));   // -a1, -a3
-    const f2 nd02 = fma2(xe, nxo, mul2(ye, nyo));  // -d0, -d2
-    const f2 nd13 = fma2(xs, nxo, mul2(ys, nyo));  // -d1, -d3
-    const f2 r2e = fma2(xe, xe, mul2(ye, ye)), r2o = fma2(nxo, nxo, mul2(yo, yo));
-    // The common case first. a_i are integers (differences of products of integers): when
-    // none is 0 each |a_i| >= 1 and every term below is finite, so the weight sum is finite.
-    // An a_i of 0 makes t_i infinite or NaN, and a vertex on the sample point (r2_i = 0)
-    // makes r_i NaN; either way sum * (1 / sum) is not near 1, and only then are the weights
-    // redone with the reference's special cases (the rare path).
-    static_assert(!RF_RASTER_EXACT_SMALL_ANGLES, "the rare path is entered only for a_i == 0 or r_i == 0");
-    const f2 ire = pk(rsqrtf(lo2(r2e)), rsqrtf(hi2(r2e))), iro = pk(rsqrtf(lo2(r2o)), rsqrtf(hi2(r2o)));
-    const f2 re = mul2(r2e, ire), ro = mul2(r2o, iro);
-    const f2 n02 = fma2(re, ro, nd02);
-    const f2 n13 = pk(fmaf(lo2(ro), hi2(re), lo2(nd13)), fmaf(hi2(ro), lo2(re), hi2(nd13)));
-    f2 t02 = mul2(n02, pk(rcp_approx(lo2(a02)), rcp_approx(hi2(a02))));
-    f2 nt13 = mul2(n13, pk(rcp_approx(lo2(na13)), rcp_approx(hi2(na13))));
-    wo = mul2(sub2(t02, nt13), iro);                                               // w1, w3
-    we = mul2(pk(lo2(t02) - hi2(nt13), hi2(t02) - lo2(nt13)), ire);                // w0, w2
-    const f2 s2 = add2(we, wo);
-    float sum = lo2(s2) + hi2(s2);
-    float inv = rcp_approx(sum);
-    if (!(sum * inv > 0.5f)) {
-        general = 1.0f;
-        const float r2[4] = {lo2(r2e), lo2(r2o), hi2(r2e), hi2(r2o)};
-        if (r2[0] == 0.0f || r2[1] == 0.0f || r2[2] == 0.0f || r2[3] == 0.0f) {
-            // a vertex on the sample point: one-hot on the first such vertex
-            const int k = r2[0] == 0.0f ? 0 : (r2[1] == 0.0f ? 1 : (r2[2] == 0.0f ? 2 : 3));
-            we = pk(k == 0 ? 1.0f : 0.0f, k == 2 ? 1.0f : 0.0f);
-            wo = pk(k == 1 ? 1.0f : 0.0f, k == 3 ? 1.0f : 0.0f);
-            return;
-        }
-        // on edge i's line: that tangent in the reference's exact operations
-        const float d0 = -lo2(nd02), d1 = -lo2(nd13), d2 = -hi2(nd02), d3 = -hi2(nd13);
-        float t[4] = {lo2(t02), -lo2(nt13), hi2(t02), -hi2(nt13)};
-        if (lo2(a02) == 0.0f) t[0] = __fdiv_rn(__fsub_rn(__fmul_rn(__fsqrt_rn(r2[0]), __fsqrt_rn(r2[1])), d0), 1e-3f);
-        if (lo2(na13) == 0.0f) t[1] = __fdiv_rn(__fsub_rn(__fmul_rn(__fsqrt_rn(r2[1]), __fsqrt_rn(r2[2])), d1), 1e-3f);
-        if (hi2(a02) == 0.0f) t[2] = __fdiv_rn(__fsub_rn(__fmul_rn(__fsqrt_rn(r2[2]), __fsqrt_rn(r2[3])), d2), 1e-3f);
-        if (hi2(na13) == 0.0f) t[3] = __fdiv_rn(__fsub_rn(__fmul_rn(__fsqrt_rn(r2[3]), __fsqrt_rn(r2[0])), d3), 1e-3f);
-        we = mul2(pk(t[3] + t[0], t[1] + t[2]), ire);
-        wo = mul2(pk(t[0] + t[1], t[2] + t[3]), iro);
-        sum = (lo2(we) + hi2(we)) + (lo2(wo) + hi2(wo));
-        inv = rcp_approx(sum);
-        // a weight sum of 0, infinity or NaN: normalised weights would be infinite or NaN, their
-        // intensity and reflectance NaN or 0 and so the clamped products 0
-        if (!(sum * inv > 0.5f)) {
-            we = wo = 0;
-            return;
-        }
+    ld2(rec.ab, a0, b0);
+    ld2(rec.ab + 4, a1, b1);
+    ld2(rec.c, c0, c1);
+    ld2(rec.nl2, nl0, nl1);
+    const f2 xe = sub2(qxe, px), xo = sub2(qxo, px);
+    const f2 xe_xe = mul2(xe, xe), xo_xo = mul2(xo, xo);
+    c0 = fma2(b0, px, c0);
+    c1 = fma2(b1, px, c1);
+    // The common case first: when no a_i is 0 each |a_i| >= 1 and every term below is finite, so
+    // the weight sum is finite. An a_i of 0 makes t_i infinite or NaN, and a vertex on the sample
+    // point (r_i = 0) makes r_i NaN; either way sum * (1 / sum) is not near 1, and only then are
+    // the weights redone with the reference's special cases.
+    float inv[kN];
+    bool bad = false, ok[kN];
+#pragma unroll
+    for (int i = 0; i < kN; i++) {
+        const f2 ye = sub2(qye, py[i]), yo = sub2(qyo, py[i]);
+        const f2 r2e = fma2(ye, ye, xe_xe), r2o = fma2(yo, yo, xo_xo);
+        const f2 a02 = fma2(a0, py[i], c0), a13 = fma2(a1, py[i], c1);  // -a0, -a2 and -a1, -a3
+        const f2 ire = pk(rsqrtf(lo2(r2e)), rsqrtf(hi2(r2e))), iro = pk(rsqrtf(lo2(r2o)), rsqrtf(hi2(r2o)));
+        const f2 re = mul2(r2e, ire), ro = mul2(r2o, iro);
+        const f2 g02 = sub2(re, ro), g13 = pk(lo2(ro) - hi2(re), hi2(ro) - lo2(re));  // r_i - r_j
+        const f2 t02 = mul2(fma2(g02, g02, nl0), pk(rcp_approx(lo2(a02)), rcp_approx(hi2(a02))));
+        const f2 t13 = mul2(fma2(g13, g13, nl1), pk(rcp_approx(lo2(a13)), rcp_approx(hi2(a13))));
+        wo[i] = mul2(add2(t02, t13), iro);                                            // w1, w3
+        we[i] = mul2(pk(lo2(t02) + hi2(t13), hi2(t02) + lo2(t13)), ire);              // w0, w2
+        const f2 s2 = add2(we[i], wo[i]);
+        const float sum = lo2(s2) + hi2(s2);
+        inv[i] = rcp_approx(sum);
+        ok[i] = !need[i] || sum * inv[i] > 0.5f;
+        bad = bad || !ok[i];
+        const f2 inv2 = pk(inv[i], inv[i]);
+        we[i] = mul2(we[i], inv2);
+        wo[i] = mul2(wo[i], inv2);
     }
-    const f2 inv2 = pk(inv, inv);
-    we = mul2(we, inv2);
-    wo = mul2(wo, inv2);
+    if (bad) {
+        general = 1.0f;
+#pragma unroll
+        for (int i = 0; i < kN; i++)
+            if (!ok[i]) special_weights(rec, lo2(px), lo2(py[i]), we[i], wo[i]);
+    }
+}
+__device__ __forceinline__ void mean_value_weights(const Rec& rec, f2 px, f2 py, f2& we, f2& wo, float& general) {
+    const f2 p1[1] = {py};
+    const bool need[1] = {true};
+    f2 e1[1], o1[1];
+    mean_value_weights<1>(rec, px, p1, need, e1, o1, general);
+    we = e1[0];
+    wo = o1[0];
 }
 // sum of weight x value over the corners, values even corners first
 __device__ __forceinline__ float blend4(f2 we, f2 wo, const float* v) {
@@ -321,14 +367,29 @@ __device__ __forceinline__ float blend4(f2 we, f2 wo, const float* v) {
     return lo2(s) + hi2(s);
 }
 
-// Bilinear ghost sample (read_imagef LINEAR, CLAMP -> border 0, rasterizing.cl:483-485)
-// at texel coordinates (u, v) = uv * size - 0.5.
-__device__ __forceinline__ float ghost_sample(const float* __restrict__ tex, int w, int h, float u, float v) {
-    if (!(fabsf(u) + fabsf(v) < 2e9f)) return 0.0f;  // non-finite or far outside
-    const float fu = floorf(u), fv = floorf(v);
-    const float a = u - fu, b = v - fv;
-    const int i0 = (int)fu, j0 = (int)fv;
-    float t00, t10, t01, t11;
+// Bilinear ghost sample (read_imagef LINEAR, CLAMP -> border 0, rasterizing.cl:483-485) at texel
+// coordinates t = uv * size - 0.5, given less half a texel: (u, v) = t - 0.5. The nearest integers
+// of those are the footprint's first texel (where t is an integer the footprint before it may
+// be taken, with a fraction of 1: the same value), found by adding and subtracting 1.5 * 2^23,
+// in packed operations (a floor would go to the same unit as the reciprocals). Returns the
+// footprint's centre (i0 + 1, j0 + 1) and the fractions (a, b). Coordinates beyond 2^22 do not
+// round to integers, but their texels are all outside.
+__device__ __forceinline__ void ghost_footprint(f2 uv, f2& centre, f2& frac) {
+    const f2 big = pk(12582912.0f, 12582912.0f), big1 = pk(12582911.0f, 12582911.0f), half3 = pk(1.5f, 1.5f);
+    centre = sub2(add2(uv, big), big1);
+    frac = add2(sub2(uv, centre), half3);
+}
+// The specification's (1-a)(1-b) t00 + a(1-b) t10 + (1-a) b t01 + a b t11, as three interpolations
+// (the same value up to rounding).
+__device__ __forceinline__ float ghost_blend(float t00, float t10, float t01, float t11, f2 frac) {
+    const float a = lo2(frac), b = hi2(frac);
+    const float top = fmaf(a, t10 - t00, t00), bottom = fmaf(a, t11 - t01, t01);
+    return fmaf(b, bottom - top, top);
+}
+// The footprint's texels by loads.
+__device__ __forceinline__ void ghost_texels(const float* __restrict__ tex, int w, int h, f2 centre, float& t00,
+                                             float& t10, float& t01, float& t11) {
+    const int i1 = cvt_rz_sat(lo2(centre)), j1 = cvt_rz_sat(hi2(centre)), i0 = wsub(i1, 1), j0 = wsub(j1, 1);
     if ((unsigned)i0 < (unsigned)(w - 1) && (unsigned)j0 < (unsigned)(h - 1)) {
         // all four texels inside (the common case)
         const float* q = tex + (j0 * w + i0);
@@ -337,58 +398,78 @@ __device__ __forceinline__ float ghost_sample(const float* __restrict__ tex, int
         t01 = __ldg(q + w);
         t11 = __ldg(q + w + 1);
     } else {
-        const bool i0_in = (unsigned)i0 < (unsigned)w, i1_in = (unsigned)(i0 + 1) < (unsigned)w;
-        const bool j0_in = (unsigned)j0 < (unsigned)h, j1_in = (unsigned)(j0 + 1) < (unsigned)h;
+        const bool i0_in = (unsigned)i0 < (unsigned)w, i1_in = (unsigned)i1 < (unsigned)w;
+        const bool j0_in = (unsigned)j0 < (unsigned)h, j1_in = (unsigned)j1 < (unsigned)h;
         // load from clamped (always valid) addresses, then zero the texels outside the image
-        const int ia = min(max(i0, 0), w - 1), ib = min(max(i0 + 1, 0), w - 1);
+        const int ia = min(max(i0, 0), w - 1), ib = min(max(i1, 0), w - 1);
         const float* row0 = tex + (size_t)min(max(j0, 0), h - 1) * w;
-        const float* row1 = tex + (size_t)min(max(j0 + 1, 0), h - 1) * w;
+        const float* row1 = tex + (size_t)min(max(j1, 0), h - 1) * w;
         t00 = (i0_in && j0_in) ? __ldg(row0 + ia) : 0.0f;
         t10 = (i1_in && j0_in) ? __ldg(row0 + ib) : 0.0f;
         t01 = (i0_in && j1_in) ? __ldg(row1 + ia) : 0.0f;
         t11 = (i1_in && j1_in) ? __ldg(row1 + ib) : 0.0f;
     }
-    // the specification's (1-a)(1-b) t00 + a(1-b) t10 + (1-a) b t01 + a b t11, as three
-    // interpolations (the same value up to rounding)
-    const float top = fmaf(a, t10 - t00, t00), bottom = fmaf(a, t11 - t01, t01);
-    return fmaf(b, bottom - top, top);
 }
-
-// ghost_sample through a texture object over the same texels (float, pitch-linear, border
-// address mode): tex2Dgather at the centre of the 2 x 2 footprint, (i0 + 1, j0 + 1), exactly
-// half a texel from every footprint boundary, returns texels (i0, j0 + 1), (i0 + 1, j0 + 1),
-// (i0 + 1, j0), (i0, j0) in x, y, z, w, and 0 for texels outside the image; one texture
-// instruction instead of the bounds test, the address arithmetic and four loads. The values,
-// and so the interpolation, are ghost_sample's. u and v are finite: the weights are, and records
-// with a texel coordinate that is not are left out (zero_record); far outside, every texel is 0.
-__device__ __forceinline__ float ghost_sample_tex(unsigned long long tex, float u, float v) {
-    const float fu = floorf(u), fv = floorf(v);
-    const float a = u - fu, b = v - fv;
-    const float4 g = tex2Dgather<float4>((cudaTextureObject_t)tex, fu + 1.0f, fv + 1.0f, 0);
-    const float top = fmaf(a, g.z - g.w, g.w), bottom = fmaf(a, g.y - g.x, g.x);
-    return fmaf(b, bottom - top, top);
+// The same texels through a texture object over them (float, pitch-linear, border address
+// mode): tex2Dgather at the footprint's centre, exactly half a texel from every footprint
+// boundary, returns texels (i0, j0 + 1), (i0 + 1, j0 + 1), (i0 + 1, j0), (i0, j0) in x, y, z, w, and
+// 0 for texels outside the image; one texture instruction instead of the bounds test, the
+// address arithmetic and four loads. The values, and so the interpolation, are the loads'. u and v
+// are finite: the weights are, and records with a texel coordinate that is not are left out
+// (zero_record).
+template <bool kTex>
+__device__ __forceinline__ float ghost_sample(const float* __restrict__ tex, const RasterParams& p, f2 uv) {
+    f2 centre, frac;
+    ghost_footprint(uv, centre, frac);
+    float t00, t10, t01, t11;
+    if (kTex) {
+        const float4 g = tex2Dgather<float4>((cudaTextureObject_t)p.ghost_tex, lo2(centre), hi2(centre), 0);
+        t00 = g.w, t10 = g.z, t01 = g.x, t11 = g.y;
+    } else {
+        ghost_texels(tex, p.ghost_w, p.ghost_h, centre, t00, t10, t01, t11);
+    }
+    return ghost_blend(t00, t10, t01, t11, frac);
 }
 
 // fragment_shader (rasterizing.cl:471-506) times the hit count. The texture coordinate
-// ((uv / scale + 1) / 2) * size - 0.5 is evaluated as uv * tex_scale + tex_offset.
+// ((uv / scale + 1) / 2) * size - 0.5, less the half texel of ghost_footprint, is evaluated as
+// uv * tex_scale + tex_offset.
 struct FragmentConsts {
     float tsx, tox, tsy, toy;  // texel coordinate scale and offset per axis
 };
+template <bool kTex, int kN>
+__device__ __forceinline__ void fragment_fast(const Rec& r, const f2 (&we)[kN], const f2 (&wo)[kN],
+                                              const float* __restrict__ ghost, const RasterParams& p, float general,
+                                              float (&f)[kN]) {
+    float gi[kN], ai[kN], ci[kN];
+#pragma unroll
+    for (int i = 0; i < kN; i++) {
+        const float u = blend4(we[i], wo[i], r.uv), v = blend4(we[i], wo[i], r.uv + 4);
+        gi[i] = ghost_sample<kTex>(ghost, p, pk(u, v));
+        ai[i] = blend4(we[i], wo[i], r.inten);
+        ci[i] = blend4(we[i], wo[i], r.refl);
+    }
+    if (general != 0.0f) {
+#pragma unroll
+        for (int i = 0; i < kN; i++) {
+            // smoothstep(1, 0.95, rrel): the ramp (rrel - 1) / (0.95 - 1) is linear in rrel, so the
+            // corners' ramps interpolate to the fragment's (the weights sum to one)
+            const float st = __saturatef(blend4(we[i], wo[i], r.rs));
+            gi[i] *= st * st * (3.0f - 2.0f * st);
+            ai[i] = fmaxf(ai[i], 0.0f);
+            ci[i] = fmaxf(ci[i], 0.0f);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kN; i++) f[i] = gi[i] * ai[i] * ci[i];
+}
 template <bool kTex = false>
 __device__ __forceinline__ float fragment_fast(const Rec& r, f2 we, f2 wo, const float* __restrict__ ghost,
                                                const RasterParams& p, float general) {
-    const float u = blend4(we, wo, r.uv), v = blend4(we, wo, r.uv + 4);
-    float gi = kTex ? ghost_sample_tex(p.ghost_tex, u, v) : ghost_sample(ghost, p.ghost_w, p.ghost_h, u, v);
-    float ai = blend4(we, wo, r.inten), ci = blend4(we, wo, r.refl);
-    if (general != 0.0f) {
-        // smoothstep(1, 0.95, rrel): the ramp (rrel - 1) / (0.95 - 1) is linear in rrel, so the
-        // corners' ramps interpolate to the fragment's (the weights sum to one)
-        const float st = __saturatef(blend4(we, wo, r.rs));
-        gi *= st * st * (3.0f - 2.0f * st);
-        ai = fmaxf(ai, 0.0f);
-        ci = fmaxf(ci, 0.0f);
-    }
-    return gi * ai * ci;
+    const f2 e1[1] = {we}, o1[1] = {wo};
+    float f[1];
+    fragment_fast<kTex, 1>(r, e1, o1, ghost, p, general, f);
+    return f[0];
 }
 
 __host__ __device__ inline FragmentConsts fragment_consts(const RasterParams& p) {
@@ -396,8 +477,8 @@ __host__ __device__ inline FragmentConsts fragment_consts(const RasterParams& p)
     const double sx = 0.5 / p.ghost_scale * p.ghost_w, sy = 0.5 / p.ghost_scale * p.ghost_h;
     fc.tsx = (float)sx;
     fc.tsy = (float)sy;
-    fc.tox = (float)(0.5 * p.ghost_w - 0.5);
-    fc.toy = (float)(0.5 * p.ghost_h - 0.5);
+    fc.tox = (float)(0.5 * p.ghost_w - 1.0);
+    fc.toy = (float)(0.5 * p.ghost_h - 1.0);
     return fc;
 }
 
@@ -428,7 +509,7 @@ __device__ __forceinline__ void load_corner(const float4* __restrict__ vtx, uint
 // is stored in texels, uv * tex_scale + tex_offset (fragment_fast): the weights sum to one,
 // so interpolating texel coordinates is the fragment's ((uv / scale + 1) / 2) * size - 0.5.
 __device__ __forceinline__ void store_corner(const CornerLoad& c, int k, float t, int S, const FragmentConsts& fc,
-                                             Rec& r) {
+                                             float ox, float oy, Rec& r) {
     const float px = c.a0.x + (c.b0.x - c.a0.x) * t, py = c.a0.y + (c.b0.y - c.a0.y) * t;
     const int s = corner_slot(k);
     r.uv[s] = (c.a0.z + (c.b0.z - c.a0.z) * t) * fc.tsx + fc.tox;
@@ -437,14 +518,10 @@ __device__ __forceinline__ void store_corner(const CornerLoad& c, int k, float t
     r.refl[s] = c.a1.y + (c.b1.y - c.a1.y) * t;
     r.inten[s] = c.a1.z + (c.b1.z - c.a1.z) * t;
     const int qx = cvt_rz_sat(px * (float)S), qy = cvt_rz_sat(py * (float)S);
-    r.q[2 * k] = qx;
-    r.q[2 * k + 1] = qy;
-    r.xy[s] = (float)qx;
-    r.xy[4 + s] = (float)qy;
-    if (!(k & 1)) {  // the even corners again, swapped
-        r.xy[8 + (s ^ 1)] = (float)qx;
-        r.xy[10 + (s ^ 1)] = (float)qy;
-    }
+    r.q()[2 * k] = qx;
+    r.q()[2 * k + 1] = qy;
+    r.xy[s] = (float)qx - ox;
+    r.xy[4 + s] = (float)qy - oy;
 }
 // Whether every fragment of a record is zero, so that shading it adds nothing:
 //  - a corner's reflectance is NaN (a ray that failed, at either wavelength of the pair):
@@ -485,10 +562,12 @@ __device__ __forceinline__ bool inside_housing(const Rec& r) {
     return low >= 0.0f && ramp >= 1.0f;
 }
 
-// edges, bounds and flags of a record whose corners are stored; (ox, oy): the tile's first sample
+// edges, bounds and flags of a record whose corners are stored; (ox, oy): the tile's first sample;
+// kRows: the pixel rows of a block
+template <int kRows>
 __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int i, int ox, int oy, const float* xyz,
                                               Rec& r) {
-    const int4 q01 = ld4i(r.q), q23 = ld4i(r.q + 4);
+    const int4 q01 = ld4i(r.q()), q23 = ld4i(r.q() + 4);
     const int q[8] = {q01.x, q01.y, q01.z, q01.w, q23.x, q23.y, q23.z, q23.w};
     const int4 bb = make_int4(min(min(q[0], q[2]), min(q[4], q[6])), max(max(q[0], q[2]), max(q[4], q[6])),
                               min(min(q[1], q[3]), min(q[5], q[7])), max(max(q[1], q[3]), max(q[5], q[7])));
@@ -501,8 +580,9 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
     const int lim = 16382;
     const bool safe = p.safe_screen && bb.x >= -lim && bb.y <= lim && bb.z >= -lim && bb.w <= lim &&
                       (p.S < 8 || (bb.y - bb.x < 16384 && bb.w - bb.z < 16384));
-    const float hx = 4.0f * (float)p.S - 0.5f, hy = 2.0f * (float)p.S - 0.5f;
-    float ea[5], eb[5], ecl[5];
+    const float hx = 4.0f * (float)p.S - 0.5f, hy = 0.5f * kRows * (float)p.S - 0.5f;
+    float ea[5], eb[5], ec[5], ecb[5];
+    bool small = safe;  // the unbiased edge functions too are exact over the tile
 #pragma unroll
     for (int k = 0; k < 5; k++) {
         const int a = k < 4 ? k : 2, b = k < 4 ? (k + 1) & 3 : 0;
@@ -511,7 +591,10 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
         const int c = wadd(e[2], wadd(wmul(e[0], oy), wmul(e[1], ox)));
         ea[k] = (float)e[0];
         eb[k] = (float)e[1];
-        ecl[k] = (float)min(max(c, -8388608), 8388608);
+        ecb[k] = (float)min(max(c, -8388608), 8388608);
+        const int cu = c + (top_left(q[2 * a], q[2 * a + 1], q[2 * b], q[2 * b + 1]) ? 0 : 1);
+        ec[k] = (float)cu;
+        if (k < 4) small = small && cu <= 8388608 && cu >= -8388608;
     }
     int flags = safe ? 1 : 0;
     const bool collinear = edge_i(q[0], q[1], q[2], q[3], q[4], q[5]) == 0 &&
@@ -536,14 +619,21 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
         col.x = c[0], col.y = c[1], col.z = c[2];
     }
     *reinterpret_cast<float4*>(r.col) = col;
-    float4* ef = reinterpret_cast<float4*>(r.ef);
-    ef[0] = make_float4(ea[0], ea[1], eb[0], eb[1]);
-    ef[1] = make_float4(ecl[0], ecl[1], ea[2], ea[3]);
-    ef[2] = make_float4(eb[2], eb[3], ecl[2], ecl[3]);
-    ef[3] = make_float4(ea[4], eb[4], ecl[4], __int_as_float(flags));
-    *reinterpret_cast<float4*>(r.ext) =
-        make_float4(fabsf(ea[0]) * hy + fabsf(eb[0]) * hx, fabsf(ea[1]) * hy + fabsf(eb[1]) * hx,
-                    fabsf(ea[2]) * hy + fabsf(eb[2]) * hx, fabsf(ea[3]) * hy + fabsf(eb[3]) * hx);
+    if (safe) {  // else q stays
+        *reinterpret_cast<float4*>(r.ab) = make_float4(ea[0], ea[2], eb[0], eb[2]);
+        *reinterpret_cast<float4*>(r.ab + 4) = make_float4(ea[1], ea[3], eb[1], eb[3]);
+    }
+    *reinterpret_cast<float4*>(r.c) = make_float4(ec[0], ec[2], ec[1], ec[3]);
+    *reinterpret_cast<float4*>(r.cb) = make_float4(ecb[0], ecb[2], ecb[1], ecb[3]);
+    *reinterpret_cast<float4*>(r.e20) = make_float4(ea[4], eb[4], ecb[4], __int_as_float(flags));
+    float l2[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) l2[k] = small ? -(ea[k] * ea[k] + eb[k] * eb[k]) : __int_as_float(0x7fffffff);
+    *reinterpret_cast<float4*>(r.nl2) = make_float4(l2[0], l2[2], l2[1], l2[3]);
+    float x[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) x[k] = fabsf(ea[k]) * hy + fabsf(eb[k]) * hx;
+    *reinterpret_cast<float4*>(r.ext) = make_float4(x[0], x[2], x[1], x[3]);
 }
 
 // How many of the S n-rook samples of this lane's pixel a record covers. (rx0, ry0): the block's first
@@ -553,7 +643,7 @@ __device__ __forceinline__ int sample_hits(const Rec& r, int S, bool wild, float
                                            int lane) {
     int hits = 0;
     if (wild) {
-        for (int s = 0; s < S; s++) hits += inside_exact(r.q, sx0 + s, sy0 + SUB_OFFSETS[S - 1 + s]) ? 1 : 0;
+        for (int s = 0; s < S; s++) hits += inside_exact(r.q(), sx0 + s, sy0 + SUB_OFFSETS[S - 1 + s]) ? 1 : 0;
         return hits;
     }
     Edges e;
@@ -566,8 +656,8 @@ __device__ __forceinline__ int sample_hits(const Rec& r, int S, bool wild, float
     return hits;
 }
 
-// A CTA of 8 warps shades one T x T tile (T = 32 or 16): the tile's T^2 / 32 blocks of
-// 8 x 4 pixels (block b at column b % (T / 8), row b / (T / 8)) go to warps one at a time,
+// A CTA of 8 warps shades one T x T tile (T = 32 or 16): the tile's blocks of 8 x 4 pixels (8 x 8
+// with two pixels per lane; block b at column b % (T / 8), row b / (T / 8)) go to warps one at a time,
 // so a record outside a block's sample bounds is skipped by the whole warp at once.
 constexpr int kThreads = 256;
 
@@ -578,18 +668,19 @@ constexpr size_t raster_smem_bytes(int maxW, int WS) {
 }
 
 // Tile (tx, ty), whose entries are tile_entries[begin, end). smem4 holds the dynamic shared
-// memory (raster_smem_bytes), next_block two shared counters. kS: the anti-aliasing sample
+// memory (raster_smem_bytes), next_block four shared counters. kS: the anti-aliasing sample
 // count when known at compile time (1), else 0 (p.S). kTex: sample the ghost texture through
 // p.ghost_tex.
-template <int T, int kS, bool kTex = false>
+template <int T, int kS, bool kTex, int kPix>
 __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint32_t begin, uint32_t end,
                                             const uint32_t* __restrict__ tile_entries,
                                             const float* __restrict__ ghost, const float* __restrict__ spectrum,
                                             const RasterParams& p, const FragmentConsts& fcs,
                                             float4* __restrict__ image, int tx, int ty, float4* smem4,
                                             int* next_block) {
-    constexpr int kBlocks = T * T / 32;  // 8 x 4 pixel blocks per tile
-    constexpr int kCols = T / 8;         // blocks per tile row
+    constexpr int kRows = 4 * kPix;                // pixel rows of a block
+    constexpr int kBlocks = T * T / (32 * kPix);   // blocks of 8 x kRows pixels per tile
+    constexpr int kCols = T / 8;                   // blocks per tile row
     Rec* recbuf = (Rec*)smem4;     // two batches of records
     float* xyz = (float*)(recbuf + 2 * kBatchRecords);  // [maxW * WS][3]
     float* blend = xyz + 3 * p.maxW * p.WS;       // [WS]
@@ -621,65 +712,52 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
     RF_STAT(unsigned long long st_iter = 0; unsigned long long st_whole = 0; unsigned long long st_frag = 0;
             unsigned long long st_frag_whole = 0; unsigned long long st_blocks = 0; unsigned long long st_zero = 0;
             unsigned long long st_zero_iter = 0; unsigned long long st_steps = 0;)
-    // accumulators of the pixel blocks, [block * 3 + channel][lane]
+    // accumulators of the pixel blocks, [(block * 3 + channel) * kPix + row][lane]
     float* acc = blend + ((p.WS + 3) & ~3);
 #pragma unroll
-    for (int i = threadIdx.x; i < kBlocks * 96; i += kThreads) acc[i] = 0.0f;
+    for (int i = threadIdx.x; i < kBlocks * 96 * kPix; i += kThreads) acc[i] = 0.0f;
 
     const int per_batch = kBatchRecords / p.WS;  // entries per batch (WS <= kBatchRecords)
     // Batches of records are double-buffered: while warps shade batch t from one buffer,
     // warps that are done build batch t + 1 in the other, one barrier per batch. Thread j
-    // loads corner j % 4 of entry j / 4 (the four corners of an entry sit in one warp), one
-    // batch ahead, into registers.
-    const int my_entry = threadIdx.x >> 2, my_corner = threadIdx.x & 3;
-    constexpr int kLoads = (kBatchRecords + 63) / 64;
-    CornerLoad next[kLoads];
-    int next_w[kLoads];
-    bool have_next[kLoads];
-    auto prefetch = [&](uint32_t first) {
-#pragma unroll
-        for (int h = 0; h < kLoads; h++) {
-            const int e = my_entry + 64 * h;
-            have_next[h] = e < per_batch && first + e < end;
-            if (have_next[h]) {
-                const uint32_t entry = tile_entries[first + e];
-                next_w[h] = (int)(entry % p.maxW);
-                load_corner(vtx, entry, my_corner, p, next[h]);
+    // loads corner j % 4 of entry j / 4 (the four corners of an entry sit in one warp). The
+    // vertices are not fetched ahead: a batch is shaded for tens of microseconds, and 18
+    // registers held through the shading loop cost more than the loads' latency.
+    const int my_corner = lane & 3;
+    // Warps take the batch's entries 8 at a time as they run out of blocks to shade: a warp held
+    // up by a heavy block does not also hold the batch up with its share of the building.
+    auto build = [&](Rec* dst, uint32_t first, int* next_entry) {
+        const int count = (int)min((uint32_t)per_batch, end - first);
+        for (;;) {
+            int e0 = 0;
+            if (lane == 0) e0 = atomicAdd(next_entry, 8);
+            e0 = __shfl_sync(0xffffffffu, e0, 0);
+            if (e0 >= count) break;
+            const int e = e0 + (lane >> 2);
+            uint32_t entry = 0;
+            if (e < count) {
+                entry = tile_entries[first + e];
+                CornerLoad c;
+                load_corner(vtx, entry, my_corner, p, c);
+                for (int i = 0; i < p.WS; i++) store_corner(c, my_corner, blend[i], S, fc, (float)(tx * T * S), (float)(ty * T * S),
+                                                                      dst[e * p.WS + i]);
             }
-        }
-    };
-    // records of the prefetched batch into dst, then prefetch the batch after it
-    auto build = [&](Rec* dst, uint32_t first) {
-#pragma unroll
-        for (int h = 0; h < kLoads; h++) {
-            const int e = my_entry + 64 * h;
-            if (have_next[h])
-                for (int i = 0; i < p.WS; i++)
-                    store_corner(next[h], my_corner, blend[i], S, fc, dst[e * p.WS + i]);
-        }
-        __syncwarp();  // the four corners of each record are stored
-#pragma unroll
-        for (int h = 0; h < kLoads; h++) {
-            const int e = my_entry + 64 * h;
-            if (have_next[h])
+            __syncwarp();  // the four corners of each record are stored
+            if (e < count)
                 for (int i = my_corner; i < p.WS; i += 4)
-                    finish_record(p, next_w[h], i, tx * T * S, ty * T * S, xyz, dst[e * p.WS + i]);
+                    finish_record<kRows>(p, (int)(entry % p.maxW), i, tx * T * S, ty * T * S, xyz, dst[e * p.WS + i]);
         }
-        prefetch(first + per_batch);
     };
-    if (threadIdx.x == 0) {
-        next_block[0] = 0;
-        next_block[1] = 0;
-    }
-    prefetch(begin);
+    // next_block[0, 1]: the next block of each buffer's batch, [2, 3]: its next entry to build
+    if (threadIdx.x < 4) next_block[threadIdx.x] = 0;
     __syncthreads();  // blend weights and colours are set
-    if (begin < end) build(recbuf, begin);
+    if (begin < end) build(recbuf, begin, next_block + 2);
     __syncthreads();
     int cur = 0;
     for (uint32_t base = begin; base < end; base += per_batch, cur ^= 1) {
         const int n_rec = (int)min((uint32_t)per_batch, end - base) * p.WS;
         const Rec* recs = recbuf + cur * kBatchRecords;
-        // Warps take the tile's 8 x 4 blocks one at a time (blocks differ widely in work);
+        // Warps take the tile's blocks one at a time (blocks differ widely in work);
         // a block is shaded by one warp per batch, batches in order, so every pixel still
         // adds its records in increasing order.
 #pragma unroll 1
@@ -689,15 +767,15 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
             blk = __shfl_sync(0xffffffffu, blk, 0);
             if (blk >= kBlocks) break;
             RF_STAT(st_blocks += lane == 0;)
-            const int x0 = tx * T + (blk % kCols) * 8, y0 = ty * T + (blk / kCols) * 4;
-            const int px = x0 + (lane & 7), py = y0 + (lane >> 3);
-            const int bx0 = x0 * S, by0 = y0 * S, bx1 = bx0 + 8 * S - 1, by1 = by0 + 4 * S - 1;
+            const int x0 = tx * T + (blk % kCols) * 8, y0 = ty * T + (blk / kCols) * kRows;
+            const int px = x0 + (lane & 7), py = y0 + (lane >> 3) * kPix;  // the lane's first pixel
+            const int bx0 = x0 * S, by0 = y0 * S, bx1 = bx0 + 8 * S - 1, by1 = by0 + kRows * S - 1;
             const bool in_image = px < p.width && py < p.height;
             const int sx0 = px * S, sy0 = py * S;
-            // which records can touch this 8 x 4 block, which cover all of it, and which need the
+            // which records can touch this block, which cover all of it, and which need the
             // exact test at every sample: lanes test 32 records at a time
-            const float rx0 = (float)((blk % kCols) * 8 * S), ry0 = (float)((blk / kCols) * 4 * S);
-            const float hx = 4.0f * (float)S - 0.5f, hy = 2.0f * (float)S - 0.5f;
+            const float rx0 = (float)((blk % kCols) * 8 * S), ry0 = (float)((blk / kCols) * kRows * S);
+            const float hx = 4.0f * (float)S - 0.5f, hy = 0.5f * kRows * (float)S - 0.5f;
             const f2 bxc = pk(rx0 + hx, rx0 + hx), byc = pk(ry0 + hy, ry0 + hy);
             unsigned sel[kBatchRecords / 32], whole[kBatchRecords / 32], wild[kBatchRecords / 32];
 #pragma unroll
@@ -706,7 +784,7 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
                 bool take = false, all = false, far = false;
                 if (j < n_rec) {
                     const Rec& r = recs[j];
-                    const int flags = __float_as_int(ld4(r.ef + 12).w);  // with ef[12..14], which rect_coverage reads
+                    const int flags = __float_as_int(ld4(r.e20).w);  // with e20, which rect_coverage reads
                     if (!(flags & 2)) {  // collinear (intersect_quad rejects all) or all-zero
                         const int4 bb = *reinterpret_cast<const int4*>(r.bb);
                         far = !(flags & 1);
@@ -722,64 +800,97 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
                 whole[m] = __ballot_sync(0xffffffffu, all);
                 wild[m] = __ballot_sync(0xffffffffu, far);
             }
-            float r0 = acc[(3 * blk) * 32 + lane];
-            float r1 = acc[(3 * blk + 1) * 32 + lane];
-            float r2 = acc[(3 * blk + 2) * 32 + lane];
+            float rgb[3][kPix];
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int i = 0; i < kPix; i++) rgb[c][i] = acc[((3 * blk + c) * kPix + i) * 32 + lane];
             // (no warp-wide operation below: lanes outside the image skip the records)
             if constexpr (kS == 1) {
                 // One sample per pixel: every lane first marks the selected records that cover
-                // its pixel (whole-block records cover every pixel; the others are tested, in a
+                // its pixels (whole-block records cover every pixel; the others are tested, in a
                 // loop that is the same for all lanes), then shades its own covered records in
-                // increasing order. A lane is not held up by records that miss its pixel, so a
-                // warp takes about as many shading steps as its busiest pixel has fragments.
+                // increasing order. A lane is not held up by records that miss its pixels, so a
+                // warp takes about as many shading steps as its busiest lane has records.
                 // Masks are kept bit-reversed (record j at bit 31 - j), so the next record is a
                 // plain count of leading zeros.
-                static_assert(kBatchRecords == 64, "two coverage masks per lane");
-                const float lx = rx0 + (float)(lane & 7), ly = ry0 + (float)(lane >> 3);
-                const f2 lx2 = pk(lx, lx), ly2 = pk(ly, ly);
-                unsigned cov[2];
+                static_assert(kBatchRecords == 64, "two coverage masks per lane and pixel");
+                const float lx = rx0 + (float)(lane & 7);
+                const f2 lx2 = pk(lx, lx);
+                unsigned cov[2][kPix];
 #pragma unroll
                 for (int m = 0; m < 2; m++) {
-                    unsigned c = __brev(whole[m]), part = __brev(sel[m] & ~whole[m] & ~wild[m]);
+                    unsigned c[kPix], part = __brev(sel[m] & ~whole[m] & ~wild[m]);
+#pragma unroll
+                    for (int i = 0; i < kPix; i++) c[i] = __brev(whole[m]);
                     while (part) {
                         const int b = __clz(part);
                         const unsigned bit = 0x80000000u >> b;
                         part ^= bit;
                         Edges e;
                         load_edges(recs[m * 32 + b], e);
-                        if (inside(e, lx2, ly2)) c |= bit;
+#pragma unroll
+                        for (int i = 0; i < kPix; i++) {
+                            const float ly = ry0 + (float)((lane >> 3) * kPix + i);
+                            if (inside(e, lx2, pk(ly, ly))) c[i] |= bit;
+                        }
                     }
                     for (part = __brev(wild[m]); part;) {
                         const int b = __clz(part);
                         const unsigned bit = 0x80000000u >> b;
                         part ^= bit;
-                        if (inside_exact(recs[m * 32 + b].q, sx0, sy0)) c |= bit;
+#pragma unroll
+                        for (int i = 0; i < kPix; i++)
+                            if (inside_exact(recs[m * 32 + b].q(), sx0, sy0 + i)) c[i] |= bit;
                     }
-                    cov[m] = in_image ? c : 0;
+#pragma unroll
+                    for (int i = 0; i < kPix; i++) cov[m][i] = px < p.width && py + i < p.height ? c[i] : 0;
                     RF_STAT(if (lane == 0) { st_iter += __popc(sel[m]); st_whole += __popc(whole[m]); })
                 }
-                const f2 fx2 = pk((float)sx0, (float)sx0), fy2 = pk((float)sy0, (float)sy0);
+                f2 fy2[kPix];
+                unsigned todo[2] = {0, 0};
+#pragma unroll
+                for (int i = 0; i < kPix; i++) {
+                    const float ly = ry0 + (float)((lane >> 3) * kPix + i);
+                    fy2[i] = pk(ly, ly);
+                    todo[0] |= cov[0][i];
+                    todo[1] |= cov[1][i];
+                }
                 const Rec* half = recs;
                 for (;;) {
-                    if (cov[0] == 0) {
-                        cov[0] = cov[1];
-                        cov[1] = 0;
+                    if (todo[0] == 0) {
+                        todo[0] = todo[1];
+                        todo[1] = 0;
                         half += 32;
-                        if (cov[0] == 0) break;
+#pragma unroll
+                        for (int i = 0; i < kPix; i++) cov[0][i] = cov[1][i];
+                        if (todo[0] == 0) break;
                     }
-                    const int j = __clz(cov[0]);
-                    cov[0] ^= 0x80000000u >> j;
+                    const int j = __clz(todo[0]);
+                    const unsigned bit = 0x80000000u >> j;
+                    todo[0] ^= bit;
                     const Rec& r = half[j];
-                    RF_STAT(const int jj = (int)(&r - recs); st_frag++;
-                            st_frag_whole += (whole[jj >> 5] >> (jj & 31)) & 1u;
+                    bool need[kPix];
+#pragma unroll
+                    for (int i = 0; i < kPix; i++) need[i] = kPix == 1 || (cov[0][i] & bit) != 0;
+                    RF_STAT(const int jj = (int)(&r - recs);
+                            for (int i = 0; i < kPix; i++) {
+                                st_frag += need[i];
+                                st_frag_whole += need[i] && ((whole[jj >> 5] >> (jj & 31)) & 1u);
+                            }
                             if (lane == __ffs(__activemask()) - 1) st_steps++;)
-                    f2 we, wo;
+                    f2 we[kPix], wo[kPix];
                     float4 col = ld4(r.col);
-                    mean_value_weights(r, fx2, fy2, we, wo, col.w);
-                    const float f = fragment_fast<kTex>(r, we, wo, ghost, p, col.w);
-                    r0 += col.x * f;
-                    r1 += col.y * f;
-                    r2 += col.z * f;
+                    mean_value_weights<kPix>(r, lx2, fy2, need, we, wo, col.w);
+                    float f[kPix];
+                    fragment_fast<kTex, kPix>(r, we, wo, ghost, p, col.w, f);
+#pragma unroll
+                    for (int i = 0; i < kPix; i++) {
+                        const float fi = need[i] ? f[i] : 0.0f;
+                        rgb[0][i] += col.x * fi;
+                        rgb[1][i] += col.y * fi;
+                        rgb[2][i] += col.z * fi;
+                    }
                 }
             }
 #pragma unroll
@@ -797,7 +908,7 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
                     if (hits == 0) continue;
                     RF_STAT(st_frag++; st_frag_whole += is_whole;)
                     f2 we, wo;
-                    const float cx = (float)(sx0 + S / 2), cy = (float)(sy0 + S / 2);
+                    const float cx = rx0 + (float)((lane & 7) * S + S / 2), cy = ry0 + (float)((lane >> 3) * S + S / 2);
                     float general = 1.0f;
                     mean_value_weights(r, pk(cx, cx), pk(cy, cy), we, wo, general);
                     RF_STAT({
@@ -808,18 +919,20 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
                     })
                     const float4 col = ld4(r.col);
                     const float f = fragment_fast<kTex>(r, we, wo, ghost, p, 1.0f) * (float)hits;
-                    r0 += col.x * f;
-                    r1 += col.y * f;
-                    r2 += col.z * f;
+                    rgb[0][0] += col.x * f;
+                    rgb[1][0] += col.y * f;
+                    rgb[2][0] += col.z * f;
                 }
             }
-            acc[(3 * blk) * 32 + lane] = r0;
-            acc[(3 * blk + 1) * 32 + lane] = r1;
-            acc[(3 * blk + 2) * 32 + lane] = r2;
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int i = 0; i < kPix; i++) acc[((3 * blk + c) * kPix + i) * 32 + lane] = rgb[c][i];
         }
-        if (base + per_batch < end) build(recbuf + (cur ^ 1) * kBatchRecords, base + per_batch);
-        // the other counter was last used by the previous batch, behind the last barrier
-        if (threadIdx.x == 0) next_block[cur ^ 1] = 0;
+        if (base + per_batch < end) build(recbuf + (cur ^ 1) * kBatchRecords, base + per_batch, next_block + 2 + (cur ^ 1));
+        // the other buffer's block counter and this one's entry counter were last used for the
+        // batch before and for building this one, behind the last barrier
+        if (threadIdx.x == 0) next_block[cur ^ 1] = next_block[2 + cur] = 0;
         __syncthreads();
     }
 
@@ -829,24 +942,35 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
             atomicAdd(&g_raster_stats[6], st_zero_iter); atomicAdd(&g_raster_stats[7], st_steps);)
     __syncthreads();  // every block's last batch is shaded
     const float scale = p.intensity / (float)(p.W * p.S * p.WS);
+    for (int blk = warp; blk < kBlocks; blk += 8) {
 #pragma unroll
-    for (int k = 0; k < kBlocks / 8; k++) {
-        const int blk = warp + 8 * k;
-        const int px = tx * T + (blk % kCols) * 8 + (lane & 7), py = ty * T + (blk / kCols) * 4 + (lane >> 3);
-        if (px >= p.width || py >= p.height) continue;
-        const float c0 = acc[(3 * blk) * 32 + lane], c1 = acc[(3 * blk + 1) * 32 + lane],
-                    c2 = acc[(3 * blk + 2) * 32 + lane];
-        float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c0 > 0.0f || c1 > 0.0f || c2 > 0.0f) out = xyz_to_ap1(c0 * scale, c1 * scale, c2 * scale);
-        image[(size_t)(p.height - (py + 1)) * p.width + px] = out;
+        for (int i = 0; i < kPix; i++) {
+            const int px = tx * T + (blk % kCols) * 8 + (lane & 7);
+            const int py = ty * T + (blk / kCols) * kRows + (lane >> 3) * kPix + i;
+            if (px >= p.width || py >= p.height) continue;
+            const float* a = acc + (3 * blk * kPix + i) * 32 + lane;
+            const float c0 = a[0], c1 = a[32 * kPix], c2 = a[64 * kPix];
+            float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c0 > 0.0f || c1 > 0.0f || c2 > 0.0f) out = xyz_to_ap1(c0 * scale, c1 * scale, c2 * scale);
+            image[(size_t)(p.height - (py + 1)) * p.width + px] = out;
+        }
     }
 }
 
-// What bounds it: instruction issue and the latency of the reciprocals and shared loads (68 %
-// issue-active on the 16-surface frame). Corners shaded in packed pairs, edge functions as exact
-// packed FP32 instead of int32, and records wholly inside the housing without falloff and clamps:
-// production frame (2048^2, 91.5 M entries) 118.7 -> 102.1 ms, 16-surface frame 4.12 -> 3.57 ms,
-// four samples x eight sub-steps at 1920 x 1080 29.6 -> 22.3 ms.
+template <int T, int kS>
+constexpr int kPixels = kS != 1 ? 1 : (T == 32 ? RF_RASTER_PIX32 : RF_RASTER_PIX16);
+
+// What bounds it: instruction issue, the FP32 pipe and the reciprocals together (69 % issue-active,
+// FP32 pipe 60 %, reciprocals 48 % on the 16-surface frame). Production frame (2048^2, 91.5 M
+// entries) / 16-surface frame / four samples x eight sub-steps at 1920 x 1080:
+//  118.7 / 4.12 / 29.6 ms  scalar corners, int32 edge functions, one pixel per lane
+//  102.1 / 3.57 / 22.3 ms  corners in packed pairs, edge functions as exact packed FP32, records
+//                          wholly inside the housing without falloff and clamps
+//   90.2 / 3.22 / 21.5 ms  two pixels of a column per lane (one sample per pixel): a record's
+//                          loads, loop and x terms serve both, and their chains overlap; next
+//                          batch's vertices not held in registers
+//   88.6 / 3.15 / 21.0 ms  cross products from the edge functions, products r_i r_j - d_i from the
+//                          edge lengths, texel origins without floors
 // One CTA per tile of a frame: CTA k shades tile order[k], or tile k without an order.
 // CTAs start in index order as slots free up, so an order by decreasing work starts the
 // heaviest tiles first and ends the launch with light ones.
@@ -857,9 +981,9 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : 
              const float* __restrict__ ghost, const float* __restrict__ spectrum, RasterParams p, FragmentConsts fcs,
              float4* __restrict__ image) {
     extern __shared__ float4 smem4[];
-    __shared__ int next_block[2];  // blocks of each buffer's batch handed out so far
+    __shared__ int next_block[4];  // per buffer: blocks handed out, entries handed out to build
     const int tile = order ? (int)order[blockIdx.x] : (int)blockIdx.x;
-    raster_tile<T, kS, kTex>(vtx, tile_offsets[tile], tile_offsets[tile + 1], tile_entries, ghost, spectrum, p, fcs,
+    raster_tile<T, kS, kTex, kPixels<T, kS>>(vtx, tile_offsets[tile], tile_offsets[tile + 1], tile_entries, ghost, spectrum, p, fcs,
                              image, tile % p.ntx, tile / p.ntx, smem4, next_block);
 }
 
@@ -877,7 +1001,7 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : 
                    const uint32_t* __restrict__ tile_entries, const float* __restrict__ ghosts,
                    const float* __restrict__ spectrum, float4* __restrict__ images) {
     extern __shared__ float4 smem4[];
-    __shared__ int next_block[2];
+    __shared__ int next_block[4];
     // the current tile's frame settings, held in shared memory rather than registers
     __shared__ RasterParams sp;
     __shared__ FragmentConsts sfc;
@@ -908,7 +1032,7 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : 
         __syncthreads();
         if (item >= tiles) break;
         const int gt = s_gt, tile = s_tile;
-        raster_tile<T, kS, kTex>(vtx_all + 2 * s_vtx, tile_offsets[gt], tile_offsets[gt + 1], tile_entries,
+        raster_tile<T, kS, kTex, kPixels<T, kS>>(vtx_all + 2 * s_vtx, tile_offsets[gt], tile_offsets[gt + 1], tile_entries,
                            ghosts + s_ghost, spectrum, sp, sfc, images + s_image, tile % sp.ntx, tile / sp.ntx, smem4,
                            next_block);
         __syncthreads();  // the tile's accumulators and `item` are free again
@@ -916,38 +1040,20 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : 
 }
 
 // ---------------------------------------------------------------- adjoint
-// ghost_sample with its derivatives with respect to the texel coordinates (u, v).
-__device__ __forceinline__ float ghost_sample_grad(const float* __restrict__ tex, int w, int h, float u, float v,
+// ghost_sample with its derivatives with respect to the texel coordinates.
+template <bool kTex>
+__device__ __forceinline__ float ghost_sample_grad(const float* __restrict__ tex, const RasterParams& p, f2 uv,
                                                    float& du, float& dv) {
-    du = dv = 0.0f;
-    if (!(fabsf(u) < 1e9f) || !(fabsf(v) < 1e9f)) return 0.0f;
-    const float fu = floorf(u), fv = floorf(v);
-    const float a = u - fu, b = v - fv;
-    const int i0 = (int)fu, j0 = (int)fv;
-    const bool i0_in = (unsigned)i0 < (unsigned)w, i1_in = (unsigned)(i0 + 1) < (unsigned)w;
-    const bool j0_in = (unsigned)j0 < (unsigned)h, j1_in = (unsigned)(j0 + 1) < (unsigned)h;
-    const int ia = min(max(i0, 0), w - 1), ib = min(max(i0 + 1, 0), w - 1);
-    const float* row0 = tex + (size_t)min(max(j0, 0), h - 1) * w;
-    const float* row1 = tex + (size_t)min(max(j0 + 1, 0), h - 1) * w;
-    const float t00 = (i0_in && j0_in) ? __ldg(row0 + ia) : 0.0f;
-    const float t10 = (i1_in && j0_in) ? __ldg(row0 + ib) : 0.0f;
-    const float t01 = (i0_in && j1_in) ? __ldg(row1 + ia) : 0.0f;
-    const float t11 = (i1_in && j1_in) ? __ldg(row1 + ib) : 0.0f;
-    du = (1.0f - b) * (t10 - t00) + b * (t11 - t01);
-    dv = (1.0f - a) * (t01 - t00) + a * (t11 - t10);
-    return (1.0f - a) * (1.0f - b) * t00 + a * (1.0f - b) * t10 + (1.0f - a) * b * t01 + a * b * t11;
-}
-
-// ghost_sample_grad with the four texels from one gather of the ghost texture's texture object
-// (border mode: texels outside the texture read 0, as the loads' bounds checks give).
-__device__ __forceinline__ float ghost_sample_grad_tex(unsigned long long tex, float u, float v, float& du,
-                                                       float& dv) {
-    du = dv = 0.0f;
-    if (!(fabsf(u) < 1e9f) || !(fabsf(v) < 1e9f)) return 0.0f;
-    const float fu = floorf(u), fv = floorf(v);
-    const float a = u - fu, b = v - fv;
-    const float4 g = tex2Dgather<float4>((cudaTextureObject_t)tex, fu + 1.0f, fv + 1.0f, 0);
-    const float t00 = g.w, t10 = g.z, t01 = g.x, t11 = g.y;
+    f2 centre, frac;
+    ghost_footprint(uv, centre, frac);
+    float t00, t10, t01, t11;
+    if (kTex) {
+        const float4 g = tex2Dgather<float4>((cudaTextureObject_t)p.ghost_tex, lo2(centre), hi2(centre), 0);
+        t00 = g.w, t10 = g.z, t01 = g.x, t11 = g.y;
+    } else {
+        ghost_texels(tex, p.ghost_w, p.ghost_h, centre, t00, t10, t01, t11);
+    }
+    const float a = lo2(frac), b = hi2(frac);
     du = (1.0f - b) * (t10 - t00) + b * (t11 - t01);
     dv = (1.0f - a) * (t01 - t00) + a * (t11 - t10);
     return (1.0f - a) * (1.0f - b) * t00 + a * (1.0f - b) * t10 + (1.0f - a) * b * t01 + a * b * t11;
@@ -1057,7 +1163,8 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? 3 : 2)
                 const uint32_t entry = tile_entries[first + e];
                 CornerLoad c;
                 load_corner(vtx, entry, my_corner, p, c);
-                for (int i = 0; i < p.WS; i++) store_corner(c, my_corner, blend[i], S, fc, dst[e * p.WS + i]);
+                for (int i = 0; i < p.WS; i++)
+                    store_corner(c, my_corner, blend[i], S, fc, (float)(tx * T * S), (float)(ty * T * S), dst[e * p.WS + i]);
                 if (my_corner == 0) {  // where the record's gradients go (the batch's flush)
                     const long long prim = entry / p.maxW;
                     const int w = (int)(entry % p.maxW);
@@ -1076,7 +1183,7 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? 3 : 2)
             if (e < per_batch && first + e < end) {
                 const uint32_t entry = tile_entries[first + e];
                 for (int i = my_corner; i < p.WS; i += 4)
-                    finish_record(p, (int)(entry % p.maxW), i, tx * T * S, ty * T * S, xyz, dst[e * p.WS + i]);
+                    finish_record<4>(p, (int)(entry % p.maxW), i, tx * T * S, ty * T * S, xyz, dst[e * p.WS + i]);
             }
         }
     };
@@ -1119,7 +1226,7 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? 3 : 2)
                 bool take = false, all = false, far = false;
                 if (j < n_rec) {
                     const Rec& r = recs[j];
-                    const int flags = __float_as_int(ld4(r.ef + 12).w);  // with ef[12..14], which rect_coverage reads
+                    const int flags = __float_as_int(ld4(r.e20).w);  // with e20, which rect_coverage reads
                     if (!(flags & 2)) {  // collinear (intersect_quad rejects all) or all-zero
                         const int4 bb = *reinterpret_cast<const int4*>(r.bb);
                         far = !(flags & 1);
@@ -1152,7 +1259,8 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? 3 : 2)
                     float wt[4] = {0.f, 0.f, 0.f, 0.f};
                     if (hits > 0) {
                         f2 we, wo;
-                        const float cx = (float)(sx0 + S / 2), cy = (float)(sy0 + S / 2);
+                        const float cx = rx0 + (float)((lane & 7) * S + S / 2);
+                        const float cy = ry0 + (float)((lane >> 3) * S + S / 2);
                         float general = 1.0f;
                         mean_value_weights(r, pk(cx, cx), pk(cy, cy), we, wo, general);
                         wt[0] = lo2(we), wt[1] = lo2(wo), wt[2] = hi2(we), wt[3] = hi2(wo);
@@ -1160,8 +1268,7 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? 3 : 2)
                         const float dLdf = g0 * col.x + g1 * col.y + g2 * col.z;
                         const float u = blend4(we, wo, r.uv), v = blend4(we, wo, r.uv + 4);
                         float dgu, dgv;
-                        const float gi = kTex ? ghost_sample_grad_tex(p.ghost_tex, u, v, dgu, dgv)
-                                              : ghost_sample_grad(ghost, p.ghost_w, p.ghost_h, u, v, dgu, dgv);
+                        const float gi = ghost_sample_grad<kTex>(ghost, p, pk(u, v), dgu, dgv);
                         const float st = __saturatef(blend4(we, wo, r.rs));
                         const float ri = st * st * (3.0f - 2.0f * st);
                         const float dri = (st > 0.0f && st < 1.0f) ? 6.0f * st * (1.0f - st) * (1.0f / (0.95f - 1.0f))
@@ -1264,11 +1371,12 @@ __global__ void __launch_bounds__(256) k_raster_masks(const float4* __restrict__
                     for (int c = 0; c < 4; c++) {
                         const long long vi = (path * VC + corners[c]) * p.W + w;
                         const CornerLoad cl = {vtx[2 * vi], vtx[2 * vi + 1], vtx[2 * vi + 2], vtx[2 * vi + 3]};
-                        store_corner(cl, c, sub_pos, S, fc, r);
+                        store_corner(cl, c, sub_pos, S, fc, 0.0f, 0.0f, r);
                     }
-                    const int* qq = r.q;
-                    const bool never = edge_i(qq[0], qq[1], qq[2], qq[3], qq[4], qq[5]) == 0 &&
-                                       edge_i(qq[0], qq[1], qq[4], qq[5], qq[6], qq[7]) == 0;
+                    const int* qq = r.q();
+                    const bool never = (edge_i(qq[0], qq[1], qq[2], qq[3], qq[4], qq[5]) == 0 &&
+                                       edge_i(qq[0], qq[1], qq[4], qq[5], qq[6], qq[7]) == 0) ||
+                                       zero_record(p, r, false);
                     int hits = 0;
                     if (!never)
                         for (int s = 0; s < S; s++)
@@ -1276,9 +1384,7 @@ __global__ void __launch_bounds__(256) k_raster_masks(const float4* __restrict__
                     float f = 0.0f;
                     if (hits > 0) {
                         f2 we, wo;
-                        const float cx = (float)(sx0 + S / 2), cy = (float)(sy0 + S / 2);
-                        float general = 1.0f;
-                        mean_value_weights(r, pk(cx, cx), pk(cy, cy), we, wo, general);
+                        special_weights(r, (float)(sx0 + S / 2), (float)(sy0 + S / 2), we, wo);
                         f += fragment_fast(r, we, wo, ghost, p, 1.0f) * (float)hits;
                     }
                     if (p.W > 1) {
