@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_intersections(const rf_
                                                                        int count) {
     __shared__ SmemElement se[kMaxElements];
     const bool disperse = !isnan(__ldg(&elements[0].coefficients[0]));
-    stage_lens(elements, wavelengths, p.E, p.W, 0, 0, false, disperse, se, nullptr);
+    stage_lens(elements, wavelengths, p.E, p.W, 0, 0, false, disperse, se, nullptr, nullptr);
     __syncthreads();
     const long long idx = (long long)blockIdx.x * kTraceThreads + threadIdx.x;
     if (idx >= p.n_rays) return;
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_intersections(const rf_
     const int gx = ray_id - gy * p.G;
     IntersectionRecorder rec{inter + idx * count, count};
     float out[6];
-    trace_ray_rec(se, nullptr, disperse, &elements[0].coefficients[0], __ldg(wavelengths + wl_id),
+    trace_ray_rec(se, nullptr, nullptr, disperse, &elements[0].coefficients[0], __ldg(wavelengths + wl_id),
                   __ldg(paths + path_id), p.grid[gx], p.grid[gy], f, out, rec);
     const long long n = p.n_rays;
 #pragma unroll

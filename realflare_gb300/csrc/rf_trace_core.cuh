@@ -17,7 +17,6 @@ namespace {
 constexpr int kTraceThreads = 256;
 constexpr int kMaxElements = 128;
 constexpr int kMaxGrid = 2048;  // (float)ray_id / G is exact enough for trunc() up to 2048
-constexpr int kMaxTableWavelengths = 64;  // per block; larger spans fall back to global
 
 struct TraceParams {
     long long n_rays;
@@ -27,16 +26,36 @@ struct TraceParams {
     float grid[kMaxGrid];  // grid_length * ((float)i / (G - 1) - 0.5), rounded from double
 };
 
-struct SmemElement {
+struct alignas(16) SmemElement {
     float radius, center, height, ior;
     int coating, layers;
     float d0, d1;
 };
 
 struct Hit {
-    float px, py, pz, nx, ny, nz, incident;
+    float px, py, pz, nx, ny, nz;
     bool hit;
 };
+
+// Correctly rounded square root and reciprocal without the range handling of the general
+// operations, which the trace's operands do not need (it is bound by instruction issue): the
+// hardware approximation and one residual correction with fused multiply-adds (P. Markstein,
+// Computation of elementary functions on the IBM RISC System/6000 processor, 1990). Compared
+// with the correctly rounded instructions for every float in [1, 4): equal; scaling by 4 (by 2)
+// scales every step exactly while the residual does not underflow. sqrt_rn: x = 0 or in
+// [2^-100, 2^127] (below, where an ulp can be lost, the roots of squared distances are added to
+// or compared with lens radii: no effect); inf gives NaN. rcp_rn: |x| in [2^-100, 2^100].
+__device__ __forceinline__ float sqrt_rn(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(x, 1.17549435e-38f)));
+    const float s = __fmul_rn(x, y);
+    return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, y), s);
+}
+__device__ __forceinline__ float rcp_rn(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return __fmaf_rn(__fmaf_rn(-x, y, 1.0f), y, y);
+}
 
 // Inlining of the reflection-only functions (RF_CORE_COLD: the Fresnel variants) and of the
 // sphere/plane intersection (RF_CORE_HOT); a unit may define them __noinline__ before
@@ -50,11 +69,12 @@ struct Hit {
 __device__ RF_CORE_HOT Hit intersect(float px, float py, float pz, float dx, float dy, float dz,
                                          const SmemElement& e) {
     Hit h;
-    h.px = h.py = h.pz = h.nx = h.ny = h.nz = h.incident = 0.0f;
+    h.px = h.py = h.pz = h.nx = h.ny = h.nz = 0.0f;
     h.hit = false;
     if (dz == 0.0f) return h;
-    if (e.radius == 0.0f) {
-        float t = (-e.center - pz) / dz;
+    const float radius = e.radius, cz = -e.center;
+    if (radius == 0.0f) {
+        float t = (cz - pz) / dz;
         h.px = px + dx * t;
         h.py = py + dy * t;
         h.pz = pz + dz * t;
@@ -62,28 +82,27 @@ __device__ RF_CORE_HOT Hit intersect(float px, float py, float pz, float dx, flo
         h.ny = 0.0f;
         h.nz = (dz < 0.0f) ? 1.0f : -1.0f;
         h.hit = true;
-        h.incident = 0.0f;
         return h;
     }
-    float r = fabsf(e.radius);
-    float cz = -e.center;
-    float ux = 0.0f - px, uy = 0.0f - py, uz = cz - pz;
-    float proj = ux * dx + uy * dy + uz * dz;
-    float u1x = dx * proj, u1y = dy * proj, u1z = dz * proj;
-    float ex = ux - u1x, ey = uy - u1y, ez = uz - u1z;
-    float d = sqrtf(ex * ex + ey * ey + ez * ez);
-    if (d > r) return h;
-    float sgn = (e.radius * dz) > 0.0f ? -1.0f : 1.0f;
-    float m = sqrtf(r * r - d * d);
-    h.px = (px + u1x) - (dx * m) * sgn;
-    h.py = (py + u1y) - (dy * m) * sgn;
-    h.pz = (pz + u1z) - (dz * m) * sgn;
-    float qx = h.px, qy = h.py, qz = h.pz - cz;
-    float inv = 1.0f / sqrtf(qx * qx + qy * qy + qz * qz);
-    h.nx = (qx * inv) * sgn;
-    h.ny = (qy * inv) * sgn;
-    h.nz = (qz * inv) * sgn;
-    h.incident = 0.0f;  // acos of the incidence cosine, needed only at reflections
+    // u = (0, 0, cz) - p; products and differences as the reference rounds them (signs moved, which
+    // is exact)
+    const float uz = cz - pz;
+    const float proj = -px * dx + -py * dy + uz * dz;
+    const float u1x = dx * proj, u1y = dy * proj, u1z = dz * proj;
+    const float ex = -px - u1x, ey = -py - u1y, ez = uz - u1z;
+    const float d2 = ex * ex + ey * ey + ez * ez;
+    const float d = sqrt_rn(d2);
+    if (d > fabsf(radius) || d2 > 1e37f) return h;
+    const float sgn = (radius * dz) > 0.0f ? -1.0f : 1.0f;
+    const float m = sqrt_rn(radius * radius - d * d) * sgn;
+    h.px = (px + u1x) - dx * m;
+    h.py = (py + u1y) - dy * m;
+    h.pz = (pz + u1z) - dz * m;
+    const float qz = h.pz - cz;
+    const float inv = rcp_rn(sqrt_rn(h.px * h.px + h.py * h.py + qz * qz)) * sgn;
+    h.nx = h.px * inv;
+    h.ny = h.py * inv;
+    h.nz = qz * inv;
     h.hit = true;
     return h;
 }
@@ -93,71 +112,76 @@ __device__ __forceinline__ float incident_angle(float dx, float dy, float dz, co
     return acosf(clampf(c, -1.0f, 1.0f));
 }
 
-__device__ RF_CORE_COLD float fresnel(float theta0, float n1, float n2) {
-    float theta1 = asinf(sinf(theta0) * n1 / n2);
-    float cosi = cosf(theta0);
-    float cost = cosf(theta1);
-    float rs = ((n1 * cosi) - (n2 * cost)) / ((n1 * cosi) + (n2 * cost));
-    float rp = ((n1 * cost) - (n2 * cosi)) / ((n1 * cost) + (n2 * cosi));
+// The reference's reflectances (fresnel, fresnel_ar; raytracing.cl:1-59) take the incidence angle
+// and evaluate sines and tangents of sums and differences of it and the refracted angles. With the
+// refraction law they are rational in the cosines, which is how they are evaluated here (c0, s0:
+// cosine and sine of the incidence angle, from the incidence cosine itself): no inverse and
+// forward trigonometric functions, and no 0 / 0 at normal incidence (where the reference adds
+// 1e-9 to the angle). Total reflection gives NaN, as the reference's arcsine does.
+__device__ __forceinline__ float incident_cos(float dx, float dy, float dz, const Hit& h) {
+    return clampf(-dx * h.nx + -dy * h.ny + -dz * h.nz, -1.0f, 1.0f);
+}
+__device__ __forceinline__ float refracted_cos(float s) {
+    const float x = 1.0f - s * s;
+    return x < 0.0f ? __int_as_float(0x7fffffff) : sqrt_rn(x);
+}
+// interface reflectances of s- and p-polarised light: -sin(i - j) / sin(i + j) and tan(i - j) /
+// tan(i + j) for angles i, j with ni sin(i) = nj sin(j)
+__device__ __forceinline__ void interface_r(float ni, float ci, float nj, float cj, float& rs, float& rp) {
+    rs = (ni * ci - nj * cj) * rcp_rn(ni * ci + nj * cj);
+    rp = (nj * ci - ni * cj) * rcp_rn(nj * ci + ni * cj);
+}
+
+__device__ RF_CORE_COLD float fresnel(float c0, float s0, float n1, float n2) {
+    float rs, rp;
+    interface_r(n1, c0, n2, refracted_cos(s0 * (n1 / n2)), rs, rp);
     return (rs * rs + rp * rp) / 2.0f;
 }
 
-__device__ RF_CORE_COLD float fresnel_ar(float theta0, float lambda, float d1, float n0, float n1, float n2) {
-    float s0 = sinf(theta0);
-    float theta1 = asinf(s0 * n0 / n1);
-    float theta2 = asinf(s0 * n0 / n2);
-    float rs01 = -sinf(theta0 - theta1) / sinf(theta0 + theta1);
-    float rp01 = tanf(theta0 - theta1) / tanf(theta0 + theta1);
-    float ts01 = 2.0f * sinf(theta1) * cosf(theta0) / sinf(theta0 + theta1);
-    float tp01 = ts01 * cosf(theta0 - theta1);
-    float rs12 = -sinf(theta1 - theta2) / sinf(theta1 + theta2);
-    float rp12 = tanf(theta1 - theta2) / tanf(theta1 + theta2);
-    float ris = ts01 * ts01 * rs12;
-    float rip = tp01 * tp01 * rp12;
-    float dy = d1 * n1;
-    float dx = tanf(theta1) * dy;
-    float delay = sqrtf(dx * dx + dy * dy);
-    float rel_phase = 4.0f * RF_MPI_F / lambda * (delay - dx * s0);
-    float c = cosf(rel_phase);
-    float out_s2 = rs01 * rs01 + ris * ris + 2.0f * rs01 * ris * c;
-    float out_p2 = rp01 * rp01 + rip * rip + 2.0f * rp01 * rip * c;
+__device__ RF_CORE_COLD float fresnel_ar(float c0, float s0, float lambda, float d1, float n0, float n1, float n2) {
+    const float s1 = s0 * n0 / n1;
+    const float c1 = refracted_cos(s1), c2 = refracted_cos(s0 * n0 / n2);
+    float rs01, rp01, rs12, rp12;
+    interface_r(n0, c0, n1, c1, rs01, rp01);
+    interface_r(n1, c1, n2, c2, rs12, rp12);
+    const float ts01 = 2.0f * (n0 * c0) * rcp_rn(n0 * c0 + n1 * c1);
+    const float tp01 = ts01 * (c0 * c1 + s0 * s1);  // cos(theta0 - theta1)
+    const float ris = ts01 * ts01 * rs12;
+    const float rip = tp01 * tp01 * rp12;
+    // delay sqrt(dx^2 + dy^2) - dx sin(theta0), dy = d1 n1, dx = tan(theta1) dy
+    const float dy = d1 * n1;
+    const float c = cosf(4.0f * RF_MPI_F / lambda * ((fabsf(dy) - dy * s1 * s0) * rcp_rn(c1)));
+    const float out_s2 = rs01 * rs01 + ris * ris + 2.0f * rs01 * ris * c;
+    const float out_p2 = rp01 * rp01 + rip * rip + 2.0f * rp01 * rip * c;
     return (out_s2 + out_p2) / 2.0f;
 }
 
 // Exact two-layer thin-film reflectance (no reference counterpart; the same definition as
 // the oracle): incident medium n0 | layer a | layer b | substrate n2, s/p averaged.
-__device__ __forceinline__ void interface_r(float ni, float ci, float nj, float cj, float& rs, float& rp) {
-    rs = (ni * ci - nj * cj) / (ni * ci + nj * cj);
-    rp = (nj * ci - ni * cj) / (nj * ci + ni * cj);
-}
-__device__ __forceinline__ float stack_r2(float r01, float r12, float r23, float d1, float d2) {
-    float s2, c2, s1, c1;
-    sincosf(d2, &s2, &c2);
-    sincosf(d1, &s1, &c1);
+__device__ __forceinline__ float stack_r2(float r01, float r12, float r23, float s1, float c1, float s2, float c2) {
     float nre = r12 + r23 * c2, nim = r23 * s2;
     float dre = 1.0f + r12 * r23 * c2, dim = r12 * r23 * s2;
-    float den = dre * dre + dim * dim;
-    float ire = (nre * dre + nim * dim) / den;
-    float iim = (nim * dre - nre * dim) / den;
+    float den = rcp_rn(dre * dre + dim * dim);
+    float ire = (nre * dre + nim * dim) * den;
+    float iim = (nim * dre - nre * dim) * den;
     float ere = ire * c1 - iim * s1, eim = ire * s1 + iim * c1;
     float tre = r01 + ere, tim = eim;
     float bre = 1.0f + r01 * ere, bim = r01 * eim;
-    return (tre * tre + tim * tim) / (bre * bre + bim * bim);
+    return (tre * tre + tim * tim) * rcp_rn(bre * bre + bim * bim);
 }
-__device__ RF_CORE_COLD float fresnel_two_layer(float theta0, float lambda, float n0, float na, float da,
+__device__ RF_CORE_COLD float fresnel_two_layer(float c0, float s0, float lambda, float n0, float na, float da,
                                                    float nb, float db, float n2) {
-    float s0, c0;
-    sincosf(theta0, &s0, &c0);
-    float sa = n0 * s0 / na, sb = n0 * s0 / nb, s2 = n0 * s0 / n2;
-    float ca = sqrtf(1.0f - sa * sa), cb = sqrtf(1.0f - sb * sb), c2 = sqrtf(1.0f - s2 * s2);
+    const float ns = n0 * s0;
+    const float ca = refracted_cos(ns / na), cb = refracted_cos(ns / nb), c2 = refracted_cos(ns / n2);
     float rs01, rp01, rs12, rp12, rs23, rp23;
     interface_r(n0, c0, na, ca, rs01, rp01);
     interface_r(na, ca, nb, cb, rs12, rp12);
     interface_r(nb, cb, n2, c2, rs23, rp23);
-    float phase = 4.0f * RF_MPI_F / lambda;
-    float d1 = phase * na * da * ca;
-    float d2 = phase * nb * db * cb;
-    return (stack_r2(rs01, rs12, rs23, d1, d2) + stack_r2(rp01, rp12, rp23, d1, d2)) / 2.0f;
+    const float phase = 4.0f * RF_MPI_F / lambda;
+    float sd1, cd1, sd2, cd2;
+    sincosf(phase * na * da * ca, &sd1, &cd1);
+    sincosf(phase * nb * db * cb, &sd2, &cd2);
+    return (stack_r2(rs01, rs12, rs23, sd1, cd1, sd2, cd2) + stack_r2(rp01, rp12, rp23, sd1, cd1, sd2, cd2)) / 2.0f;
 }
 
 // dispersion, raytracing.cl:107-120 (lambda * 1e-3 is a double expression there)
@@ -179,16 +203,19 @@ __device__ __forceinline__ void reflect_dir(float& dx, float& dy, float& dz, con
 }
 
 // refract (raytracing.cl:70-86) with o = n1 / n2; the direction is zeroed past total
-// internal reflection
-__device__ __forceinline__ void refract_dir(float& dx, float& dy, float& dz, const Hit& h, float n1, float n2) {
-    const float o = n1 / n2;
+// internal reflection (the reference multiplies by 0 there and by 1 elsewhere)
+__device__ __forceinline__ void refract_dir(float& dx, float& dy, float& dz, const Hit& h, float o) {
     const float cost = -dx * h.nx + -dy * h.ny + -dz * h.nz;
     const float sint2 = (o * o) * (1.0f - cost * cost);
-    const float k = o * cost - sqrtf(fabsf(1.0f - sint2));
-    const float valid = (float)(sint2 < 1.0f);
-    dx = (o * dx + k * h.nx) * valid;
-    dy = (o * dy + k * h.ny) * valid;
-    dz = (o * dz + k * h.nz) * valid;
+    const float k = o * cost - sqrt_rn(fabsf(1.0f - sint2));
+    dx = o * dx + k * h.nx;
+    dy = o * dy + k * h.ny;
+    dz = o * dz + k * h.nz;
+    if (!(sint2 < 1.0f)) {
+        dx *= 0.0f;
+        dy *= 0.0f;
+        dz *= 0.0f;
+    }
 }
 
 // Per-frame constants of the trace.
@@ -210,11 +237,28 @@ struct NoRecord {
     __device__ __forceinline__ void reflect() {}
 };
 
+// A wavelength's entry for one element: its index and the index ratios n1 / n2 a ray refracted there
+// sees going towards the light (dz < 0: n1 is the element before) or the sensor (the element after);
+// an index outside the lens is 1.
+struct IorEntry {
+    float ior, down, up;
+};
+template <class IorOf>
+__device__ __forceinline__ IorEntry ior_entry(int el, int E, IorOf ior_of) {
+    IorEntry r;
+    r.ior = ior_of(el);
+    r.down = (el > 0 ? ior_of(el - 1) : 1.0f) / r.ior;
+    r.up = (el + 1 < E ? ior_of(el + 1) : 1.0f) / r.ior;
+    return r;
+}
+
 // One ray: init_ray (raytracing.cl:178-215) from grid point (grid_x, grid_y), then the
 // element loop of raytrace (218-359). ior_row: this ray's wavelength row of the (wavelength,
 // element) index table in shared memory, or nullptr to evaluate dispersion per element.
+// ratio_row: the row's index ratios, or nullptr to divide.
 template <class Recorder>
-__device__ __forceinline__ void trace_ray_rec(const SmemElement* __restrict__ se, const float* ior_row, bool disperse,
+__device__ __forceinline__ void trace_ray_rec(const SmemElement* __restrict__ se, const float* ior_row,
+                                              const float2* ratio_row, bool disperse,
                                               const float* __restrict__ coef_base, float wavelength, int2 path,
                                               float grid_x, float grid_y, const TraceFrame& f, float out[6],
                                               Recorder& rec) {
@@ -239,7 +283,11 @@ __device__ __forceinline__ void trace_ray_rec(const SmemElement* __restrict__ se
     pz = pz - dz;
     float apt_x = 0.0f, apt_y = 0.0f, rrel = 0.0f, refl = 1.0f;
 
-    int step = 0, delta = 1;
+    int delta = 1;
+    int target = path.x, target2 = path.y;  // the element the ray reflects at next, and then
+    // rrel = max |xy| / height: an element whose ratio is below the maximum by more than the
+    // roundings (2^-20) is passed over by comparing squares; the others are evaluated exactly
+    float rrel2 = 0.0f;
     int lens_id, inter_id = 0;  // inter_id: loop steps so far (raytracing.cl:256)
     for (lens_id = 0; lens_id >= 0 && lens_id < E; lens_id += delta, inter_id++) {
         const SmemElement& e = se[lens_id];
@@ -255,39 +303,45 @@ __device__ __forceinline__ void trace_ray_rec(const SmemElement* __restrict__ se
             apt_y = h.py / e.height;
             continue;
         }
-        const float r_here = sqrtf(h.px * h.px + h.py * h.py) / e.height;
-        rec.rrel(r_here, rrel);
-        rrel = fmaxf(rrel, r_here);
-        if (lens_id == E - 1) continue;
-        bool do_reflect = false;
-        if ((step == 0 && lens_id == path.x) || (step == 1 && lens_id == path.y)) {
-            do_reflect = true;
-            step++;
-            delta = -delta;
+        const float xy2 = h.px * h.px + h.py * h.py;
+        if (!(xy2 < rrel2 * (e.height * e.height))) {
+            const float r_here = sqrtf(xy2) / e.height;
+            rec.rrel(r_here, rrel);
+            rrel = fmaxf(rrel, r_here);
+            rrel2 = rrel * rrel * (1.0f - 0x1p-20f);
         }
-        const int n_index = (dz < 0.0f) ? lens_id - 1 : lens_id + 1;
-        const float n1 = (0 <= n_index && n_index < E) ? ior_of(n_index) : 1.0f;
-        const float n2 = ior_of(lens_id);
-        if (do_reflect) {
+        if (lens_id == E - 1) continue;
+        if (lens_id == target) {
+            target = target2;
+            target2 = -1;
+            delta = -delta;
+            const int n_index = (dz < 0.0f) ? lens_id - 1 : lens_id + 1;
+            const float n1 = (0 <= n_index && n_index < E) ? ior_of(n_index) : 1.0f;
+            const float n2 = ior_of(lens_id);
             rec.reflect();
-            const float incident = incident_angle(dx, dy, dz, h);
+            const float c0 = incident_cos(dx, dy, dz, h), s0 = sqrt_rn((1.0f - c0) * (1.0f + c0));
             reflect_dir(dx, dy, dz, h);
-            // theta = incident + 1e-9 (a double sum there); only angles below 0.02 rad
-            // are close enough to 1e-9 for the double sum to differ from `incident`
-            float theta = incident < 0.02f ? (float)((double)incident + 1e-9) : incident;
             float reflectance;
             if (e.layers == 2) {
-                reflectance = fresnel_two_layer(theta, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
+                reflectance = fresnel_two_layer(c0, s0, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
             } else if (e.layers == 1 || e.coating > 0) {
                 float nc = fmaxf(sqrtf(n1 * n2), f.cmin);
                 float d1 = e.layers == 1 ? e.d0 : (float)e.coating / (4.0f * nc);
-                reflectance = fresnel_ar(theta, wavelength, d1, n1, nc, n2);
+                reflectance = fresnel_ar(c0, s0, wavelength, d1, n1, nc, n2);
             } else {
-                reflectance = fresnel(theta, n1, n2);
+                reflectance = fresnel(c0, s0, n1, n2);
             }
             if (reflectance > 0.0f) refl *= reflectance;
         } else {
-            refract_dir(dx, dy, dz, h, n1, n2);
+            float o;
+            if (ratio_row) {
+                const float2 q = ratio_row[lens_id];
+                o = dz < 0.0f ? q.x : q.y;
+            } else {
+                const int n_index = (dz < 0.0f) ? lens_id - 1 : lens_id + 1;
+                o = ((0 <= n_index && n_index < E) ? ior_of(n_index) : 1.0f) / ior_of(lens_id);
+            }
+            refract_dir(dx, dy, dz, h, o);
             if (dz == 0.0f) break;
         }
     }
@@ -300,18 +354,32 @@ __device__ __forceinline__ void trace_ray_rec(const SmemElement* __restrict__ se
     out[5] = refl;
 }
 
-__device__ __forceinline__ void trace_ray(const SmemElement* __restrict__ se, const float* ior_row, bool disperse,
+__device__ __forceinline__ void trace_ray(const SmemElement* __restrict__ se, const float* ior_row,
+                                          const float2* ratio_row, bool disperse,
                                           const float* __restrict__ coef_base, float wavelength, int2 path,
                                           float grid_x, float grid_y, const TraceFrame& f, float out[6]) {
     NoRecord none;
-    trace_ray_rec(se, ior_row, disperse, coef_base, wavelength, path, grid_x, grid_y, f, out, none);
+    trace_ray_rec(se, ior_row, ratio_row, disperse, coef_base, wavelength, path, grid_x, grid_y, f, out, none);
 }
 
-// Stage the lens elements and the refractive indices of wavelength rows [row0, row0 + span)
-// (row r = wavelength (row0 + r) % W) in shared memory; table false: too many rows.
+// Wavelength rows that kTraceThreads * rays consecutive rays can span, and the shared memory of
+// their tables (12 bytes per row and element); none past kMaxTableBytes.
+constexpr int kMaxTableBytes = 40 * 1024;
+__host__ __device__ inline int table_rows(long long rays, int R, int W) {
+    const long long rows = (rays + R - 2) / R + 1;
+    return (int)(rows < W ? rows : W);
+}
+inline size_t table_bytes(long long rays, int R, int W, int E) {
+    const size_t bytes = sizeof(IorEntry) * (size_t)table_rows(rays, R, W) * E;
+    return bytes <= kMaxTableBytes ? bytes : 0;
+}
+
+// Stage the lens elements and the refractive indices and ratios of wavelength rows [row0, row0 +
+// span) (row r = wavelength (row0 + r) % W) in shared memory; table false: too many rows. ior is
+// [span][E], ratio [span][E] after it.
 __device__ __forceinline__ void stage_lens(const rf_lens_element* __restrict__ elements, const float* __restrict__ wavelengths,
                                            int E, int W, long long row0, int span, bool table, bool disperse,
-                                           SmemElement* se, float* ior_tab) {
+                                           SmemElement* se, float2* ratio, float* ior) {
     for (int i = threadIdx.x; i < E; i += kTraceThreads) {
         const rf_lens_element& e = elements[i];
         se[i].radius = e.radius;
@@ -329,7 +397,13 @@ __device__ __forceinline__ void stage_lens(const rf_lens_element* __restrict__ e
             int wl = (int)((row0 + row) % W);
             float n = elements[el].ior;
             if (disperse && n > 1.0f) n = dispersion(wavelengths[wl], elements[el].coefficients);
-            ior_tab[row * E + el] = n;
+            ior[row * E + el] = n;
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < span * E; k += kTraceThreads) {
+            const int row = k / E, el = k % E;
+            const IorEntry r = ior_entry(el, E, [&](int i) { return ior[row * E + i]; });
+            ratio[k] = make_float2(r.down, r.up);
         }
     }
 }
