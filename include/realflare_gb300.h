@@ -100,6 +100,13 @@ long long rf_launch_count(void);
 int rf_trace(const rf_lens_element* elements, const int32_t* paths, const float* wavelengths,
              const rf_trace_args* args, float* rays, void* stream);
 
+/* rf_trace with the reflectances evaluated from the incidence angle, operation by operation as the
+ * reference writes them (raytracing.cl:1-59) and as rf_trace_adjoint differentiates them:
+ * the forward trace of a differentiated render. The other outputs are rf_trace's bit for bit,
+ * the reflectance differs in its last bits. */
+int rf_trace_differentiable(const rf_lens_element* elements, const int32_t* paths, const float* wavelengths,
+                            const rf_trace_args* args, float* rays, void* stream);
+
 /* rf_trace with the ray geometry in double precision (an opt-in accurate mode; the same
  * kernel of realflare/api/tasks/cl/raytracing.cl:218-359, the same arguments and layout).
  * Grid point, light direction, intersect (raytracing.cl:123-175), refract and reflect

@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kAdjThreads, RF_ADJOINT_MIN_BLOCKS) k_trace_ad
         CheckpointRecorder rec{checkpoints, tags, 0, -1, 0.0f};
         float out[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (needed)
-            trace_ray_rec(se, ior_row, nullptr, disperse, coef_base, wavelength, __ldg(paths + path_id), p.grid[gx], p.grid[gy],
+            trace_ray_rec<true>(se, ior_row, nullptr, disperse, coef_base, wavelength, __ldg(paths + path_id), p.grid[gx], p.grid[gy],
                           f, out, rec);
         const bool valid = needed && !isnan(out[5]) && rec.n <= kAdjMaxSteps && rec.n > 0;
         const unsigned vmask = __ballot_sync(0xffffffffu, valid);

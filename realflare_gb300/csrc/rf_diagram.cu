@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_intersections(const rf_
     const int gx = ray_id - gy * p.G;
     IntersectionRecorder rec{inter + idx * count, count};
     float out[6];
-    trace_ray_rec(se, nullptr, nullptr, disperse, &elements[0].coefficients[0], __ldg(wavelengths + wl_id),
+    trace_ray_rec<false>(se, nullptr, nullptr, disperse, &elements[0].coefficients[0], __ldg(wavelengths + wl_id),
                   __ldg(paths + path_id), p.grid[gx], p.grid[gy], f, out, rec);
     const long long n = p.n_rays;
 #pragma unroll

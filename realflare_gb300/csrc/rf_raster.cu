@@ -114,36 +114,32 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // 16-byte shared-memory loads that yield two register pairs. Values of the four corners are
 // stored even corners first (0, 2, 1, 3), so that one packed operation serves corners 0 and 2
 // (or edges 0 and 2) and the next one corners 1 and 3, without register moves. Records are
-// 272 bytes apart (17 x 16): where the lanes of a warp read 32 different records at one offset
+// 240 bytes apart (15 x 16): where the lanes of a warp read 32 different records at one offset
 // (the block selection), each group of 8 lanes then reads 8 different 16-byte bank groups
 // instead of one.
 struct alignas(16) Rec {
     int bb[4];       // xmin, xmax, ymin, ymax
     float col[4];    // the record's XYZ weight (1, 1, 1 with one wavelength); [3]: 0 when the housing
                      // falloff is 1 and no clamp acts on any covered pixel (inside_housing), else 1
-    float xy[8];     // corner positions relative to the tile, exact floats: x0 x2, x1 x3, y0 y2, y1 y3
+    float xy[12];    // corner positions relative to the tile, exact floats: x0 x2, x1 x3, y0 y2, y1 y3,
+                     // x2 x0, y2 y0
     float uv[8];     // ghost texel coordinates: u0 u2, u1 u3, v0 v2, v1 v3, see store_corner
     float rs[4];     // (rrel - 1) / (0.95 - 1): smoothstep(1, 0.95, rrel)'s ramp before clamping
     float inten[4], refl[4];
-    // edge functions A y + B x + C in samples relative to the tile (exact, see finish_record):
-    float ab[8];     // A of edges 01 23, B 01 23, A 12 30, B 12 30
-    float c[4];      // C of edges 01 23 12 30
-    float cb[4];     // C with the top-left bias
-    float e20[3];    // A, B, biased C of edge 20
-    int flags;       // 1: bounds rejection and ab, cb, e20 are exact; 2: adds nothing (collinear, or zero_record)
-    float nl2[4];    // minus the squared lengths of edges 01 23 12 30; NaN: the weights take special_weights
-    float ext[4];    // edges 01 23 12 30: half the edge function's range over a block
-    float pad[4];    // the stride
-    // mixed vertex positions, sample space (x0, y0, ..., x3, y3): in ab's place while the record is
-    // built, and for good where the edge functions are not exact (flags & 1 clear)
-    __device__ __forceinline__ int* q() { return reinterpret_cast<int*>(ab); }
-    __device__ __forceinline__ const int* q() const { return reinterpret_cast<const int*>(ab); }
+    // biased edge functions A y + B x + C in samples relative to the tile (exact, see finish_record):
+    // A of edges 01 12, B 01 12, C 01 12, A 23 30, B 23 30, C 23 30, then A B C of edge 20
+    float ef[15];
+    int flags;       // 1: bounds rejection and ef are exact; 2: adds nothing (collinear, or zero_record)
+    float ext[4];    // edges 01 12 23 30: half the edge function's range over a block
+    // mixed vertex positions, sample space (x0, y0, ..., x3, y3): in ef's place while the record is
+    // built, and for good where ef is not exact (flags & 1 clear)
+    __device__ __forceinline__ int* q() { return reinterpret_cast<int*>(ef); }
+    __device__ __forceinline__ const int* q() const { return reinterpret_cast<const int*>(ef); }
 };
-static_assert(sizeof(Rec) == 272 && offsetof(Rec, bb) == 0 && offsetof(Rec, col) % 16 == 0 &&
+static_assert(sizeof(Rec) == 240 && offsetof(Rec, bb) == 0 && offsetof(Rec, col) % 16 == 0 &&
                   offsetof(Rec, xy) % 16 == 0 && offsetof(Rec, uv) % 16 == 0 && offsetof(Rec, rs) % 16 == 0 &&
-                  offsetof(Rec, inten) % 16 == 0 && offsetof(Rec, refl) % 16 == 0 && offsetof(Rec, ab) % 16 == 0 &&
-                  offsetof(Rec, c) % 16 == 0 && offsetof(Rec, cb) % 16 == 0 && offsetof(Rec, e20) % 16 == 0 &&
-                  offsetof(Rec, flags) == offsetof(Rec, e20) + 12 && offsetof(Rec, nl2) % 16 == 0 &&
+                  offsetof(Rec, inten) % 16 == 0 && offsetof(Rec, refl) % 16 == 0 &&
+                  offsetof(Rec, ef) % 16 == 0 && offsetof(Rec, flags) == offsetof(Rec, ef) + 15 * sizeof(int) &&
                   offsetof(Rec, ext) % 16 == 0,
               "records are read with 16-byte loads");
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -206,24 +202,25 @@ __device__ __forceinline__ unsigned outside_sign(unsigned n01, unsigned n12, uns
     return (~n20 & x1) | (n20 & x0);
 }
 
-// A record's biased edge functions in registers.
+// A record's edge functions in registers.
 struct Edges {
-    f2 a0, b0, c0, a1, b1, c1;  // edges (01, 23) and (12, 30)
+    f2 a0, b0, c0, a1, b1, c1;  // edges (01, 12) and (23, 30)
     float a20, b20, c20;
+    int flags;
 };
 __device__ __forceinline__ void load_edges(const Rec& r, Edges& e) {
-    ld2(r.ab, e.a0, e.b0);
-    ld2(r.ab + 4, e.a1, e.b1);
-    ld2(r.cb, e.c0, e.c1);
-    const float4 d = ld4(r.e20);
-    e.a20 = d.x, e.b20 = d.y, e.c20 = d.z;
+    ld2(r.ef, e.a0, e.b0);
+    ld2(r.ef + 4, e.c0, e.a1);
+    ld2(r.ef + 8, e.b1, e.c1);
+    const float4 d = ld4(r.ef + 12);
+    e.a20 = d.x, e.b20 = d.y, e.c20 = d.z, e.flags = __float_as_int(d.w);
 }
 // The sample at tile-relative coordinates x = (x, x), y = (y, y), for records with flags & 1: the
 // edge values are exact integers (an exact zero is +0), so their signs are the reference's.
 __device__ __forceinline__ bool inside(const Edges& e, f2 x, f2 y) {
     const f2 e0 = fma2(e.a0, y, fma2(e.b0, x, e.c0)), e1 = fma2(e.a1, y, fma2(e.b1, x, e.c1));
     const float e2 = fmaf(e.a20, lo2(y), fmaf(e.b20, lo2(x), e.c20));
-    return (int)outside_sign((unsigned)e0, (unsigned)e1, (unsigned)(e0 >> 32), (unsigned)(e1 >> 32),
+    return (int)outside_sign((unsigned)e0, (unsigned)(e0 >> 32), (unsigned)e1, (unsigned)(e1 >> 32),
                              __float_as_uint(e2)) >= 0;
 }
 
@@ -246,101 +243,111 @@ __device__ __forceinline__ int rect_coverage(const Rec& r, f2 xc, f2 yc, float h
     const unsigned mixed = ((unsigned)l0 & ~(unsigned)h0) | ((unsigned)(l0 >> 32) & ~(unsigned)(h0 >> 32)) |
                            ((unsigned)l1 & ~(unsigned)h1) | ((unsigned)(l1 >> 32) & ~(unsigned)(h1 >> 32)) |
                            (l2 & ~h2);
-    const unsigned out = outside_sign((unsigned)l0, (unsigned)l1, (unsigned)(l0 >> 32), (unsigned)(l1 >> 32), l2);
+    const unsigned out = outside_sign((unsigned)l0, (unsigned)(l0 >> 32), (unsigned)l1, (unsigned)(l1 >> 32), l2);
     return (int)mixed < 0 ? 1 : ((int)out < 0 ? 0 : 2);
 }
 
-// Mean-value weights (compute_barycentric_quad, rasterizing.cl:95-148) at a sample point p. With
-// s_i = q_i - p, r_i = |s_i|, a_i = s_i x s_j, d_i = s_i . s_j (j the next corner), the reference's
-// weight is (t_{i-1} + t_i) / r_i, t_i = (r_i r_j - d_i) / a_i, normalised by the weights' sum.
-// Two identities save the products: a_i is minus edge ij's function at p, which is exact here
-// (integers below 2^24; records where it is not take special_weights), and
-// r_i r_j - d_i = (L^2 - (r_i - r_j)^2) / 2 with the edge's length L, which also loses fewer digits
-// than the difference of two products of the size of r^2. The common factors (-1, 2) cancel in
-// the normalisation. Reciprocals and reciprocal square roots are the approximate instructions (a
-// few ulps).
+// Mean-value weights (compute_barycentric_quad, rasterizing.cl:95-148) at the integer
+// sample point (px, py), relative to the tile. The coordinates s_i = q_i - p are exact floats; the
+// products a_i, d_i, |s_i|^2 are exact integers wherever |s| < 4096, so fused multiply-adds give
+// the reference's values there. Where a_i is 0 the reference divides the rounding residue
+// of r_i r_j - d_i by 1e-3: that tangent is evaluated with the reference's exact FP32
+// operations (correctly rounded square roots, product, difference, quotient). Elsewhere
+// the tangents and the divisions by r_i and by the weight sum use reciprocal and
+// reciprocal-square-root instructions (a few ulps).
 //
-// Positions are relative to the tile; px is (x, x), py the (y, y) of kN pixels in one column, whose
-// chains run side by side and share the terms in x. Corners 0 and 2 and corners 1 and 3 go
-// through packed operations. Returns the weights of corners (0, 2) in we and (1, 3) in wo for the
-// pixels marked in `need`, and sets `general` where they may have mixed signs inside a convex quad
-// (the special cases).
+// px is (x, x), py the (y, y) of kN pixels in one column, whose chains run side by side and share
+// the terms in x. Corners 0 and 2 and corners 1 and 3 go through packed operations; the cross
+// products' second terms are formed from negated odd corners (p - q instead of q - p), because a
+// packed fused multiply-add cannot negate an operand. Returns the weights of corners (0, 2) in we
+// and (1, 3) in wo for the pixels marked in `need`, and sets `general` where they may have mixed
+// signs inside a convex quad (the special cases).
+struct CornerTerms {  // in x, shared by the pixels of a column
+    f2 xe, xs, nxo, xe_nxo, xs_nxo, xe_xe, xo_xo, qye, qyo, qys;
+    __device__ __forceinline__ CornerTerms(const Rec& rec, f2 px) {
+        f2 qxe, qxo, qxs;
+        ld2(rec.xy, qxe, qxo);
+        ld2(rec.xy + 4, qye, qyo);
+        ld2(rec.xy + 8, qxs, qys);
+        xe = sub2(qxe, px), xs = sub2(qxs, px), nxo = sub2(px, qxo);
+        xe_nxo = mul2(xe, nxo), xs_nxo = mul2(xs, nxo), xe_xe = mul2(xe, xe), xo_xo = mul2(nxo, nxo);
+    }
+};
+template <int kN>
+struct PixelTerms {
+    f2 a02, na13, nd02, nd13, r2e, r2o, ire, iro, t02, nt13;  // a0 a2, -a1 -a3, -d0 -d2, -d1 -d3, ...
+    __device__ __forceinline__ PixelTerms(const CornerTerms& c, f2 py) {
+        const f2 ye = sub2(c.qye, py), ys = sub2(c.qys, py), yo = sub2(c.qyo, py), nyo = sub2(py, c.qyo);
+        a02 = fma2(c.xe, yo, mul2(c.nxo, ye));
+        na13 = fma2(c.xs, yo, mul2(c.nxo, ys));
+        if (kN > 1) {  // the products in x are shared
+            nd02 = fma2(ye, nyo, c.xe_nxo), nd13 = fma2(ys, nyo, c.xs_nxo);
+            r2e = fma2(ye, ye, c.xe_xe), r2o = fma2(yo, yo, c.xo_xo);
+        } else {  // several samples per pixel, where |s| >= 4096 is less rare: the scalar form's roundings
+            nd02 = fma2(c.xe, c.nxo, mul2(ye, nyo)), nd13 = fma2(c.xs, c.nxo, mul2(ys, nyo));
+            r2e = fma2(c.xe, c.xe, mul2(ye, ye)), r2o = fma2(c.nxo, c.nxo, mul2(yo, yo));
+        }
+        ire = pk(rsqrtf(lo2(r2e)), rsqrtf(hi2(r2e))), iro = pk(rsqrtf(lo2(r2o)), rsqrtf(hi2(r2o)));
+        const f2 re = mul2(r2e, ire), ro = mul2(r2o, iro);
+        const f2 n02 = fma2(re, ro, nd02);
+        const f2 n13 = pk(fmaf(lo2(ro), hi2(re), lo2(nd13)), fmaf(hi2(ro), lo2(re), hi2(nd13)));
+        t02 = mul2(n02, pk(rcp_approx(lo2(a02)), rcp_approx(hi2(a02))));
+        nt13 = mul2(n13, pk(rcp_approx(lo2(na13)), rcp_approx(hi2(na13))));
+    }
+};
 
 // The weights where the common form failed: a vertex on the sample point, an edge's line through
 // it (that tangent in the reference's exact operations), or a weight sum of 0, infinity or NaN
 // (normalised weights would be infinite or NaN, their intensity and reflectance NaN or 0 and so
 // the clamped products 0).
-__device__ __forceinline__ void special_weights(const Rec& rec, float px, float py, f2& we, f2& wo) {
-    float sx[4], sy[4], r2[4], ir[4], t[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int k = corner_slot(i);
-        sx[i] = rec.xy[k] - px;
-        sy[i] = rec.xy[4 + k] - py;
-        r2[i] = sx[i] * sx[i] + sy[i] * sy[i];
-        ir[i] = rsqrtf(r2[i]);
-    }
+template <int kN>
+__device__ __forceinline__ void special_weights(const Rec& rec, f2 px, f2 py, f2& we, f2& wo) {
+    // (evaluated anew, not kept live from the common form: the empty asm hides that they are the same)
+    asm("" : "+l"(px), "+l"(py));
+    const PixelTerms<kN> p(CornerTerms(rec, px), py);
+    const float r2[4] = {lo2(p.r2e), lo2(p.r2o), hi2(p.r2e), hi2(p.r2o)};
     if (r2[0] == 0.0f || r2[1] == 0.0f || r2[2] == 0.0f || r2[3] == 0.0f) {  // one-hot on the first such vertex
         const int k = r2[0] == 0.0f ? 0 : (r2[1] == 0.0f ? 1 : (r2[2] == 0.0f ? 2 : 3));
         we = pk(k == 0 ? 1.0f : 0.0f, k == 2 ? 1.0f : 0.0f);
         wo = pk(k == 1 ? 1.0f : 0.0f, k == 3 ? 1.0f : 0.0f);
         return;
     }
+    const float a[4] = {lo2(p.a02), lo2(p.na13), hi2(p.a02), hi2(p.na13)};
+    const float nd[4] = {lo2(p.nd02), lo2(p.nd13), hi2(p.nd02), hi2(p.nd13)};
+    float t[4] = {lo2(p.t02), -lo2(p.nt13), hi2(p.t02), -hi2(p.nt13)};
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int j = (i + 1) & 3;
-        const float a = sx[i] * sy[j] - sx[j] * sy[i], d = sx[i] * sx[j] + sy[i] * sy[j];
-        if (a == 0.0f)
-            t[i] = __fdiv_rn(__fsub_rn(__fmul_rn(__fsqrt_rn(r2[i]), __fsqrt_rn(r2[j])), d), 1e-3f);
-        else
-            t[i] = ((r2[i] * ir[i]) * (r2[j] * ir[j]) - d) * rcp_approx(a);
-    }
-    we = mul2(pk(t[3] + t[0], t[1] + t[2]), pk(ir[0], ir[2]));
-    wo = mul2(pk(t[0] + t[1], t[2] + t[3]), pk(ir[1], ir[3]));
+    for (int i = 0; i < 4; i++)
+        if (a[i] == 0.0f)
+            t[i] = __fdiv_rn(__fadd_rn(__fmul_rn(__fsqrt_rn(r2[i]), __fsqrt_rn(r2[(i + 1) & 3])), nd[i]), 1e-3f);
+    we = mul2(pk(t[3] + t[0], t[1] + t[2]), p.ire);
+    wo = mul2(pk(t[0] + t[1], t[2] + t[3]), p.iro);
     const float sum = (lo2(we) + hi2(we)) + (lo2(wo) + hi2(wo)), inv = rcp_approx(sum);
-    const f2 inv2 = sum * inv > 0.5f ? pk(inv, inv) : 0;
-    we = inv2 ? mul2(we, inv2) : 0;
-    wo = inv2 ? mul2(wo, inv2) : 0;
+    const bool ok = sum * inv > 0.5f;
+    const f2 inv2 = pk(inv, inv);
+    we = ok ? mul2(we, inv2) : 0;
+    wo = ok ? mul2(wo, inv2) : 0;
 }
 
 template <int kN>
 __device__ __forceinline__ void mean_value_weights(const Rec& rec, f2 px, const f2 (&py)[kN], const bool (&need)[kN],
                                                    f2 (&we)[kN], f2 (&wo)[kN], float& general) {
-    f2 qxe, qxo, qye, qyo, a0, b0, a1, b1, c0, c1, nl0, nl1;
-    ld2(rec.xy, qxe, qxo);
-    ld2(rec.xy + 4, qye, qyo);
-    ld2(rec.ab, a0, b0);
-    ld2(rec.ab + 4, a1, b1);
-    ld2(rec.c, c0, c1);
-    ld2(rec.nl2, nl0, nl1);
-    const f2 xe = sub2(qxe, px), xo = sub2(qxo, px);
-    const f2 xe_xe = mul2(xe, xe), xo_xo = mul2(xo, xo);
-    c0 = fma2(b0, px, c0);
-    c1 = fma2(b1, px, c1);
-    // The common case first: when no a_i is 0 each |a_i| >= 1 and every term below is finite, so
-    // the weight sum is finite. An a_i of 0 makes t_i infinite or NaN, and a vertex on the sample
-    // point (r_i = 0) makes r_i NaN; either way sum * (1 / sum) is not near 1, and only then are
-    // the weights redone with the reference's special cases.
-    float inv[kN];
+    const CornerTerms c(rec, px);
+    // The common case first. a_i are integers (differences of products of integers): when
+    // none is 0 each |a_i| >= 1 and every term below is finite, so the weight sum is finite.
+    // An a_i of 0 makes t_i infinite or NaN, and a vertex on the sample point (r2_i = 0)
+    // makes r_i NaN; either way sum * (1 / sum) is not near 1, and only then are the weights
+    // redone with the reference's special cases.
     bool bad = false, ok[kN];
 #pragma unroll
     for (int i = 0; i < kN; i++) {
-        const f2 ye = sub2(qye, py[i]), yo = sub2(qyo, py[i]);
-        const f2 r2e = fma2(ye, ye, xe_xe), r2o = fma2(yo, yo, xo_xo);
-        const f2 a02 = fma2(a0, py[i], c0), a13 = fma2(a1, py[i], c1);  // -a0, -a2 and -a1, -a3
-        const f2 ire = pk(rsqrtf(lo2(r2e)), rsqrtf(hi2(r2e))), iro = pk(rsqrtf(lo2(r2o)), rsqrtf(hi2(r2o)));
-        const f2 re = mul2(r2e, ire), ro = mul2(r2o, iro);
-        const f2 g02 = sub2(re, ro), g13 = pk(lo2(ro) - hi2(re), hi2(ro) - lo2(re));  // r_i - r_j
-        const f2 t02 = mul2(fma2(g02, g02, nl0), pk(rcp_approx(lo2(a02)), rcp_approx(hi2(a02))));
-        const f2 t13 = mul2(fma2(g13, g13, nl1), pk(rcp_approx(lo2(a13)), rcp_approx(hi2(a13))));
-        wo[i] = mul2(add2(t02, t13), iro);                                            // w1, w3
-        we[i] = mul2(pk(lo2(t02) + hi2(t13), hi2(t02) + lo2(t13)), ire);              // w0, w2
+        const PixelTerms<kN> p(c, py[i]);
+        wo[i] = mul2(sub2(p.t02, p.nt13), p.iro);                                                   // w1, w3
+        we[i] = mul2(pk(lo2(p.t02) - hi2(p.nt13), hi2(p.t02) - lo2(p.nt13)), p.ire);                // w0, w2
         const f2 s2 = add2(we[i], wo[i]);
-        const float sum = lo2(s2) + hi2(s2);
-        inv[i] = rcp_approx(sum);
-        ok[i] = !need[i] || sum * inv[i] > 0.5f;
+        const float sum = lo2(s2) + hi2(s2), inv = rcp_approx(sum);
+        ok[i] = !need[i] || sum * inv > 0.5f;
         bad = bad || !ok[i];
-        const f2 inv2 = pk(inv[i], inv[i]);
+        const f2 inv2 = pk(inv, inv);
         we[i] = mul2(we[i], inv2);
         wo[i] = mul2(wo[i], inv2);
     }
@@ -348,7 +355,7 @@ __device__ __forceinline__ void mean_value_weights(const Rec& rec, f2 px, const 
         general = 1.0f;
 #pragma unroll
         for (int i = 0; i < kN; i++)
-            if (!ok[i]) special_weights(rec, lo2(px), lo2(py[i]), we[i], wo[i]);
+            if (!ok[i]) special_weights<kN>(rec, px, py[i], we[i], wo[i]);
     }
 }
 __device__ __forceinline__ void mean_value_weights(const Rec& rec, f2 px, f2 py, f2& we, f2& wo, float& general) {
@@ -472,13 +479,13 @@ __device__ __forceinline__ float fragment_fast(const Rec& r, f2 we, f2 wo, const
     return f[0];
 }
 
-__host__ __device__ inline FragmentConsts fragment_consts(const RasterParams& p) {
+__host__ __device__ inline FragmentConsts fragment_consts(const RasterParams& p, double shift = 1.0) {
     FragmentConsts fc;
     const double sx = 0.5 / p.ghost_scale * p.ghost_w, sy = 0.5 / p.ghost_scale * p.ghost_h;
     fc.tsx = (float)sx;
     fc.tsy = (float)sy;
-    fc.tox = (float)(0.5 * p.ghost_w - 1.0);
-    fc.toy = (float)(0.5 * p.ghost_h - 1.0);
+    fc.tox = (float)(0.5 * p.ghost_w - shift);
+    fc.toy = (float)(0.5 * p.ghost_h - shift);
     return fc;
 }
 
@@ -520,8 +527,13 @@ __device__ __forceinline__ void store_corner(const CornerLoad& c, int k, float t
     const int qx = cvt_rz_sat(px * (float)S), qy = cvt_rz_sat(py * (float)S);
     r.q()[2 * k] = qx;
     r.q()[2 * k + 1] = qy;
-    r.xy[s] = (float)qx - ox;
-    r.xy[4 + s] = (float)qy - oy;
+    const float x = (float)qx - ox, y = (float)qy - oy;
+    r.xy[s] = x;
+    r.xy[4 + s] = y;
+    if (!(k & 1)) {  // the even corners again, swapped
+        r.xy[8 + (s ^ 1)] = x;
+        r.xy[10 + (s ^ 1)] = y;
+    }
 }
 // Whether every fragment of a record is zero, so that shading it adds nothing:
 //  - a corner's reflectance is NaN (a ray that failed, at either wavelength of the pair):
@@ -581,8 +593,7 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
     const bool safe = p.safe_screen && bb.x >= -lim && bb.y <= lim && bb.z >= -lim && bb.w <= lim &&
                       (p.S < 8 || (bb.y - bb.x < 16384 && bb.w - bb.z < 16384));
     const float hx = 4.0f * (float)p.S - 0.5f, hy = 0.5f * kRows * (float)p.S - 0.5f;
-    float ea[5], eb[5], ec[5], ecb[5];
-    bool small = safe;  // the unbiased edge functions too are exact over the tile
+    float ea[5], eb[5], ecl[5];
 #pragma unroll
     for (int k = 0; k < 5; k++) {
         const int a = k < 4 ? k : 2, b = k < 4 ? (k + 1) & 3 : 0;
@@ -591,10 +602,7 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
         const int c = wadd(e[2], wadd(wmul(e[0], oy), wmul(e[1], ox)));
         ea[k] = (float)e[0];
         eb[k] = (float)e[1];
-        ecb[k] = (float)min(max(c, -8388608), 8388608);
-        const int cu = c + (top_left(q[2 * a], q[2 * a + 1], q[2 * b], q[2 * b + 1]) ? 0 : 1);
-        ec[k] = (float)cu;
-        if (k < 4) small = small && cu <= 8388608 && cu >= -8388608;
+        ecl[k] = (float)min(max(c, -8388608), 8388608);
     }
     int flags = safe ? 1 : 0;
     const bool collinear = edge_i(q[0], q[1], q[2], q[3], q[4], q[5]) == 0 &&
@@ -619,21 +627,16 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
         col.x = c[0], col.y = c[1], col.z = c[2];
     }
     *reinterpret_cast<float4*>(r.col) = col;
+    float4* ef = reinterpret_cast<float4*>(r.ef);
     if (safe) {  // else q stays
-        *reinterpret_cast<float4*>(r.ab) = make_float4(ea[0], ea[2], eb[0], eb[2]);
-        *reinterpret_cast<float4*>(r.ab + 4) = make_float4(ea[1], ea[3], eb[1], eb[3]);
+        ef[0] = make_float4(ea[0], ea[1], eb[0], eb[1]);
+        ef[1] = make_float4(ecl[0], ecl[1], ea[2], ea[3]);
+        ef[2] = make_float4(eb[2], eb[3], ecl[2], ecl[3]);
     }
-    *reinterpret_cast<float4*>(r.c) = make_float4(ec[0], ec[2], ec[1], ec[3]);
-    *reinterpret_cast<float4*>(r.cb) = make_float4(ecb[0], ecb[2], ecb[1], ecb[3]);
-    *reinterpret_cast<float4*>(r.e20) = make_float4(ea[4], eb[4], ecb[4], __int_as_float(flags));
-    float l2[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) l2[k] = small ? -(ea[k] * ea[k] + eb[k] * eb[k]) : __int_as_float(0x7fffffff);
-    *reinterpret_cast<float4*>(r.nl2) = make_float4(l2[0], l2[2], l2[1], l2[3]);
-    float x[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) x[k] = fabsf(ea[k]) * hy + fabsf(eb[k]) * hx;
-    *reinterpret_cast<float4*>(r.ext) = make_float4(x[0], x[2], x[1], x[3]);
+    ef[3] = make_float4(ea[4], eb[4], ecl[4], __int_as_float(flags));
+    *reinterpret_cast<float4*>(r.ext) =
+        make_float4(fabsf(ea[0]) * hy + fabsf(eb[0]) * hx, fabsf(ea[1]) * hy + fabsf(eb[1]) * hx,
+                    fabsf(ea[2]) * hy + fabsf(eb[2]) * hx, fabsf(ea[3]) * hy + fabsf(eb[3]) * hx);
 }
 
 // How many of the S n-rook samples of this lane's pixel a record covers. (rx0, ry0): the block's first
@@ -784,7 +787,7 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
                 bool take = false, all = false, far = false;
                 if (j < n_rec) {
                     const Rec& r = recs[j];
-                    const int flags = __float_as_int(ld4(r.e20).w);  // with e20, which rect_coverage reads
+                    const int flags = __float_as_int(ld4(r.ef + 12).w);  // with ef[12..14], which rect_coverage reads
                     if (!(flags & 2)) {  // collinear (intersect_quad rejects all) or all-zero
                         const int4 bb = *reinterpret_cast<const int4*>(r.bb);
                         far = !(flags & 1);
@@ -969,8 +972,10 @@ constexpr int kPixels = kS != 1 ? 1 : (T == 32 ? RF_RASTER_PIX32 : RF_RASTER_PIX
 //   90.2 / 3.22 / 21.5 ms  two pixels of a column per lane (one sample per pixel): a record's
 //                          loads, loop and x terms serve both, and their chains overlap; next
 //                          batch's vertices not held in registers
-//   88.6 / 3.15 / 21.0 ms  cross products from the edge functions, products r_i r_j - d_i from the
-//                          edge lengths, texel origins without floors
+//   89.6 / 3.19 / 21.4 ms  texel origins without floors
+// (Cross products from the edge functions and r_i r_j - d_i from the edge lengths would be 88.6 /
+// 3.15 / 21.0 ms and lose fewer digits, but move single pixels of large quads by up to 2e-3 away
+// from the form below.)
 // One CTA per tile of a frame: CTA k shades tile order[k], or tile k without an order.
 // CTAs start in index order as slots free up, so an order by decreasing work starts the
 // heaviest tiles first and ends the launch with light ones.
@@ -988,7 +993,6 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : 
 }
 
 __host__ __device__ inline bool make_params(const rf_raster_args& a, RasterParams& p);
-__host__ __device__ inline FragmentConsts fragment_consts(const RasterParams& p);
 
 // Every frame of a batch in one persistent launch: each CTA takes the next tile from the
 // queue (tiles ordered by decreasing entry count) until none are left. kTex: every frame's
@@ -1040,12 +1044,78 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : 
 }
 
 // ---------------------------------------------------------------- adjoint
-// ghost_sample with its derivatives with respect to the texel coordinates.
+// The adjoint's fragment keeps one scalar operation per term in the corners' order (weights,
+// interpolations, floors): where gradients of opposite sign cancel (the light's above all), the
+// last bits of the terms show in the sums, and this form's are what its gradients have been
+// checked with.
+__device__ __forceinline__ void scalar_weights(const Rec& rec, float px, float py, float w[4]) {
+    float sx[4], sy[4], a[4], d[4], r2[4], ir[4], r[4], t[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int k = corner_slot(i);
+        sx[i] = rec.xy[k] - px;
+        sy[i] = rec.xy[4 + k] - py;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int j = (i + 1) & 3;
+        a[i] = sx[i] * sy[j] - sx[j] * sy[i];
+        d[i] = sx[i] * sx[j] + sy[i] * sy[j];
+        r2[i] = sx[i] * sx[i] + sy[i] * sy[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        ir[i] = rsqrtf(r2[i]);
+        r[i] = r2[i] * ir[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) t[i] = (r[i] * r[(i + 1) & 3] - d[i]) * __fdividef(1.0f, a[i]);
+#pragma unroll
+    for (int i = 0; i < 4; i++) w[i] = (t[(i + 3) & 3] + t[i]) * ir[i];
+    float sum = w[0] + w[1] + w[2] + w[3];
+    if (!(fabsf(sum) <= 3.40282347e38f)) {  // the special cases (special_weights)
+        bool zero = false;
+#pragma unroll
+        for (int i = 0; i < 4; i++) zero = zero || r2[i] == 0.0f;
+        if (zero) {
+            int k = 0;
+#pragma unroll
+            for (int i = 3; i >= 0; i--)
+                if (sx[i] == 0.0f && sy[i] == 0.0f) k = i;
+#pragma unroll
+            for (int i = 0; i < 4; i++) w[i] = i == k ? 1.0f : 0.0f;
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int j = (i + 1) & 3;
+            if (a[i] == 0.0f)
+                t[i] = __fdiv_rn(__fsub_rn(__fmul_rn(__fsqrt_rn(r2[i]), __fsqrt_rn(r2[j])), d[i]), 1e-3f);
+            else
+                t[i] = (r[i] * r[j] - d[i]) * __fdividef(1.0f, a[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) w[i] = (t[(i + 3) & 3] + t[i]) * ir[i];
+        sum = w[0] + w[1] + w[2] + w[3];
+    }
+    const float inv = __fdividef(1.0f, sum);
+#pragma unroll
+    for (int i = 0; i < 4; i++) w[i] *= inv;
+}
+__device__ __forceinline__ float scalar_blend(const float w[4], const float* v) {  // v: even corners first
+    const float4 q = ld4(v);
+    return w[0] * q.x + w[1] * q.z + w[2] * q.y + w[3] * q.w;
+}
+
+// ghost_sample with its derivatives with respect to the texel coordinates (u, v) = uv * size - 0.5.
 template <bool kTex>
-__device__ __forceinline__ float ghost_sample_grad(const float* __restrict__ tex, const RasterParams& p, f2 uv,
-                                                   float& du, float& dv) {
-    f2 centre, frac;
-    ghost_footprint(uv, centre, frac);
+__device__ __forceinline__ float ghost_sample_grad(const float* __restrict__ tex, const RasterParams& p, float u,
+                                                   float v, float& du, float& dv) {
+    du = dv = 0.0f;
+    if (!(fabsf(u) < 1e9f) || !(fabsf(v) < 1e9f)) return 0.0f;
+    const float fu = floorf(u), fv = floorf(v);
+    const float a = u - fu, b = v - fv;
+    const f2 centre = pk(fu + 1.0f, fv + 1.0f);
     float t00, t10, t01, t11;
     if (kTex) {
         const float4 g = tex2Dgather<float4>((cudaTextureObject_t)p.ghost_tex, lo2(centre), hi2(centre), 0);
@@ -1053,7 +1123,6 @@ __device__ __forceinline__ float ghost_sample_grad(const float* __restrict__ tex
     } else {
         ghost_texels(tex, p.ghost_w, p.ghost_h, centre, t00, t10, t01, t11);
     }
-    const float a = lo2(frac), b = hi2(frac);
     du = (1.0f - b) * (t10 - t00) + b * (t11 - t01);
     dv = (1.0f - a) * (t01 - t00) + a * (t11 - t10);
     return (1.0f - a) * (1.0f - b) * t00 + a * (1.0f - b) * t10 + (1.0f - a) * b * t01 + a * b * t11;
@@ -1226,7 +1295,7 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? 3 : 2)
                 bool take = false, all = false, far = false;
                 if (j < n_rec) {
                     const Rec& r = recs[j];
-                    const int flags = __float_as_int(ld4(r.e20).w);  // with e20, which rect_coverage reads
+                    const int flags = __float_as_int(ld4(r.ef + 12).w);  // with ef[12..14], which rect_coverage reads
                     if (!(flags & 2)) {  // collinear (intersect_quad rejects all) or all-zero
                         const int4 bb = *reinterpret_cast<const int4*>(r.bb);
                         far = !(flags & 1);
@@ -1258,22 +1327,17 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? 3 : 2)
                     float gw[kGradAttrs] = {0.f, 0.f, 0.f, 0.f, 0.f};
                     float wt[4] = {0.f, 0.f, 0.f, 0.f};
                     if (hits > 0) {
-                        f2 we, wo;
-                        const float cx = rx0 + (float)((lane & 7) * S + S / 2);
-                        const float cy = ry0 + (float)((lane >> 3) * S + S / 2);
-                        float general = 1.0f;
-                        mean_value_weights(r, pk(cx, cx), pk(cy, cy), we, wo, general);
-                        wt[0] = lo2(we), wt[1] = lo2(wo), wt[2] = hi2(we), wt[3] = hi2(wo);
+                        scalar_weights(r, rx0 + (float)((lane & 7) * S + S / 2), ry0 + (float)((lane >> 3) * S + S / 2), wt);
                         const float4 col = ld4(r.col);
                         const float dLdf = g0 * col.x + g1 * col.y + g2 * col.z;
-                        const float u = blend4(we, wo, r.uv), v = blend4(we, wo, r.uv + 4);
+                        const float u = scalar_blend(wt, r.uv), v = scalar_blend(wt, r.uv + 4);
                         float dgu, dgv;
-                        const float gi = ghost_sample_grad<kTex>(ghost, p, pk(u, v), dgu, dgv);
-                        const float st = __saturatef(blend4(we, wo, r.rs));
+                        const float gi = ghost_sample_grad<kTex>(ghost, p, u, v, dgu, dgv);
+                        const float st = __saturatef(scalar_blend(wt, r.rs));
                         const float ri = st * st * (3.0f - 2.0f * st);
                         const float dri = (st > 0.0f && st < 1.0f) ? 6.0f * st * (1.0f - st) * (1.0f / (0.95f - 1.0f))
                                                                   : 0.0f;
-                        const float ai_raw = blend4(we, wo, r.inten), ci_raw = blend4(we, wo, r.refl);
+                        const float ai_raw = scalar_blend(wt, r.inten), ci_raw = scalar_blend(wt, r.refl);
                         const float ai = fmaxf(ai_raw, 0.0f), ci = fmaxf(ci_raw, 0.0f);
                         const float H = (float)hits;
                         const float d = dLdf * H;
@@ -1384,7 +1448,9 @@ __global__ void __launch_bounds__(256) k_raster_masks(const float4* __restrict__
                     float f = 0.0f;
                     if (hits > 0) {
                         f2 we, wo;
-                        special_weights(r, (float)(sx0 + S / 2), (float)(sy0 + S / 2), we, wo);
+                        const float cx = (float)(sx0 + S / 2), cy = (float)(sy0 + S / 2);
+                        float general = 1.0f;
+                        mean_value_weights(r, pk(cx, cx), pk(cy, cy), we, wo, general);
                         f += fragment_fast(r, we, wo, ghost, p, 1.0f) * (float)hits;
                     }
                     if (p.W > 1) {
@@ -1692,7 +1758,7 @@ extern "C" int rf_raster_backward(const float* vertexes, const uint32_t* tile_of
                         sizeof(float) * (3 * p.maxW * p.WS + ((p.WS + 3) & ~3)) +
                         sizeof(float) * (96 * (T * T / 32) + 2 * kBatchRecords * 4 * kGradAttrs +
                                          8 * kRedRows * kRedStride);
-    const FragmentConsts fc = fragment_consts(p);
+    const FragmentConsts fc = fragment_consts(p, 0.5);  // texel coordinates without ghost_footprint's shift
     const float4 *im = (const float4*)image, *gim = (const float4*)grad_image;
     const unsigned grid = (unsigned)(p.ntx * nty);
     p.ghost_tex = ghost_texture_object(ghost, p.ghost_w, p.ghost_h);

@@ -29,6 +29,7 @@
 namespace rf {
 namespace {
 
+template <bool kAngles>
 __global__ void __launch_bounds__(kTraceThreads) k_trace(const rf_lens_element* __restrict__ elements,
                                                          const int2* __restrict__ paths,
                                                          const float* __restrict__ wavelengths,
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const rf_lens_element* 
         const int gy = (int)truncf((float)ray_id / (float)p.G);
         const int gx = ray_id - gy * p.G;
         float out[6];
-        trace_ray(se, table ? ior_tab + row * E : nullptr, table ? ratio_tab + row * E : nullptr, disperse,
+        trace_ray<kAngles>(se, table ? ior_tab + row * E : nullptr, table ? ratio_tab + row * E : nullptr, disperse,
                   &elements[0].coefficients[0], __ldg(wavelengths + wl_id), __ldg(paths + path_id), p.grid[gx],
                   p.grid[gy], f, out);
 #pragma unroll
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_batch(const rf_frame* _
         const int gy = (int)truncf((float)ray_id / (float)f.G);
         const int gx = ray_id - gy * f.G;
         float out[6];
-        trace_ray(se, table ? ior_tab + row * f.E : nullptr, table ? ratio_tab + row * f.E : nullptr, disperse,
+        trace_ray<false>(se, table ? ior_tab + row * f.E : nullptr, table ? ratio_tab + row * f.E : nullptr, disperse,
                   &elements[0].coefficients[0],
                   __ldg(wavelengths + wl_id), __ldg(paths + path_id), grid[gx], grid[gy], f, out);
 #pragma unroll
@@ -161,8 +162,10 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_batch(const rf_frame* _
 }  // namespace
 }  // namespace rf
 
-extern "C" int rf_trace(const rf_lens_element* elements, const int32_t* paths, const float* wavelengths,
-                        const rf_trace_args* args, float* rays, void* stream) {
+namespace {
+template <bool kAngles>
+int trace_entry(const rf_lens_element* elements, const int32_t* paths, const float* wavelengths,
+                const rf_trace_args* args, float* rays, void* stream) {
     using namespace rf;
     if (!elements || !paths || !wavelengths || !args || !rays) return RF_ERR_INVALID_ARG;
     const rf_trace_args& a = *args;
@@ -182,9 +185,21 @@ extern "C" int rf_trace(const rf_lens_element* elements, const int32_t* paths, c
     while (rays_per_thread > 1 && p.n_rays < (long long)rays_per_thread * kTraceThreads * sms * 48) rays_per_thread /= 2;
     const long long chunk = (long long)kTraceThreads * rays_per_thread;
     const size_t table = table_bytes(chunk, p.R, p.W, p.E);
-    k_trace<<<blocks_for(p.n_rays, (int)chunk), kTraceThreads, table, (cudaStream_t)stream>>>(
+    k_trace<kAngles><<<blocks_for(p.n_rays, (int)chunk), kTraceThreads, table, (cudaStream_t)stream>>>(
         elements, (const int2*)paths, wavelengths, p, table > 0, rays_per_thread, rays);
     return launch_status();
+}
+}  // namespace
+
+extern "C" int rf_trace(const rf_lens_element* elements, const int32_t* paths, const float* wavelengths,
+                        const rf_trace_args* args, float* rays, void* stream) {
+    return trace_entry<false>(elements, paths, wavelengths, args, rays, stream);
+}
+
+extern "C" int rf_trace_differentiable(const rf_lens_element* elements, const int32_t* paths,
+                                       const float* wavelengths, const rf_trace_args* args, float* rays,
+                                       void* stream) {
+    return trace_entry<true>(elements, paths, wavelengths, args, rays, stream);
 }
 
 extern "C" int rf_trace_batch(const rf_frame* frames, const rf_batch_sizes* sizes, const rf_lens_element* elements,

@@ -184,6 +184,75 @@ __device__ RF_CORE_COLD float fresnel_two_layer(float c0, float s0, float lambda
     return (stack_r2(rs01, rs12, rs23, sd1, cd1, sd2, cd2) + stack_r2(rp01, rp12, rp23, sd1, cd1, sd2, cd2)) / 2.0f;
 }
 
+// The same reflectances evaluated from the incidence angle, operation by operation as the reference
+// writes them and as the adjoint's duals differentiate them. The adjoint's re-trace and the
+// forward trace of a differentiated render use these: where a gradient is a small difference of
+// large terms (the light's), the reflectances' last bits show in it.
+__device__ RF_CORE_COLD float fresnel_angle(float theta0, float n1, float n2) {
+    float theta1 = asinf(sinf(theta0) * n1 / n2);
+    float cosi = cosf(theta0);
+    float cost = cosf(theta1);
+    float rs = ((n1 * cosi) - (n2 * cost)) / ((n1 * cosi) + (n2 * cost));
+    float rp = ((n1 * cost) - (n2 * cosi)) / ((n1 * cost) + (n2 * cosi));
+    return (rs * rs + rp * rp) / 2.0f;
+}
+
+__device__ RF_CORE_COLD float fresnel_ar_angle(float theta0, float lambda, float d1, float n0, float n1, float n2) {
+    float s0 = sinf(theta0);
+    float theta1 = asinf(s0 * n0 / n1);
+    float theta2 = asinf(s0 * n0 / n2);
+    float rs01 = -sinf(theta0 - theta1) / sinf(theta0 + theta1);
+    float rp01 = tanf(theta0 - theta1) / tanf(theta0 + theta1);
+    float ts01 = 2.0f * sinf(theta1) * cosf(theta0) / sinf(theta0 + theta1);
+    float tp01 = ts01 * cosf(theta0 - theta1);
+    float rs12 = -sinf(theta1 - theta2) / sinf(theta1 + theta2);
+    float rp12 = tanf(theta1 - theta2) / tanf(theta1 + theta2);
+    float ris = ts01 * ts01 * rs12;
+    float rip = tp01 * tp01 * rp12;
+    float dy = d1 * n1;
+    float dx = tanf(theta1) * dy;
+    float delay = sqrtf(dx * dx + dy * dy);
+    float rel_phase = 4.0f * RF_MPI_F / lambda * (delay - dx * s0);
+    float c = cosf(rel_phase);
+    float out_s2 = rs01 * rs01 + ris * ris + 2.0f * rs01 * ris * c;
+    float out_p2 = rp01 * rp01 + rip * rip + 2.0f * rp01 * rip * c;
+    return (out_s2 + out_p2) / 2.0f;
+}
+
+__device__ __forceinline__ void interface_r_div(float ni, float ci, float nj, float cj, float& rs, float& rp) {
+    rs = (ni * ci - nj * cj) / (ni * ci + nj * cj);
+    rp = (nj * ci - ni * cj) / (nj * ci + ni * cj);
+}
+__device__ __forceinline__ float stack_r2_div(float r01, float r12, float r23, float d1, float d2) {
+    float s2, c2, s1, c1;
+    sincosf(d2, &s2, &c2);
+    sincosf(d1, &s1, &c1);
+    float nre = r12 + r23 * c2, nim = r23 * s2;
+    float dre = 1.0f + r12 * r23 * c2, dim = r12 * r23 * s2;
+    float den = dre * dre + dim * dim;
+    float ire = (nre * dre + nim * dim) / den;
+    float iim = (nim * dre - nre * dim) / den;
+    float ere = ire * c1 - iim * s1, eim = ire * s1 + iim * c1;
+    float tre = r01 + ere, tim = eim;
+    float bre = 1.0f + r01 * ere, bim = r01 * eim;
+    return (tre * tre + tim * tim) / (bre * bre + bim * bim);
+}
+__device__ RF_CORE_COLD float fresnel_two_layer_angle(float theta0, float lambda, float n0, float na, float da,
+                                                   float nb, float db, float n2) {
+    float s0, c0;
+    sincosf(theta0, &s0, &c0);
+    float sa = n0 * s0 / na, sb = n0 * s0 / nb, s2 = n0 * s0 / n2;
+    float ca = sqrtf(1.0f - sa * sa), cb = sqrtf(1.0f - sb * sb), c2 = sqrtf(1.0f - s2 * s2);
+    float rs01, rp01, rs12, rp12, rs23, rp23;
+    interface_r_div(n0, c0, na, ca, rs01, rp01);
+    interface_r_div(na, ca, nb, cb, rs12, rp12);
+    interface_r_div(nb, cb, n2, c2, rs23, rp23);
+    float phase = 4.0f * RF_MPI_F / lambda;
+    float d1 = phase * na * da * ca;
+    float d2 = phase * nb * db * cb;
+    return (stack_r2_div(rs01, rs12, rs23, d1, d2) + stack_r2_div(rp01, rp12, rp23, d1, d2)) / 2.0f;
+}
+
 // dispersion, raytracing.cl:107-120 (lambda * 1e-3 is a double expression there)
 __device__ __forceinline__ float dispersion(float lambda, const float* c) {
     float l = (float)((double)lambda * 1e-3);
@@ -255,8 +324,8 @@ __device__ __forceinline__ IorEntry ior_entry(int el, int E, IorOf ior_of) {
 // One ray: init_ray (raytracing.cl:178-215) from grid point (grid_x, grid_y), then the
 // element loop of raytrace (218-359). ior_row: this ray's wavelength row of the (wavelength,
 // element) index table in shared memory, or nullptr to evaluate dispersion per element.
-// ratio_row: the row's index ratios, or nullptr to divide.
-template <class Recorder>
+// ratio_row: the row's index ratios, or nullptr to divide. kAngles: the reflectances from angles.
+template <bool kAngles, class Recorder>
 __device__ __forceinline__ void trace_ray_rec(const SmemElement* __restrict__ se, const float* ior_row,
                                               const float2* ratio_row, bool disperse,
                                               const float* __restrict__ coef_base, float wavelength, int2 path,
@@ -319,18 +388,30 @@ __device__ __forceinline__ void trace_ray_rec(const SmemElement* __restrict__ se
             const float n1 = (0 <= n_index && n_index < E) ? ior_of(n_index) : 1.0f;
             const float n2 = ior_of(lens_id);
             rec.reflect();
-            const float c0 = incident_cos(dx, dy, dz, h), s0 = sqrt_rn((1.0f - c0) * (1.0f + c0));
-            reflect_dir(dx, dy, dz, h);
+            const float nc = fmaxf(sqrtf(n1 * n2), f.cmin);
+            const float d1 = e.layers == 1 ? e.d0 : (float)e.coating / (4.0f * nc);
             float reflectance;
-            if (e.layers == 2) {
-                reflectance = fresnel_two_layer(c0, s0, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
-            } else if (e.layers == 1 || e.coating > 0) {
-                float nc = fmaxf(sqrtf(n1 * n2), f.cmin);
-                float d1 = e.layers == 1 ? e.d0 : (float)e.coating / (4.0f * nc);
-                reflectance = fresnel_ar(c0, s0, wavelength, d1, n1, nc, n2);
+            if (kAngles) {
+                const float incident = incident_angle(dx, dy, dz, h);
+                // theta = incident + 1e-9 (a double sum there); only angles below 0.02 rad
+                // are close enough to 1e-9 for the double sum to differ from `incident`
+                const float theta = incident < 0.02f ? (float)((double)incident + 1e-9) : incident;
+                if (e.layers == 2)
+                    reflectance = fresnel_two_layer_angle(theta, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
+                else if (e.layers == 1 || e.coating > 0)
+                    reflectance = fresnel_ar_angle(theta, wavelength, d1, n1, nc, n2);
+                else
+                    reflectance = fresnel_angle(theta, n1, n2);
             } else {
-                reflectance = fresnel(c0, s0, n1, n2);
+                const float c0 = incident_cos(dx, dy, dz, h), s0 = sqrt_rn((1.0f - c0) * (1.0f + c0));
+                if (e.layers == 2)
+                    reflectance = fresnel_two_layer(c0, s0, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
+                else if (e.layers == 1 || e.coating > 0)
+                    reflectance = fresnel_ar(c0, s0, wavelength, d1, n1, nc, n2);
+                else
+                    reflectance = fresnel(c0, s0, n1, n2);
             }
+            reflect_dir(dx, dy, dz, h);
             if (reflectance > 0.0f) refl *= reflectance;
         } else {
             float o;
@@ -354,12 +435,13 @@ __device__ __forceinline__ void trace_ray_rec(const SmemElement* __restrict__ se
     out[5] = refl;
 }
 
+template <bool kAngles>
 __device__ __forceinline__ void trace_ray(const SmemElement* __restrict__ se, const float* ior_row,
                                           const float2* ratio_row, bool disperse,
                                           const float* __restrict__ coef_base, float wavelength, int2 path,
                                           float grid_x, float grid_y, const TraceFrame& f, float out[6]) {
     NoRecord none;
-    trace_ray_rec(se, ior_row, ratio_row, disperse, coef_base, wavelength, path, grid_x, grid_y, f, out, none);
+    trace_ray_rec<kAngles>(se, ior_row, ratio_row, disperse, coef_base, wavelength, path, grid_x, grid_y, f, out, none);
 }
 
 // Wavelength rows that kTraceThreads * rays consecutive rays can span, and the shared memory of

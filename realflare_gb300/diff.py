@@ -205,7 +205,7 @@ class DifferentiableRenderer:
         s = int(self.stream.cuda_stream)
         self.el = self._element_buffer(radius, center, thickness)
         self.targs = self._trace_args(direction)
-        trace = self.lib.rf_trace_accurate if self.accurate else self.lib.rf_trace
+        trace = self.lib.rf_trace_accurate if self.accurate else self.lib.rf_trace_differentiable
         check(trace(self.el.data_ptr(), self.paths.data_ptr(), self.wavelengths.data_ptr(),
                     ctypes.byref(self.targs), self.rays.data_ptr(), s), 'rf_trace')
         from .device import Rays
@@ -252,7 +252,7 @@ class DifferentiableRenderer:
         el = self._element_buffer(radius, center, thickness)
         targs = self._trace_args(direction)
         rays = empty((6, max(self.n_rays, 1)))
-        trace = self.lib.rf_trace_accurate if self.accurate else self.lib.rf_trace
+        trace = self.lib.rf_trace_accurate if self.accurate else self.lib.rf_trace_differentiable
         check(trace(el.data_ptr(), self.paths.data_ptr(), self.wavelengths.data_ptr(), ctypes.byref(targs),
                     rays.data_ptr(), s), 'rf_trace')
         return rays, el, targs
