@@ -172,9 +172,18 @@ __global__ void k_tile_offsets(const uint32_t* __restrict__ keys, long long n, i
     tile_offsets[t] = (uint32_t)lo;
 }
 
-// Raster tiles are 32 x 32 (default) or 16 x 16 pixels (rf_raster.cu); bins must be
-// multiples of the tile.
-__host__ __device__ inline int auto_tile(const rf_raster_args& a) { return a.tile_size > 0 ? a.tile_size : 32; }
+// Raster tiles are 32 x 32 or 16 x 16 pixels (rf_raster.cu); bins must be multiples of the tile.
+// Without a tile size in the arguments: 32, or 16 where an image has too few 32-pixel tiles to fill
+// the 152 SMs' 4 resident CTAs evenly (a tile's list is walked by one CTA). k_raster, 32- against
+// 16-pixel tiles: 512 x 512, 8 wavelengths (256 tiles) 2.83 / 1.21 ms; 800 x 800 (625) 2.67 / 2.38;
+// 900 x 900 (841) 2.89 / 2.94; 1024 x 1024 (1024) 3.18 / 3.57. With several samples per pixel the
+// per-entry work is small against the fragments' and the line lies higher: four samples 900 x 900
+// 4.00 / 3.59 ms, 1024 x 1024 4.51 / 4.32 ms.
+__host__ __device__ inline int auto_tile(const rf_raster_args& a) {
+    if (a.tile_size > 0) return a.tile_size;
+    const long long tiles = (long long)((a.width + 31) / 32) * ((a.height + 31) / 32);
+    return a.bin_size % 32 == 0 && tiles <= (a.sub_steps > 1 ? 1216 : 640) ? 16 : 32;
+}
 
 __host__ __device__ inline bool make_geometry(const rf_raster_args& a, BinGeometry& g) {
     if (a.width < 1 || a.height < 1 || a.bin_size < 1 || a.grid_count < 2 || a.wavelength_count < 1 ||
