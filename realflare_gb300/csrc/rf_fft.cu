@@ -1,22 +1,29 @@
 // rf_fft.cu — 2-D FFTs for the diffraction stages.
 //
-// A 2-D transform of a [batch][h][w] complex64 array is two passes of the same kernel:
-// each block loads one row into shared memory in bit-reversed order, runs the radix-2
-// decimation-in-time butterflies in place (twiddles from a per-block sincospi table), and
-// writes the row transposed ([batch][w][h]); the second pass transforms those rows and
-// transposes back, applying the normalisation. Pre- and post-operations of the two
-// callers are fused into the first load and the last store:
+// A 2-D transform of a [batch][h][w] complex64 array is a pass over rows and a pass over the
+// rows of the transposed result. A block holds a few rows in shared memory, each thread eight
+// elements of one row in registers: radix-8 steps (the last one 8, 4 or 2) in Stockham's
+// self-sorting order, so data stays in natural order and a row of 512 takes three exchanges
+// instead of nine. What the callers do before, between and after transforms happens in the
+// passes: a pass loads elements through a program, transforms, optionally multiplies and
+// transforms the same rows again, and stores through the program.
 //  * the starburst power spectrum (realflare/api/tasks/starburst.py:45-81): load
 //    A * exp(i pi (x^2 + y^2) / (lambda d)), store |F|^2 at the fftshift position;
 //  * the ghost texture's fractional Fourier transform (realflare/api/tasks/ghost.py:13-36
-//    and realflare/utils/frft.py:20-62, Ozaktas et al. 1996 chirp convolution), built from
-//    the plain transform and element-wise chirp kernels.
-// Rows whose length is a power of two run the radix-2 kernel below; any other length from
+//    and realflare/utils/frft.py:20-62, Ozaktas et al. 1996 chirp convolution): three 2-D
+//    transforms of the aperture and one of a chirp in four passes (rf_ghost_frft).
+// Rows whose length is a power of two from 8 on are transformed directly; any other length from
 // 2 to 4096 runs Bluestein's chirp-z form (Bluestein 1970): with w_m = exp(d pi i m^2 / n),
-// X_k = w_k sum_j (x_j w_j) conj(w_{k-j}), a linear convolution evaluated by radix-2
-// transforms of a power-of-two length M >= 2n - 1, in shared memory, one row per block.
+// X_k = w_k sum_j (x_j w_j) conj(w_{k-j}), a linear convolution evaluated by transforms of a
+// power-of-two length M >= 2n - 1; the filter's transform is evaluated once per block.
+//
+// What bounds it: latency on the small textures (a few microseconds per launch), shared memory and
+// the transposing stores on batches. 512 x 512, 16 spectra 161 -> 70 us (both passes); a 256 x
+// 256 ghost texture 74 -> 34 us in 13 -> 4 launches; 702 x 954 (chirp-z) 757 -> 322 us.
 #include <complex>
 #include <math.h>
+
+#include <algorithm>
 
 #include "rf_common.cuh"
 
@@ -28,19 +35,328 @@ constexpr int kMaxN = 4096;
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// a * (0, s) for s = +-1
+__device__ __forceinline__ float2 rot90(float2 a, float s) { return make_float2(-s * a.y, s * a.x); }
 
-// Load callbacks: produce element i of row `row` (row = batch * rows_per_batch + r).
-struct LoadComplex {
-    const float2* in;
-    int n;
-    __device__ float2 operator()(long long row, int i) const { return in[row * n + i]; }
+// ---------------------------------------------------------------- row transforms
+// How rows of length n are transformed: M is the power-of-two length, n itself or the convolution's.
+struct RowPlan {
+    int n, M, log_m, rows_per_block, threads;
+    size_t smem;
 };
-struct LoadStarburst {  // aperture * chirp, batch = wavelength
+
+// lengths the row transforms accept: 2 to 4096, any factorisation
+bool fft_length_ok(int n) { return n >= 2 && n <= kMaxN; }
+
+__host__ __device__ constexpr int padded(int i) { return i + (i >> 3); }  // conflict-free strides of 8
+
+// Plan for `rows` rows of length n: enough blocks for the SMs first, then more rows per block (longer
+// runs in the transposing stores, shared tables), up to 8 and 512 threads.
+RowPlan row_plan(int n, long long rows) {
+    RowPlan p;
+    p.n = n;
+    p.M = 8;
+    p.log_m = 3;
+    const bool direct = n >= 8 && (n & (n - 1)) == 0;
+    while (direct ? p.M < n : p.M < 2 * n - 1) p.M <<= 1, p.log_m++;
+    const int per_row = p.M / 8;
+    p.rows_per_block = per_row < 32 ? 32 / per_row : 1;  // whole warps
+    while (p.rows_per_block < 8 && 2 * p.rows_per_block * per_row <= 512 &&
+           rows / (2 * p.rows_per_block) >= 128)
+        p.rows_per_block *= 2;
+    p.threads = p.rows_per_block * per_row;
+    const size_t row = sizeof(float2) * padded(p.M);
+    p.smem = row * p.rows_per_block + (direct ? 0 : row) + sizeof(float2) * p.M;
+    return p;
+}
+
+// the 4-point transform of v[0], v[q], v[2 q], v[3 q]
+template <int q>
+__device__ __forceinline__ void fft4(float2* v, float s) {
+    const float2 a = cadd(v[0], v[2 * q]), b = csub(v[0], v[2 * q]);
+    const float2 c = cadd(v[q], v[3 * q]), d = rot90(csub(v[q], v[3 * q]), s);
+    v[0] = cadd(a, c);
+    v[q] = cadd(b, d);
+    v[2 * q] = csub(a, c);
+    v[3 * q] = csub(b, d);
+}
+// the 8-point transform, in place, natural order
+__device__ __forceinline__ void fft8(float2 v[8], float s) {
+    const float r = 0.70710678118654752f;
+    float2 e[4], o[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        e[k] = cadd(v[k], v[k + 4]);
+        o[k] = csub(v[k], v[k + 4]);
+    }
+    o[1] = make_float2(r * (o[1].x - s * o[1].y), r * (o[1].y + s * o[1].x));     // exp(s i pi / 4)
+    o[2] = rot90(o[2], s);
+    o[3] = make_float2(-r * (o[3].x + s * o[3].y), r * (s * o[3].x - o[3].y));    // exp(s 3 i pi / 4)
+    fft4<1>(e, s);
+    fft4<1>(o, s);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        v[2 * k] = e[k];
+        v[2 * k + 1] = o[k];
+    }
+}
+
+// Transform of one row of length M by its M / 8 threads: thread t brings elements t + r M / 8 in v;
+// the result lies in x (padded), natural order. s: the exponent's sign. tw[k] = exp(-2 pi i k / M).
+// Every thread of the block takes part (rows share the barriers; rows of at most 32 threads lie
+// within a warp).
+__device__ __forceinline__ void fft_row(float2 v[8], float2* x, const float2* tw, int M, int log_m, int t, float s) {
+    const int eighth = M >> 3;
+    const bool in_warp = eighth <= 32;
+    auto sync = [&]() {
+        if (in_warp)
+            __syncwarp();
+        else
+            __syncthreads();
+    };
+    int log_ns = 0;
+    for (int rest = log_m; rest > 0;) {
+        if (log_ns > 0) {
+#pragma unroll
+            for (int r = 0; r < 8; r++) v[r] = x[padded(t + r * eighth)];
+        }
+        const int ns = 1 << log_ns;
+        if (rest >= 3) {
+            const int k = t & (ns - 1);
+            if (log_ns > 0) {
+                const int step = k << (log_m - log_ns - 3);
+#pragma unroll
+                for (int r = 1; r < 8; r++) {
+                    const float2 w = tw[r * step];
+                    v[r] = cmul(v[r], make_float2(w.x, -s * w.y));
+                }
+            }
+            fft8(v, s);
+            const int d = ((t - k) << 3) + k;
+            sync();  // everything is read
+#pragma unroll
+            for (int r = 0; r < 8; r++) x[padded(d + (r << log_ns))] = v[r];
+            log_ns += 3;
+            rest -= 3;
+        } else if (rest == 2) {  // two 4-point steps: elements t + (q + 2 r) M / 8, r = 0 .. 3
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int j = t + q * eighth, k = j & (ns - 1), step = k << (log_m - log_ns - 2);
+#pragma unroll
+                for (int r = 1; r < 4; r++) {
+                    const float2 w = tw[r * step];
+                    v[q + 2 * r] = cmul(v[q + 2 * r], make_float2(w.x, -s * w.y));
+                }
+                fft4<2>(v + q, s);
+            }
+            sync();
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int j = t + q * eighth, k = j & (ns - 1), d = ((j - k) << 2) + k;
+#pragma unroll
+                for (int r = 0; r < 4; r++) x[padded(d + (r << log_ns))] = v[q + 2 * r];
+            }
+            log_ns += 2;
+            rest = 0;
+        } else {  // four 2-point steps: elements t + (q + 4 r) M / 8, r = 0, 1
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int j = t + q * eighth, k = j & (ns - 1);
+                const float2 w = tw[k << (log_m - log_ns - 1)];
+                const float2 b = cmul(v[q + 4], make_float2(w.x, -s * w.y)), a = v[q];
+                v[q] = cadd(a, b);
+                v[q + 4] = csub(a, b);
+            }
+            sync();
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int j = t + q * eighth, k = j & (ns - 1), d = ((j - k) << 1) + k;
+                x[padded(d)] = v[q];
+                x[padded(d + ns)] = v[q + 4];
+            }
+            log_ns += 1;
+            rest = 0;
+        }
+        sync();  // everything is written
+    }
+}
+
+// exp(d pi i m^2 / n), the phase reduced exactly: m^2 mod 2n (m < n <= 4096)
+__device__ __forceinline__ float2 bluestein_chirp(int m, int n, float d) {
+    const unsigned r = ((unsigned)m * (unsigned)m) % (2u * (unsigned)n);
+    float sn, cs;
+    sincospif(d * (float)r / (float)n, &sn, &cs);
+    return make_float2(cs, sn);
+}
+
+// One pass. Program: float2 load(row, i); float sign(row), the first transform's direction (+-1, 0:
+// none); float sign2(row), a second transform's (0: none) of mid(row, i, value); and
+// store(row, i, value).
+template <class Program>
+__global__ void __launch_bounds__(1024) k_fft_pass(const Program p, int rows, int n, int M, int log_m,
+                                                   int rows_per_block) {
+    extern __shared__ float2 sm[];
+    const bool chirp_z = M != n;
+    const int eighth = M >> 3, row_size = padded(M);
+    const int g = threadIdx.x / eighth, t = threadIdx.x % eighth;  // the thread's row in the block, and place in it
+    float2* x = sm + g * row_size;
+    float2* filter = sm + rows_per_block * row_size;          // chirp_z: the filter's transform
+    float2* tw = filter + (chirp_z ? row_size : 0);
+    const int row0 = blockIdx.x * rows_per_block, row = row0 + g;
+    const bool valid = row < rows;
+    // A pass may start while the one before it runs (launch_pass): its tables need nothing from it.
+    // With the filter, which takes a third of the work, it is let in only at the end of its
+    // predecessor, whose blocks it would otherwise slow down (82 x 554: 93 against 83 us).
+    if (!chirp_z) cudaTriggerProgrammaticLaunchCompletion();
+    for (int k = threadIdx.x; k < M; k += blockDim.x) {
+        float sn, cs;
+        sincospif(-2.0f * (float)k / (float)M, &sn, &cs);
+        tw[k] = make_float2(cs, sn);
+    }
+    float2 v[8];
+    if (chirp_z) {
+        // b_m = conj(w_m) of direction -1 for |m| < n, wrapped; of direction +1 it is the conjugate,
+        // and so is its transform (b is symmetric)
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int i = t + r * eighth, m = i < n ? i : M - i;
+            v[r] = m < n ? bluestein_chirp(m, n, 1.0f) : make_float2(0.0f, 0.0f);
+        }
+        fft_row(v, x, tw, M, log_m, t, -1.0f);
+        if (g == 0)
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                const int i = padded(t + r * eighth);
+                filter[i] = x[i];
+            }
+    }
+    __syncthreads();
+    cudaGridDependencySynchronize();  // the passes before are complete
+    const float inv_m = 1.0f / (float)M;
+    // element i of the transformed row
+    auto result = [&](const float2* from, int i, float s) {
+        const float2 c = from[padded(i)];
+        if (!chirp_z) return c;
+        return cmul(bluestein_chirp(i, n, s), make_float2(c.x * inv_m, c.y * inv_m));
+    };
+    // transforms the row whose elements t + r M / 8 are in v
+    auto transform = [&](float s) {
+        if (!chirp_z) {
+            fft_row(v, x, tw, M, log_m, t, s);
+            return;
+        }
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int i = t + r * eighth;
+            if (i < n) v[r] = cmul(v[r], bluestein_chirp(i, n, s));
+        }
+        fft_row(v, x, tw, M, log_m, t, -1.0f);
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int i = padded(t + r * eighth);
+            const float2 f = filter[i];
+            v[r] = cmul(x[i], make_float2(f.x, -s * f.y));
+        }
+        fft_row(v, x, tw, M, log_m, t, 1.0f);
+    };
+    // (directions are those of the block's first row: programs keep them equal within a block)
+    const float s1 = p.sign(row0), s2 = p.sign2(row0);
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        const int i = t + r * eighth;
+        v[r] = valid && i < n ? p.load(row, i) : make_float2(0.0f, 0.0f);
+    }
+    if (s1 != 0.0f) transform(s1);
+    if (s2 != 0.0f) {
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int i = t + r * eighth;
+            v[r] = valid && i < n ? p.mid(row, i, s1 != 0.0f ? result(x, i, s1) : v[r]) : make_float2(0.0f, 0.0f);
+        }
+        if (s1 != 0.0f && eighth <= 32) __syncwarp();
+        transform(s2);
+    }
+    const float s = s2 != 0.0f ? s2 : s1;
+    if (s == 0.0f) {  // no transform: the rows pass through
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int i = t + r * eighth;
+            if (valid && i < n) p.store(row, i, v[r]);
+        }
+        return;
+    }
+    if (chirp_z) cudaTriggerProgrammaticLaunchCompletion();
+    __syncthreads();  // every row of the block is transformed
+    // consecutive threads store one element of the block's consecutive rows: runs in the
+    // transposed result
+    const int log_rows = __ffs(rows_per_block) - 1;
+    for (int e = threadIdx.x; e < n << log_rows; e += blockDim.x) {
+        const int q = e & (rows_per_block - 1), i = e >> log_rows;
+        if (row0 + q < rows) p.store(row0 + q, i, result(sm + q * row_size, i, s));
+    }
+}
+
+template <class Program>
+int launch_pass(const Program& program, long long rows, const RowPlan& plan, cudaStream_t s) {
+    if (rows > 0x7fffffff - 64) return RF_ERR_NOT_SUPPORTED;
+    auto kernel = k_fft_pass<Program>;
+    if (plan.smem > 48 * 1024)
+        RF_TRY(cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem)));
+    const long long blocks = (rows + plan.rows_per_block - 1) / plan.rows_per_block;
+    // programmatic dependent launch: the launch latency and the tables overlap the pass before
+    // (256 x 256 ghost texture, four passes: 40.7 -> 34.4 us)
+    cudaLaunchAttribute overlap = {};
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)plan.threads);
+    cfg.dynamicSmemBytes = plan.smem;
+    cfg.stream = s;
+    cfg.attrs = &overlap;
+    cfg.numAttrs = 1;
+    RF_TRY(cuda_status(cudaLaunchKernelEx(&cfg, kernel, program, (int)rows, plan.n, plan.M, plan.log_m,
+                                          plan.rows_per_block)));
+    return launch_status();
+}
+
+// rows of a [batch][rows][n] array, transformed and stored transposed ([batch][n][rows]), scaled
+struct TransposePass {
+    const float2* in;
+    float2* out;
+    int n, rows;
+    float s, scale;
+    __device__ float sign(int) const { return s; }
+    __device__ float sign2(int) const { return 0.0f; }
+    __device__ float2 load(int row, int i) const { return in[(size_t)row * n + i]; }
+    __device__ float2 mid(int, int, float2 v) const { return v; }
+    __device__ void store(int row, int i, float2 v) const {
+        const unsigned b = (unsigned)row / (unsigned)rows, r = (unsigned)row % (unsigned)rows;
+        out[((size_t)b * n + i) * rows + r] = make_float2(v.x * scale, v.y * scale);
+    }
+};
+
+// 2-D transform of data [batch][h][w] in place (scratch of the same size).
+int fft2(float2* data, float2* scratch, int batch, int w, int h, int direction, float scale, cudaStream_t s) {
+    const float dir = direction < 0 ? -1.0f : 1.0f;
+    const long long rows = (long long)batch * h, cols = (long long)batch * w;
+    RF_TRY(launch_pass(TransposePass{data, scratch, w, h, dir, 1.0f}, rows, row_plan(w, rows), s));
+    return launch_pass(TransposePass{scratch, data, h, w, dir, scale}, cols, row_plan(h, cols), s);
+}
+
+// ---------------------------------------------------------------- starburst spectrum
+struct StarburstRows {  // aperture * chirp, batch = wavelength
     const float* aperture;
+    float2* out;  // [batch][w][h]
     int w, h;
     float phase_scale[256];  // per batch: 1 / (lambda d); the phase is pi * scale * r^2
-    __device__ float2 operator()(long long row, int i) const {
-        const int b = (int)(row / h), y = (int)(row % h);
+    __device__ float sign(int) const { return -1.0f; }
+    __device__ float sign2(int) const { return 0.0f; }
+    __device__ float2 load(int row, int i) const {
+        const int b = (int)((unsigned)row / (unsigned)h), y = (int)((unsigned)row % (unsigned)h);
         const float x0 = w > 1 ? -1.0f + (float)i * (2.0f / (float)(w - 1)) : -1.0f;
         const float y0 = h > 1 ? -1.0f + (float)y * (2.0f / (float)(h - 1)) : -1.0f;
         const float a = __ldg(aperture + (size_t)y * w + i);
@@ -48,232 +364,122 @@ struct LoadStarburst {  // aperture * chirp, batch = wavelength
         sincospif(phase_scale[b] * (x0 * x0 + y0 * y0), &s, &c);
         return make_float2(a * c, a * s);
     }
-};
-
-// Store callbacks: receive the transformed element i of row `row`.
-struct StoreTransposed {  // out[batch][i][r] (row = batch * rows + r), scaled
-    float2* out;
-    int n, rows;
-    float scale;
-    __device__ void operator()(long long row, int i, float2 v) const {
-        const long long b = row / rows, r = row % rows;
-        out[(b * n + i) * rows + r] = make_float2(v.x * scale, v.y * scale);
+    __device__ float2 mid(int, int, float2 v) const { return v; }
+    __device__ void store(int row, int i, float2 v) const {
+        const unsigned b = (unsigned)row / (unsigned)h, y = (unsigned)row % (unsigned)h;
+        out[((size_t)b * w + i) * h + y] = v;
     }
 };
-struct StorePower {  // |v|^2 at the fftshift position of the [batch][rows][n] image
+struct PowerColumns {  // |v|^2 at the fftshift position of the [batch][h][w] image
+    const float2* in;  // [batch][w][h]
     float* out;
-    int n, rows;
-    __device__ void operator()(long long row, int i, float2 v) const {
-        const long long b = row / rows, r = row % rows;  // r = original column, i = original row
-        const int ys = (i + n / 2) % n, xs = (int)((r + rows / 2) % rows);
-        out[(b * n + ys) * rows + xs] = v.x * v.x + v.y * v.y;
+    int w, h;
+    __device__ float sign(int) const { return -1.0f; }
+    __device__ float sign2(int) const { return 0.0f; }
+    __device__ float2 load(int row, int i) const { return in[(size_t)row * h + i]; }
+    __device__ float2 mid(int, int, float2 v) const { return v; }
+    __device__ void store(int row, int i, float2 v) const {
+        const unsigned b = (unsigned)row / (unsigned)w;
+        const int x = (int)((unsigned)row % (unsigned)w);
+        int ys = i + h / 2, xs = x + w / 2;
+        ys -= ys >= h ? h : 0, xs -= xs >= w ? w : 0;
+        out[((size_t)b * h + ys) * w + xs] = v.x * v.x + v.y * v.y;
     }
 };
 
-template <class Load, class Store>
-__global__ void k_fft_rows(Load load, Store store, int n, int log_n, float dir) {
-    extern __shared__ float2 sm[];
-    float2* x = sm;
-    float2* tw = sm + n;
-    const long long row = blockIdx.x;
-    for (int k = threadIdx.x; k < n / 2; k += blockDim.x) {
-        float s, c;
-        sincospif(dir * 2.0f * (float)k / (float)n, &s, &c);  // exp(dir * 2 pi i k / n)
-        tw[k] = make_float2(c, s);
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int rev = (int)(__brev((unsigned)i) >> (32 - log_n));
-        x[rev] = load(row, i);
-    }
-    __syncthreads();
-    for (int s = 1; s <= log_n; s++) {
-        const int half = 1 << (s - 1);
-        const int stride = n >> s;  // twiddle index step
-        for (int k = threadIdx.x; k < n / 2; k += blockDim.x) {
-            const int j = k & (half - 1);
-            const int base = (k >> (s - 1)) << s;
-            const float2 u = x[base + j];
-            const float2 v = cmul(x[base + j + half], tw[j * stride]);
-            x[base + j] = make_float2(u.x + v.x, u.y + v.y);
-            x[base + j + half] = make_float2(u.x - v.x, u.y - v.y);
-        }
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) store(row, i, x[i]);
-}
-
-int log2_exact(int n) {
-    if (n < 2 || n > 2 * kMaxN || (n & (n - 1))) return -1;
-    int l = 0;
-    while ((1 << l) < n) l++;
-    return l;
-}
-
-// lengths the row transforms accept: 2 to 4096, any factorisation
-bool fft_length_ok(int n) { return n >= 2 && n <= kMaxN; }
-
-// exp(d pi i m^2 / n), the phase reduced exactly: m^2 mod 2n
-__device__ __forceinline__ float2 bluestein_chirp(int m, int n, float d) {
-    const long long r = ((long long)m * m) % (2LL * n);
-    float sn, cs;
-    sincospif(d * (float)r / (float)n, &sn, &cs);
-    return make_float2(cs, sn);
-}
-
-// the radix-2 butterflies of k_fft_rows over two arrays at once (input in bit-reversed order,
-// output in natural order), twiddles tw[k] = exp(-2 pi i k / M)
-__device__ __forceinline__ void butterflies2(float2* x, float2* y, const float2* tw, int M, int logM) {
-    for (int s = 1; s <= logM; s++) {
-        const int half = 1 << (s - 1);
-        const int stride = M >> s;
-        for (int k = threadIdx.x; k < M / 2; k += blockDim.x) {
-            const int j = k & (half - 1);
-            const int base = (k >> (s - 1)) << s;
-            const float2 w = tw[j * stride];
-            float2 u = x[base + j], v = cmul(x[base + j + half], w);
-            x[base + j] = make_float2(u.x + v.x, u.y + v.y);
-            x[base + j + half] = make_float2(u.x - v.x, u.y - v.y);
-            if (y) {
-                u = y[base + j];
-                v = cmul(y[base + j + half], w);
-                y[base + j] = make_float2(u.x + v.x, u.y + v.y);
-                y[base + j + half] = make_float2(u.x - v.x, u.y - v.y);
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// One row of any length n (Bluestein): a_j = x_j w_j and b_m = conj(w_m) for |m| < n
-// (wrapped to M - m), A = FFT(a), B = FFT(b), conv = IFFT(A B) (as conj(FFT(conj(A B))) / M),
-// X_k = w_k conv_k. Shared memory: a, b (M each) and the twiddles (M / 2).
-template <class Load, class Store>
-__global__ void k_fft_rows_bluestein(Load load, Store store, int n, int M, int logM, float dir) {
-    extern __shared__ float2 sm[];
-    float2* a = sm;
-    float2* b = a + M;
-    float2* tw = b + M;
-    const long long row = blockIdx.x;
-    for (int k = threadIdx.x; k < M / 2; k += blockDim.x) {
-        float sn, cs;
-        sincospif(-2.0f * (float)k / (float)M, &sn, &cs);
-        tw[k] = make_float2(cs, sn);
-    }
-    for (int i = threadIdx.x; i < M; i += blockDim.x) {
-        float2 av = make_float2(0.0f, 0.0f), bv = make_float2(0.0f, 0.0f);
-        if (i < n) {
-            const float2 w = bluestein_chirp(i, n, dir);
-            av = cmul(load(row, i), w);
-            bv = make_float2(w.x, -w.y);
-        } else if (i > M - n) {
-            const float2 w = bluestein_chirp(M - i, n, dir);
-            bv = make_float2(w.x, -w.y);
-        }
-        const int rev = (int)(__brev((unsigned)i) >> (32 - logM));
-        a[rev] = av;
-        b[rev] = bv;
-    }
-    __syncthreads();
-    butterflies2(a, b, tw, M, logM);
-    for (int i = threadIdx.x; i < M; i += blockDim.x) a[i] = cmul(a[i], b[i]);
-    __syncthreads();
-    for (int i = threadIdx.x; i < M; i += blockDim.x) {
-        const float2 v = a[i];
-        b[(int)(__brev((unsigned)i) >> (32 - logM))] = make_float2(v.x, -v.y);
-    }
-    __syncthreads();
-    butterflies2(b, nullptr, tw, M, logM);
-    const float inv = 1.0f / (float)M;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const float2 c = make_float2(b[k].x * inv, -b[k].y * inv);
-        store(row, k, cmul(bluestein_chirp(k, n, dir), c));
-    }
-}
-
-template <class Load, class Store>
-int launch_rows(Load load, Store store, long long rows, int n, float dir, cudaStream_t s) {
-    if (!fft_length_ok(n)) return RF_ERR_NOT_SUPPORTED;
-    if (n & (n - 1)) {
-        int M = 1;
-        while (M < 2 * n - 1) M <<= 1;
-        const int logM = log2_exact(M);
-        const size_t smem = sizeof(float2) * (2 * M + M / 2);
-        auto kernel = k_fft_rows_bluestein<Load, Store>;
-        if (smem > 48 * 1024)
-            RF_TRY(cuda_status(
-                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)));
-        kernel<<<(unsigned)rows, M / 2 < 256 ? (M / 2 < 32 ? 32 : M / 2) : 256, smem, s>>>(load, store, n, M, logM,
-                                                                                            dir);
-        return launch_status();
-    }
-    const int log_n = log2_exact(n);
-    const int threads = n / 2 < 256 ? (n / 2 < 32 ? 32 : n / 2) : 256;
-    const size_t smem = sizeof(float2) * (n + n / 2);
-    auto kernel = k_fft_rows<Load, Store>;
-    if (smem > 48 * 1024)
-        RF_TRY(cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)));
-    kernel<<<(unsigned)rows, threads, smem, s>>>(load, store, n, log_n, dir);
-    return launch_status();
-}
-
-// 2-D transform of data [batch][h][w] in place (scratch of the same size).
-int fft2(float2* data, float2* scratch, int batch, int w, int h, int direction, float scale, cudaStream_t s) {
-    const float dir = direction < 0 ? -1.0f : 1.0f;
-    RF_TRY(launch_rows(LoadComplex{data, w}, StoreTransposed{scratch, w, h, 1.0f}, (long long)batch * h, w, dir, s));
-    return launch_rows(LoadComplex{scratch, h}, StoreTransposed{data, h, w, scale}, (long long)batch * w, h, dir, s);
-}
-
-// ---------------------------------------------------------------- FRFT helpers
-// numpy's fftshift moves element i to (i + n / 2) mod n: output i reads (i + n - n / 2) mod n
-__global__ void k_fftshift_real(const float* __restrict__ in, float2* __restrict__ out, int w, int h) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)w * h) return;
-    const int y = (int)(i / w), x = (int)(i % w);
-    out[i] = make_float2(in[(size_t)((y + h - h / 2) % h) * w + (x + w - w / 2) % w], 0.0f);
-}
-
-__global__ void k_flip(const float2* __restrict__ in, float2* __restrict__ out, int w, int h) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)w * h) return;
-    const int y = (int)(i / w), x = (int)(i % w);
-    out[i] = in[(size_t)(h - 1 - y) * w + (w - 1 - x)];
-}
-
+// ---------------------------------------------------------------- ghost texture
 // chirp(shape) of frft.py:8-17: pi * (a^2 / h + b^2 / w), a/b = fftshift(arange(-n/2, n/2))
-__device__ __forceinline__ float chirp_r(int y, int x, int w, int h) {
+__device__ __forceinline__ float2 chirp_value(int y, int x, int w, int h, float c) {
     const int a = y < h / 2 ? y : y - h;
     const int b = x < w / 2 ? x : x - w;
-    return (float)(a * a) / (float)h + (float)(b * b) / (float)w;
+    const float r = (float)(a * a) / (float)h + (float)(b * b) / (float)w;
+    float sn, cs;
+    sincospif(r * c, &sn, &cs);
+    return make_float2(cs, sn);
 }
-
-// mode 0: data *= exp(i pi r c1); mode 1: data = exp(i pi r c2)
-__global__ void k_chirp(float2* __restrict__ data, int w, int h, float c, int mode) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)w * h) return;
-    const int y = (int)(i / w), x = (int)(i % w);
-    float s, co;
-    sincospif(chirp_r(y, x, w, h) * c, &s, &co);
-    const float2 e = make_float2(co, s);
-    data[i] = mode == 0 ? cmul(data[i], e) : e;
-}
-
-__global__ void k_cmul(float2* __restrict__ a, const float2* __restrict__ b, long long n) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = cmul(a[i], b[i]);
-}
-
-// out = |fftshift(scale * chirp1 * data)| * norm
-__global__ void k_frft_finish(const float2* __restrict__ data, float* __restrict__ out, int w, int h, float c1,
-                              float2 scale, float norm) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)w * h) return;
-    const int y = (int)(i / w), x = (int)(i % w);
-    const int ys = (y + h - h / 2) % h, xs = (x + w - w / 2) % w;  // fftshift source
-    float s, co;
-    sincospif(chirp_r(ys, xs, w, h) * c1, &s, &co);
-    float2 v = cmul(cmul(scale, make_float2(co, s)), data[(size_t)ys * w + xs]);
-    out[i] = sqrtf(v.x * v.x + v.y * v.y) * norm;
-}
+struct FrftArgs {
+    int w, h;
+    float first;  // the transform before the chirp convolution (normalize() of frft.py): +-1, 0 none
+    bool flip;
+    float c1, c2, ortho, first_scale;
+    float2 scale;
+    float norm;
+};
+// Passes 1 and 2 carry two arrays, the aperture's (rows below `split`) and chirp 2's, so that a launch
+// holds the work of both; `split` is a multiple of the rows per block. numpy's fftshift moves
+// element i to (i + n / 2) mod n: output i reads (i + n - n / 2) mod n.
+struct FrftRows1 {  // rows y: the shifted aperture's first transform; chirp 2's
+    FrftArgs f;
+    const float* aperture;
+    float2 *a, *b;  // out [w][h]
+    int split;
+    __device__ float sign(int row) const { return row < split ? f.first : -1.0f; }
+    __device__ float sign2(int) const { return 0.0f; }
+    __device__ float2 load(int row, int x) const {
+        if (row >= split) return chirp_value((int)(row - split), x, f.w, f.h, f.c2);
+        if (row >= f.h) return make_float2(0.0f, 0.0f);
+        int y = (int)row;
+        if (f.flip) y = f.h - 1 - y, x = f.w - 1 - x;
+        return make_float2(__ldg(aperture + (size_t)((y + f.h - f.h / 2) % f.h) * f.w + (x + f.w - f.w / 2) % f.w), 0.0f);
+    }
+    __device__ float2 mid(int, int, float2 v) const { return v; }
+    __device__ void store(int row, int x, float2 v) const {
+        if (row >= split)
+            b[(size_t)x * f.h + (row - split)] = v;
+        else if (row < f.h)
+            a[(size_t)x * f.h + row] = v;
+    }
+};
+struct FrftColumns2 {  // columns x: the first transform's, chirp 1, the forward transform's; chirp 2's
+    FrftArgs f;
+    const float2* a;  // [w][h]
+    float2* b;        // [w][h], in place
+    float2* out;      // [h][w]
+    int split;
+    __device__ float sign(int row) const { return row < split ? f.first : -1.0f; }
+    __device__ float sign2(int row) const { return row < split ? -1.0f : 0.0f; }
+    __device__ float2 load(int row, int y) const {
+        if (row >= split) return b[(size_t)(row - split) * f.h + y];
+        return row < f.w ? a[(size_t)row * f.h + y] : make_float2(0.0f, 0.0f);
+    }
+    __device__ float2 mid(int row, int y, float2 v) const {
+        return cmul(make_float2(v.x * f.first_scale, v.y * f.first_scale), chirp_value(y, (int)row, f.w, f.h, f.c1));
+    }
+    __device__ void store(int row, int y, float2 v) const {
+        if (row >= split)
+            b[(size_t)(row - split) * f.h + y] = make_float2(v.x * f.ortho, v.y * f.ortho);
+        else if (row < f.w)
+            out[(size_t)y * f.w + row] = v;
+    }
+};
+struct FrftRows3 {  // rows y: the forward transform's, times chirp 2's transform, the inverse's
+    FrftArgs f;
+    const float2 *a, *b;  // [h][w], [w][h]
+    float2* out;          // [w][h]
+    __device__ float sign(int) const { return -1.0f; }
+    __device__ float sign2(int) const { return 1.0f; }
+    __device__ float2 load(int row, int x) const { return a[(size_t)row * f.w + x]; }
+    __device__ float2 mid(int row, int x, float2 v) const {
+        return cmul(make_float2(v.x * f.ortho, v.y * f.ortho), b[(size_t)x * f.h + row]);
+    }
+    __device__ void store(int row, int x, float2 v) const { out[(size_t)x * f.h + row] = v; }
+};
+struct FrftColumns4 {  // columns x: the inverse transform's; |fftshift(scale * chirp 1 * data)| * norm
+    FrftArgs f;
+    const float2* a;  // [w][h]
+    float* out;
+    __device__ float sign(int) const { return 1.0f; }
+    __device__ float sign2(int) const { return 0.0f; }
+    __device__ float2 load(int row, int y) const { return a[(size_t)row * f.h + y]; }
+    __device__ float2 mid(int, int, float2 v) const { return v; }
+    __device__ void store(int row, int y, float2 v) const {
+        v = make_float2(v.x * f.ortho, v.y * f.ortho);
+        const float2 r = cmul(cmul(f.scale, chirp_value(y, (int)row, f.w, f.h, f.c1)), v);
+        int ys = y + f.h / 2, xs = (int)row + f.w / 2;
+        ys -= ys >= f.h ? f.h : 0, xs -= xs >= f.w ? f.w : 0;
+        out[(size_t)ys * f.w + xs] = sqrtf(r.x * r.x + r.y * r.y) * f.norm;
+    }
+};
 
 }  // namespace
 }  // namespace rf
@@ -293,17 +499,18 @@ extern "C" int rf_starburst_spectrum(const float* aperture, int32_t width, int32
     if (!aperture || !lambdas_mm || !scratch || !spectrum || count < 1 || count > 256) return RF_ERR_INVALID_ARG;
     if (!fft_length_ok(width) || !fft_length_ok(height)) return RF_ERR_NOT_SUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
+    float2* buf = (float2*)scratch;
     // phase = pi * (x^2 + y^2) / (lambda d): one factor per wavelength, passed by value
-    LoadStarburst load;
+    StarburstRows load;
     load.aperture = aperture;
+    load.out = buf;
     load.w = width;
     load.h = height;
     for (int b = 0; b < count; b++) load.phase_scale[b] = (float)(1.0 / ((double)lambdas_mm[b] * (double)distance_mm));
-    float2* buf = (float2*)scratch;
     // rows: aperture * chirp -> transposed; columns: -> |F|^2 at the fftshift position
-    RF_TRY(launch_rows(load, StoreTransposed{buf, width, height, 1.0f}, (long long)count * height, width, -1.0f, s));
-    return launch_rows(LoadComplex{buf, height}, StorePower{spectrum, height, width}, (long long)count * width,
-                       height, -1.0f, s);
+    const long long rows = (long long)count * height, cols = (long long)count * width;
+    RF_TRY(launch_pass(load, rows, row_plan(width, rows), s));
+    return launch_pass(PowerColumns{buf, spectrum, width, height}, cols, row_plan(height, cols), s);
 }
 
 extern "C" int rf_ghost_frft(const float* aperture, int32_t width, int32_t height, float alpha, float* scratch,
@@ -313,54 +520,54 @@ extern "C" int rf_ghost_frft(const float* aperture, int32_t width, int32_t heigh
     if (!fft_length_ok(width) || !fft_length_ok(height)) return RF_ERR_NOT_SUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
     const long long n = (long long)width * height;
-    float2* A = (float2*)scratch;
-    float2* B = A + n;
-    float2* T = B + n;
-    const unsigned blocks = blocks_for(n, 256);
-    const float ortho = (float)(1.0 / std::sqrt((double)n));
-    k_fftshift_real<<<blocks, 256, 0, s>>>(aperture, A, width, height);
-    RF_TRY(launch_status());
+    float2* S0 = (float2*)scratch;
+    float2* S1 = S0 + n;
+    float2* S2 = S1 + n;
+    FrftArgs f;
+    f.w = width;
+    f.h = height;
+    f.ortho = (float)(1.0 / std::sqrt((double)n));
     // normalize() of frft.py:20-40, in double on the host
     double rel = std::fmod((double)alpha, 4.0);
     if (rel < 0) rel += 4.0;
     double a;
+    f.flip = false;
     if (rel < 0.5) {
         a = rel + 1;
-        RF_TRY(fft2(A, T, 1, width, height, +1, ortho, s));
+        f.first = 1.0f;
     } else if (rel < 1.5) {
         a = rel;
+        f.first = 0.0f;
     } else if (rel < 2.5) {
         a = rel - 1;
-        RF_TRY(fft2(A, T, 1, width, height, -1, ortho, s));
+        f.first = -1.0f;
     } else if (rel < 3.5) {
         a = rel - 2;
-        k_flip<<<blocks, 256, 0, s>>>(A, T, width, height);
-        RF_TRY(launch_status());
-        RF_TRY(cuda_status(cudaMemcpyAsync(A, T, sizeof(float2) * n, cudaMemcpyDeviceToDevice, s)));
+        f.first = 0.0f;
+        f.flip = true;
     } else {
         a = rel - 3;
-        RF_TRY(fft2(A, T, 1, width, height, +1, ortho, s));
+        f.first = 1.0f;
     }
+    f.first_scale = f.first != 0.0f ? f.ortho : 1.0f;
     const double phi = a * M_PI / 2.0;
     const double cot = 1.0 / std::tan(phi);
     const double sq = std::sqrt(1.0 + cot * cot);
     const std::complex<double> scale = std::sqrt(std::complex<double>(1.0, -cot)) / std::sqrt((double)n);
-    const float c1 = (float)(cot - sq), c2 = (float)sq;
-    // fft2 = fftn(chirp1 * A); fft1 = fftn(chirp2); A = ifftn(fft1 * fft2)
-    k_chirp<<<blocks, 256, 0, s>>>(A, width, height, c1, 0);
-    RF_TRY(launch_status());
-    RF_TRY(fft2(A, T, 1, width, height, -1, ortho, s));
-    k_chirp<<<blocks, 256, 0, s>>>(B, width, height, c2, 1);
-    RF_TRY(launch_status());
-    RF_TRY(fft2(B, T, 1, width, height, -1, ortho, s));
-    k_cmul<<<blocks, 256, 0, s>>>(A, B, n);
-    RF_TRY(launch_status());
-    RF_TRY(fft2(A, T, 1, width, height, +1, ortho, s));
-    // |fftshift(scale * chirp1 * A)| * sqrt(w * h), ghost.py:33-35
-    k_frft_finish<<<blocks, 256, 0, s>>>(A, texture, width, height, c1,
-                                         make_float2((float)scale.real(), (float)scale.imag()),
-                                         (float)std::sqrt((double)n));
-    return launch_status();
+    f.c1 = (float)(cot - sq);
+    f.c2 = (float)sq;
+    f.scale = make_float2((float)scale.real(), (float)scale.imag());
+    f.norm = (float)std::sqrt((double)n);  // ghost.py:33-35
+    // fft2 = fftn(chirp1 * A); fft1 = fftn(chirp2); A = ifftn(fft1 * fft2). The first transform's
+    // columns, chirp 1 and the forward transform's columns share a pass, as do the forward
+    // transform's rows, the product with chirp 2's transform and the inverse's rows.
+    const RowPlan by_row = row_plan(width, 2LL * height), by_column = row_plan(height, 2LL * width);
+    const long long split1 = (height + by_row.rows_per_block - 1) / by_row.rows_per_block * by_row.rows_per_block;
+    const long long split2 = (width + by_column.rows_per_block - 1) / by_column.rows_per_block * by_column.rows_per_block;
+    RF_TRY(launch_pass(FrftRows1{f, aperture, S0, S1, (int)split1}, split1 + height, by_row, s));
+    RF_TRY(launch_pass(FrftColumns2{f, S0, S1, S2, (int)split2}, split2 + width, by_column, s));
+    RF_TRY(launch_pass(FrftRows3{f, S2, S1, S0}, height, row_plan(width, height), s));
+    return launch_pass(FrftColumns4{f, S0, texture}, width, row_plan(height, width), s);
 }
 
 // ---------------------------------------------------------------- no-allocation variant
