@@ -305,6 +305,11 @@ int rf_aperture_shape(float* image, int32_t width, int32_t height, float size_x,
 int rf_aperture_dust(float* image, int32_t width, int32_t height, float size_x, float size_y,
                      float strength, float density, float radius, float parallax_x,
                      float parallax_y, float softness, void* stream);
+/* The first count values of numpy's Generator(PCG64(seed)).random(dtype=float32), bit for bit:
+ * out, device float[count], 16-byte aligned. state and inc are the generator's 128-bit words
+ * (PCG64(seed).state['state']), each as its high and its low half. */
+int rf_noise_pcg64(uint64_t state_hi, uint64_t state_lo, uint64_t inc_hi, uint64_t inc_lo,
+                   float* out, int64_t count, void* stream);
 /* Blurred-noise dust (no reference counterpart): image *= 1 - strength * G_sigma * noise,
  * a separable Gaussian of radius ceil(4 sigma), clamp-to-edge. noise: device float[h][w];
  * scratch: device float[h][w]. */

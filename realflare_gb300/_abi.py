@@ -140,6 +140,7 @@ class BatchSizes(ctypes.Structure):
 P = ctypes.c_void_p
 I32 = ctypes.c_int32
 I64 = ctypes.c_int64
+U64 = ctypes.c_uint64
 F32 = ctypes.c_float
 
 # name -> argtypes (every entry point returns int status)
@@ -168,6 +169,7 @@ SIGNATURES = {
     'rf_ghost_frft_static': [P, I32, I32, F32, P, P],
     'rf_aperture_shape': [P, I32, I32, F32, F32, I32, F32, F32, F32, P],
     'rf_aperture_dust': [P, I32, I32, F32, F32, F32, F32, F32, F32, F32, F32, P],
+    'rf_noise_pcg64': [U64, U64, U64, U64, P, I64, P],
     'rf_aperture_noise_dust': [P, P, P, I32, I32, F32, F32, P],
     'rf_axpby': [P, F32, P, F32, P, I64, P],
     'rf_accumulate_mirrored': [P, P, I32, I32, I32, F32, P, P],

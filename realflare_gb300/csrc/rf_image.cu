@@ -238,6 +238,51 @@ __global__ void __launch_bounds__(256) k_aperture_dust(float* __restrict__ image
     image[(size_t)y * w + x] = v;
 }
 
+// numpy's Generator(PCG64(seed)).random(dtype=float32): the permuted congruential generator PCG
+// XSL-RR 128/64 (M. E. O'Neill, PCG: A Family of Simple Fast Space-Efficient Statistically Good
+// Algorithms for Random Number Generation, 2014), each 64-bit output giving two floats (low half
+// first), the top 24 bits of each half over 2^24. Threads jump to their place in the sequence (F.
+// B. Brown, Random Number Generation with Arbitrary Strides, 1994): the state after n steps is
+// an affine map of the first one, by squaring. 512 x 512: 7.4 us, where the host's generator and
+// the copy of its pageable result took about 700.
+constexpr int kNoiseOutputs = 4;  // 64-bit outputs per thread
+__global__ void __launch_bounds__(256) k_noise_pcg64(unsigned long long state_hi, unsigned long long state_lo,
+                                                     unsigned long long inc_hi, unsigned long long inc_lo,
+                                                     float* __restrict__ out, long long n) {
+    using u128 = unsigned __int128;
+    const u128 mult = ((u128)0x2360ed051fc65da4ull << 64) | 0x4385df649fccf645ull;
+    const u128 inc = ((u128)inc_hi << 64) | inc_lo;
+    const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * kNoiseOutputs;
+    if (2 * first >= n) return;
+    u128 a = 1, c = 0, step_a = mult, step_c = inc;  // state -> a state + c: so far, and per power of two
+    for (unsigned long long d = (unsigned long long)first; d; d >>= 1) {
+        if (d & 1) {
+            a *= step_a;
+            c = c * step_a + step_c;
+        }
+        step_c *= step_a + 1;
+        step_a *= step_a;
+    }
+    u128 state = a * (((u128)state_hi << 64) | state_lo) + c;
+    float v[2 * kNoiseOutputs];
+#pragma unroll
+    for (int k = 0; k < kNoiseOutputs; k++) {
+        state = state * mult + inc;
+        const unsigned long long x = (unsigned long long)(state >> 64) ^ (unsigned long long)state;
+        const int r = (int)(state >> 122);
+        const unsigned long long o = (x >> r) | (x << ((64 - r) & 63));
+        v[2 * k] = (float)((unsigned)o >> 8) * (1.0f / 16777216.0f);
+        v[2 * k + 1] = (float)((unsigned)(o >> 32) >> 8) * (1.0f / 16777216.0f);
+    }
+    if (2 * first + 2 * kNoiseOutputs <= n) {
+#pragma unroll
+        for (int k = 0; k < kNoiseOutputs / 2; k++)
+            reinterpret_cast<float4*>(out + 2 * first)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    } else {
+        for (int k = 0; k < 2 * kNoiseOutputs && 2 * first + k < n; k++) out[2 * first + k] = v[k];
+    }
+}
+
 // Separable Gaussian over the noise (no reference counterpart): pass 0 blurs rows into
 // tmp, pass 1 blurs columns of tmp and multiplies the image by 1 - strength * blur.
 struct BlurWeights {
@@ -349,6 +394,18 @@ extern "C" int rf_aperture_dust(float* image, int32_t width, int32_t height, flo
     dim3 grid((width + 15) / 16, (height + 15) / 16);
     k_aperture_dust<<<grid, 256, 0, (cudaStream_t)stream>>>(image, width, height, size_x, size_y, strength, count,
                                                             radius, parallax_x, parallax_y, softness);
+    return launch_status();
+}
+
+extern "C" int rf_noise_pcg64(uint64_t state_hi, uint64_t state_lo, uint64_t inc_hi, uint64_t inc_lo, float* out,
+                              int64_t count, void* stream) {
+    using namespace rf;
+    if (!out || count < 0 || !aligned16(out)) return RF_ERR_INVALID_ARG;
+    if (count == 0) return RF_OK;
+    const long long threads = (count + 2 * kNoiseOutputs - 1) / (2 * kNoiseOutputs);
+    if (threads > 0x7fffffffLL) return RF_ERR_NOT_SUPPORTED;
+    k_noise_pcg64<<<blocks_for(threads, 256), 256, 0, (cudaStream_t)stream>>>(state_hi, state_lo, inc_hi, inc_lo, out,
+                                                                            count);
     return launch_status();
 }
 

@@ -263,9 +263,12 @@ class ApertureTask(Task):
         d = aperture.dust
         if d.strength > 0:
             if d.blur_sigma > 0:
-                rng = np.random.Generator(np.random.PCG64(d.seed))
-                noise = to_device(rng.random((h, w), dtype=np.float32))
-                scratch = empty((h, w))
+                # Generator(PCG64(seed)).random((h, w), dtype=float32), generated on the device
+                g = np.random.PCG64(d.seed).state['state']
+                word = (1 << 64) - 1
+                noise, scratch = empty((h, w)), empty((h, w))
+                check(self.lib.rf_noise_pcg64(g['state'] >> 64, g['state'] & word, g['inc'] >> 64, g['inc'] & word,
+                                              ptr(noise), h * w, self.stream), 'rf_noise_pcg64')
                 check(self.lib.rf_aperture_noise_dust(ptr(image), ptr(noise), ptr(scratch), w, h, d.strength,
                                                       d.blur_sigma, self.stream), 'rf_aperture_noise_dust')
             else:
