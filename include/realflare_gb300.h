@@ -340,7 +340,7 @@ typedef struct rf_frame {
     int64_t trace_block, quad_block, vertex_block, pair_block;  /* first block of each stage */
     int32_t tile_offset, tile_count;  /* the frame's raster tiles in the batch's tile numbering */
     float direction_n[3];     /* normalize(-direction.xyz) in FP32, as rf_trace computes it */
-    int32_t pad1;
+    int32_t trace_item;       /* the frame's first work item in the batch's trace */
     uint64_t ghost_texture;   /* rf_ghost_texture_object of the frame's ghost texture, or 0 */
 } rf_frame;
 

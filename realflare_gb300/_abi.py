@@ -107,7 +107,7 @@ class Frame(ctypes.Structure):
         ('tile_offset', ctypes.c_int32),
         ('tile_count', ctypes.c_int32),
         ('direction_n', ctypes.c_float * 3),
-        ('pad1', ctypes.c_int32),
+        ('trace_item', ctypes.c_int32),
         ('ghost_texture', ctypes.c_uint64),
     ]
 

@@ -11,7 +11,7 @@
 namespace rf {
 namespace {
 
-constexpr int kThreads = 256;       // block size of every batched stage
+constexpr int kThreads = 256;       // block size of every batched stage but the trace
 constexpr int kMaxElements = 128;   // rf_trace.cu
 constexpr int kMaxGrid = 2048;      // rf_trace.cu
 constexpr int kMaxSub = 64;         // records per raster batch (rf_raster.cu)
@@ -98,7 +98,18 @@ extern "C" int rf_batch_plan(rf_frame* frames, int32_t frame_count, int32_t tile
         f.direction_n[0] = vx * inv;
         f.direction_n[1] = vy * inv;
         f.direction_n[2] = vz * inv;
-        f.pad1 = 0;
+    }
+    // the trace's work items: some paths and (wavelength, grid point) pairs of a frame each
+    const int trace_paths = batch_trace_paths(z.rays, rays_per_thread);
+    long long items = 0;
+    for (int i = 0; i < frame_count; i++) {
+        const rf_trace_args& t = frames[i].trace;
+        frames[i].trace_item = (int32_t)items;
+        items += batch_trace_items(t, trace_paths, rays_per_thread);
+        if (items > 0x7fffffffLL) {
+            set_error_text("rf_batch_plan: the batch exceeds 2^31 trace items");
+            return RF_ERR_NOT_SUPPORTED;
+        }
     }
     z.ghost_textures = 1;
     for (int i = 0; i < frame_count; i++) z.ghost_textures = z.ghost_textures && frames[i].ghost_texture != 0;

@@ -40,6 +40,33 @@ inline int cuda_status(cudaError_t e) {
 inline unsigned blocks_for(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
+// The traces: threads of a block, ghost paths a thread may trace at once (rf_trace_core.cuh), and the
+// blocks per SM that a launch should have, below which a block takes fewer paths.
+constexpr int kTraceThreads = 128;
+constexpr int kMaxTracePaths = 16;
+constexpr int kTraceBlocksPerSm = 16;
+// The largest number of paths a block takes at once, up to kMaxTracePaths, that leaves blocks_wanted
+// blocks (ray_blocks per path): more paths share more legs, too few blocks leave SMs idle at the
+// end. Limits of 12 / 16 / 20 blocks per SM: 3.9 M rays 0.371 / 0.334 / 0.337 ms, 7.9 M 0.597 / 0.592 /
+// 0.596 ms, 72.4 M no difference. Up to 32 paths: 72.4 M rays (276 paths) 5.40 instead of 5.63 ms, but
+// 15.1 M (182 paths) 0.939 instead of 0.800 ms. Blocks of 64 and of 256 threads: 72.4 M 5.86 ms.
+inline int paths_per_block(long long path_count, long long ray_blocks, long long blocks_wanted) {
+    int k = kMaxTracePaths;
+    while (k > 1 && (path_count + k - 1) / k * ray_blocks < blocks_wanted) k /= 2;
+    return k;
+}
+// The same for a batch, from its number of rays, and a frame's work items with k paths each.
+inline int batch_trace_paths(long long rays, int rays_per_thread) {
+    int k = kMaxTracePaths;
+    while (k > 1 && rays / ((long long)k * kTraceThreads * rays_per_thread) < 152 * kTraceBlocksPerSm) k /= 2;
+    return k;
+}
+__host__ __device__ inline long long batch_trace_items(const rf_trace_args& t, int k, int rays_per_thread) {
+    const long long pairs = (long long)t.wavelength_count * t.grid_count * t.grid_count;
+    const int chunk = kTraceThreads * rays_per_thread;
+    return ((long long)t.path_count + k - 1) / k * ((pairs + chunk - 1) / chunk);
+}
+
 // ---------------------------------------------------------------- batched frames
 // The frame owning work unit `unit` of a stage: the last frame whose first unit of that
 // stage (first(frame), non-decreasing over the frames) is <= unit. Frames without units

@@ -14,7 +14,6 @@
 namespace rf {
 namespace {
 
-constexpr int kTraceThreads = 256;
 constexpr int kMaxElements = 128;
 constexpr int kMaxGrid = 2048;  // (float)ray_id / G is exact enough for trunc() up to 2048
 
@@ -294,17 +293,34 @@ struct TraceFrame {
     float dir[3];  // normalize(-direction.xyz), host-computed in FP32
 };
 
+// The reflectance of element e for a ray (dx, dy, dz) that hits it from a medium of index n1, the
+// element's own index being n2. kAngles: from the incidence angle.
+template <bool kAngles>
+__device__ __forceinline__ float surface_reflectance(float dx, float dy, float dz, const Hit& h, const SmemElement& e,
+                                                     float n1, float n2, float wavelength, const TraceFrame& f) {
+    const float nc = fmaxf(sqrtf(n1 * n2), f.cmin);
+    const float d1 = e.layers == 1 ? e.d0 : (float)e.coating / (4.0f * nc);
+    if (kAngles) {
+        const float incident = incident_angle(dx, dy, dz, h);
+        // theta = incident + 1e-9 (a double sum there); only angles below 0.02 rad
+        // are close enough to 1e-9 for the double sum to differ from `incident`
+        const float theta = incident < 0.02f ? (float)((double)incident + 1e-9) : incident;
+        if (e.layers == 2)
+            return fresnel_two_layer_angle(theta, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
+        if (e.layers == 1 || e.coating > 0) return fresnel_ar_angle(theta, wavelength, d1, n1, nc, n2);
+        return fresnel_angle(theta, n1, n2);
+    }
+    const float c0 = incident_cos(dx, dy, dz, h), s0 = sqrt_rn((1.0f - c0) * (1.0f + c0));
+    if (e.layers == 2) return fresnel_two_layer(c0, s0, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
+    if (e.layers == 1 || e.coating > 0) return fresnel_ar(c0, s0, wavelength, d1, n1, nc, n2);
+    return fresnel(c0, s0, n1, n2);
+}
+
 // Observer of a traced ray: step() sees the ray entering each element (element index,
 // position, direction), hit() each successful intersection (loop step index, the hit, the
 // incoming direction, whether the element is flat), rrel() each candidate of the running
 // maximum before it is taken, reflect() each reflection. The adjoint records steps, the
-// intersection trace records hits; the forward trace uses NoRecord (inlined away).
-struct NoRecord {
-    __device__ __forceinline__ void step(int, float, float, float, float, float, float) {}
-    __device__ __forceinline__ void hit(int, const Hit&, float, float, float, bool) {}
-    __device__ __forceinline__ void rrel(float, float) {}
-    __device__ __forceinline__ void reflect() {}
-};
+// intersection trace records hits.
 
 // A wavelength's entry for one element: its index and the index ratios n1 / n2 a ray refracted there
 // sees going towards the light (dz < 0: n1 is the element before) or the sensor (the element after);
@@ -388,29 +404,7 @@ __device__ __forceinline__ void trace_ray_rec(const SmemElement* __restrict__ se
             const float n1 = (0 <= n_index && n_index < E) ? ior_of(n_index) : 1.0f;
             const float n2 = ior_of(lens_id);
             rec.reflect();
-            const float nc = fmaxf(sqrtf(n1 * n2), f.cmin);
-            const float d1 = e.layers == 1 ? e.d0 : (float)e.coating / (4.0f * nc);
-            float reflectance;
-            if (kAngles) {
-                const float incident = incident_angle(dx, dy, dz, h);
-                // theta = incident + 1e-9 (a double sum there); only angles below 0.02 rad
-                // are close enough to 1e-9 for the double sum to differ from `incident`
-                const float theta = incident < 0.02f ? (float)((double)incident + 1e-9) : incident;
-                if (e.layers == 2)
-                    reflectance = fresnel_two_layer_angle(theta, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
-                else if (e.layers == 1 || e.coating > 0)
-                    reflectance = fresnel_ar_angle(theta, wavelength, d1, n1, nc, n2);
-                else
-                    reflectance = fresnel_angle(theta, n1, n2);
-            } else {
-                const float c0 = incident_cos(dx, dy, dz, h), s0 = sqrt_rn((1.0f - c0) * (1.0f + c0));
-                if (e.layers == 2)
-                    reflectance = fresnel_two_layer(c0, s0, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
-                else if (e.layers == 1 || e.coating > 0)
-                    reflectance = fresnel_ar(c0, s0, wavelength, d1, n1, nc, n2);
-                else
-                    reflectance = fresnel(c0, s0, n1, n2);
-            }
+            const float reflectance = surface_reflectance<kAngles>(dx, dy, dz, h, e, n1, n2, wavelength, f);
             reflect_dir(dx, dy, dz, h);
             if (reflectance > 0.0f) refl *= reflectance;
         } else {
@@ -435,14 +429,172 @@ __device__ __forceinline__ void trace_ray_rec(const SmemElement* __restrict__ se
     out[5] = refl;
 }
 
-template <bool kAngles>
-__device__ __forceinline__ void trace_ray(const SmemElement* __restrict__ se, const float* ior_row,
-                                          const float2* ratio_row, bool disperse,
-                                          const float* __restrict__ coef_base, float wavelength, int2 path,
-                                          float grid_x, float grid_y, const TraceFrame& f, float out[6]) {
-    NoRecord none;
-    trace_ray_rec<kAngles>(se, ior_row, ratio_row, disperse, coef_base, wavelength, path, grid_x, grid_y, f, out, none);
+// A thread traces one grid point and wavelength along several ghost paths at once. Paths differ only
+// from their reflections on: the way to the first reflecting element serves every path that
+// reflects there or later, the way back from it every path of that first element, and only the last
+// leg from the second reflection is a path's own. Sorted by (first element, second element
+// descending) the paths are the leaves of a tree of depth two that is walked once, a ray that goes
+// on past a reflection being kept meanwhile. Every ray sees the operations of its own trace in
+// their order, so nothing changes in the results; 120 paths of 18 elements take 16 at a time 1860
+// surface interactions instead of 3648, 276 of 26 elements 5890 instead of 12064, and half the
+// first reflections' reflectances are shared.
+constexpr int kMaxPaths = kMaxTracePaths;
+static_assert(kMaxPaths <= 32, "one lane of a warp per path");
+struct PathList {
+    // first and second reflecting element (E, -1: none is reached), the path's index, the next path
+    // that differs and the next with another first element
+    int x[kMaxPaths], y[kMaxPaths], id[kMaxPaths], next[kMaxPaths], next_x[kMaxPaths];
+};
+// Paths [first, first + count) (count <= kMaxPaths) into l; the first warp of a block calls it.
+__device__ __forceinline__ void stage_paths(const int2* __restrict__ paths, int first, int count, int E, int aperture,
+                                            PathList& l) {
+    const int lane = threadIdx.x & 31;
+    int x = E + 1, y = 0;
+    if (lane < count) {
+        // no reflection at the stop or the last element, nor a second one outside the way back
+        const int2 q = __ldg(paths + first + lane);
+        const bool reflects = q.x >= 0 && q.x < E - 1 && q.x != aperture;
+        x = reflects ? q.x : E;
+        y = reflects && q.y >= 0 && q.y < q.x && q.y != aperture ? q.y : -1;
+    }
+    int rank = 0, next = 0, next_x = 0;
+#pragma unroll
+    for (int k = 0; k < kMaxPaths; k++) {
+        const int ox = __shfl_sync(0xffffffffu, x, k), oy = __shfl_sync(0xffffffffu, y, k);
+        rank += ox < x || (ox == x && (oy > y || (oy == y && k < lane)));
+        next += k < count && (ox < x || (ox == x && oy >= y));
+        next_x += k < count && ox <= x;
+    }
+    if (lane < count) {
+        l.x[rank] = x;
+        l.y[rank] = y;
+        l.id[rank] = first + lane;
+        l.next[rank] = next;
+        l.next_x[rank] = next_x;
+    }
 }
+// Walks the paths of l. The walk is the warp's; a lane whose ray has failed waits. Ray: State (the ray),
+// hit(element, state) (intersects and moves the ray there; false: missed), refract(element, state)
+// (false: the ray ends), reflect(element, state), store(path, state, whether it reached the end).
+template <class Ray>
+__device__ __forceinline__ void trace_paths(Ray& ray, typename Ray::State s, bool alive, const PathList& l, int count,
+                                            int E, int aperture) {
+    typename Ray::State kept[2];  // rays that go on past a reflection, per leg
+    bool kept_alive[2];
+    int i = 0, leg = 0, at = 0, step = 1, turn = l.x[0], last_x = 0, last_y = 0;
+    for (;;) {
+        if (alive) alive = ray.hit(at, s);
+        if (at == turn) {  // (never the stop or the last element)
+            if (leg == 0 ? l.next_x[i] < count : l.next[i] < l.next_x[i]) {  // paths after this one go on
+                typename Ray::State c = s;
+                kept_alive[leg] = alive && ray.refract(at, c);
+                kept[leg] = c;
+            }
+            if (alive) ray.reflect(at, s);
+            step = -step;
+            if (leg++ == 0) last_x = at, turn = l.y[i];
+            else last_y = at, turn = -1;
+        } else if (at != aperture && at != E - 1) {
+            if (alive) alive = ray.refract(at, s);
+        }
+        at += step;
+        while ((unsigned)at >= (unsigned)E || !__any_sync(0xffffffffu, alive)) {
+            // the ray is the last for these paths (those it would have turned at, where it failed)
+            const int end = leg == 2 ? l.next[i] : (leg == 1 ? l.next_x[i] : count);
+            const int group = l.next_x[i];
+            for (; i < end; i++) ray.store(l.id[i], s, alive);
+            if (end == count) return;
+            leg = leg == 2 && end < group ? 1 : 0;
+            s = kept[leg];
+            alive = kept_alive[leg];
+            step = leg == 0 ? 1 : -1;
+            at = (leg == 0 ? last_x : last_y) + step;
+            turn = leg == 0 ? l.x[i] : l.y[i];
+        }
+    }
+}
+// A ray in FP32.
+template <bool kAngles>
+struct FloatRay {
+    struct State {
+        float px, py, pz, dx, dy, dz, apt_x, apt_y, rrel, rrel2, refl;  // rrel2: see trace_ray_rec
+    };
+    const SmemElement* se;
+    const float* ior_row;     // this wavelength's row of the (wavelength, element) index table, or nullptr
+    const float2* ratio_row;  // and of the index ratios
+    bool disperse;
+    const float* coef_base;
+    float wavelength;
+    TraceFrame f;
+    float* out;  // rays + the ray's place in a path
+    long long per_path, plane;
+    bool mine;  // the lane has a ray
+    Hit h;
+
+    __device__ __forceinline__ float ior_of(int el) const {
+        if (ior_row) return ior_row[el];
+        float n = se[el].ior;
+        if (disperse && n > 1.0f) n = dispersion(wavelength, coef_base + (size_t)el * 16);
+        return n;
+    }
+    // init_ray, raytracing.cl:178-215
+    __device__ __forceinline__ State start(float grid_x, float grid_y) const {
+        const Hit h0 = intersect(grid_x, -grid_y, 1.0f, 0.0f, 0.0f, -1.0f, se[0]);
+        State s;  // the origin when the grid point misses element 0
+        s.dx = f.dir[0], s.dy = f.dir[1], s.dz = f.dir[2];
+        s.px = h0.px - s.dx, s.py = h0.py - s.dy, s.pz = h0.pz - s.dz;
+        s.apt_x = s.apt_y = s.rrel = s.rrel2 = 0.0f;
+        s.refl = 1.0f;
+        return s;
+    }
+    __device__ __forceinline__ bool hit(int at, State& s) {
+        const SmemElement& e = se[at];
+        h = intersect(s.px, s.py, s.pz, s.dx, s.dy, s.dz, e);
+        if (!h.hit) return false;
+        s.px = h.px, s.py = h.py, s.pz = h.pz;
+        if (at == f.aperture) {
+            s.apt_x = h.px / e.height;
+            s.apt_y = h.py / e.height;
+        } else {
+            const float xy2 = h.px * h.px + h.py * h.py;
+            if (!(xy2 < s.rrel2 * (e.height * e.height))) {
+                s.rrel = fmaxf(s.rrel, sqrtf(xy2) / e.height);
+                s.rrel2 = s.rrel * s.rrel * (1.0f - 0x1p-20f);
+            }
+        }
+        return true;
+    }
+    __device__ __forceinline__ bool refract(int at, State& s) {
+        float o;
+        if (ratio_row) {
+            const float2 q = ratio_row[at];
+            o = s.dz < 0.0f ? q.x : q.y;
+        } else {
+            const int n_index = (s.dz < 0.0f) ? at - 1 : at + 1;
+            o = ((0 <= n_index && n_index < f.E) ? ior_of(n_index) : 1.0f) / ior_of(at);
+        }
+        refract_dir(s.dx, s.dy, s.dz, h, o);
+        return s.dz != 0.0f;
+    }
+    __device__ __forceinline__ void reflect(int at, State& s) {
+        const int n_index = (s.dz < 0.0f) ? at - 1 : at + 1;
+        const float n1 = (0 <= n_index && n_index < f.E) ? ior_of(n_index) : 1.0f;
+        const float reflectance =
+            surface_reflectance<kAngles>(s.dx, s.dy, s.dz, h, se[at], n1, ior_of(at), wavelength, f);
+        reflect_dir(s.dx, s.dy, s.dz, h);
+        if (reflectance > 0.0f) s.refl *= reflectance;
+    }
+    __device__ __forceinline__ void store(int path, const State& s, bool alive) const {
+        if (!mine) return;
+        float* q = out + path * per_path;
+        q[0] = s.px;
+        q[plane] = s.py;
+        q[2 * plane] = s.apt_x;
+        q[3 * plane] = s.apt_y;
+        q[4 * plane] = s.rrel;
+        q[5 * plane] = alive ? s.refl : __int_as_float(0x7fffffff);
+    }
+};
 
 // Wavelength rows that kTraceThreads * rays consecutive rays can span, and the shared memory of
 // their tables (12 bytes per row and element); none past kMaxTableBytes.
