@@ -90,6 +90,20 @@ __device__ __forceinline__ int32_t wadd(int32_t a, int32_t b) { return (int32_t)
 __device__ __forceinline__ int32_t wsub(int32_t a, int32_t b) { return (int32_t)((uint32_t)a - (uint32_t)b); }
 __device__ __forceinline__ int32_t wmul(int32_t a, int32_t b) { return (int32_t)((uint32_t)a * (uint32_t)b); }
 
+// Correctly rounded square root without the range handling of the general operation, which the
+// trace's and the noise's operands do not need (both are bound by instruction issue): the hardware
+// approximation and one residual correction with fused multiply-adds (P. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000 processor, 1990). Compared with the correctly
+// rounded instruction for every float in [1, 4): equal; scaling by 4 scales every step exactly while
+// the residual does not underflow. x = 0 or in [2^-100, 2^127] (below, where an ulp can be lost, the
+// roots of the trace's squared distances are added to or compared with lens radii: no effect); inf
+// gives NaN. rcp_rn (rf_trace_core.cuh) is the reciprocal's like.
+__device__ __forceinline__ float sqrt_rn(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(x, 1.17549435e-38f)));
+    const float s = __fmul_rn(x, y);
+    return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, y), s);
+}
 __device__ __forceinline__ float clampf(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
 __device__ __forceinline__ float smoothstepf(float e0, float e1, float x) {
     float t = clampf((x - e0) / (e1 - e0), 0.0f, 1.0f);

@@ -24,10 +24,13 @@ __device__ __forceinline__ float hash_sin(float x) {
     float r = fmaf(-k, 0x1.921fb6p+0f, x);
     r = fmaf(-k, -0x1.777a5cp-25f, r);
     r = fmaf(-k, -0x1.ee59dap-50f, r);
+    // (beyond 2^22 k loses bits and r grows, to less than 10^5 for every sample index there is: no
+    // case for the slow reduction path, which the compiler then leaves out)
+    __builtin_assume(fabsf(r) < 1.0e5f);
     float sr, cr;
     sincosf(r, &sr, &cr);
-    const int q = (int)k & 3;
-    return q == 0 ? sr : (q == 1 ? cr : (q == 2 ? -sr : -cr));
+    const unsigned q = (unsigned)(int)k;
+    return __uint_as_float(__float_as_uint((q & 1) ? cr : sr) ^ (q & 2) << 30);
 }
 // noise(x, y, z) of noise.cl:1-5, with the terms in x and y given
 __device__ __forceinline__ float noise_at(float xy, float z) {
@@ -66,9 +69,9 @@ struct alignas(16) StarburstSample {
 // noise); coordinates too large for that come out as integers outside every texture.
 //
 // What bounds it: instruction issue. 1920 x 1080, 100 samples, 16 spectra, no jitter: 733 -> 310 us
-// (lookups were evaluated with 64-bit indices and divisions); 1000 samples with jitter 16.1 -> 12.3
-// ms (two noise hashes with their sines are most of what is left); 512 x 512 with jitter and
-// rotation 434 -> 317 us.
+// (lookups were evaluated with 64-bit indices and divisions); 1000 samples with jitter 16.1 -> 10.6
+// ms (12.3 with the sines' slow path, their quadrant by three selections and a general square root;
+// the two noise hashes are most of what is left); 512 x 512 with jitter and rotation 434 -> 256 us.
 template <bool kJitter, bool kRotate, int kPix>
 __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const float* __restrict__ spectrum,
                                                    const float* __restrict__ light, rf_starburst_args a,
@@ -132,7 +135,7 @@ __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const floa
             for (int k = 0; k < kPix; k++) {
                 float px = nx, py = ny[k];
                 if (kJitter) {
-                    const float radius = a.blur * sqrtf(noise_at(hash0[k], seed));
+                    const float radius = a.blur * sqrt_rn(noise_at(hash0[k], seed));
                     float sa, ca;
                     sincospif(2.0f * noise_at(hash0[k], seed + 1.0f), &sa, &ca);
                     px += ca * radius;

@@ -36,20 +36,7 @@ struct Hit {
     bool hit;
 };
 
-// Correctly rounded square root and reciprocal without the range handling of the general
-// operations, which the trace's operands do not need (it is bound by instruction issue): the
-// hardware approximation and one residual correction with fused multiply-adds (P. Markstein,
-// Computation of elementary functions on the IBM RISC System/6000 processor, 1990). Compared
-// with the correctly rounded instructions for every float in [1, 4): equal; scaling by 4 (by 2)
-// scales every step exactly while the residual does not underflow. sqrt_rn: x = 0 or in
-// [2^-100, 2^127] (below, where an ulp can be lost, the roots of squared distances are added to
-// or compared with lens radii: no effect); inf gives NaN. rcp_rn: |x| in [2^-100, 2^100].
-__device__ __forceinline__ float sqrt_rn(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(x, 1.17549435e-38f)));
-    const float s = __fmul_rn(x, y);
-    return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, y), s);
-}
+// The reciprocal, correctly rounded like sqrt_rn (rf_common.cuh): |x| in [2^-100, 2^100].
 __device__ __forceinline__ float rcp_rn(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
