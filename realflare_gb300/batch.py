@@ -112,13 +112,13 @@ def _frame_inputs(projects: list, ghost_offsets: list, ghost_shapes: list,
 
 def frame_bytes(project: Project) -> int:
     """Device bytes one frame holds in a batch, before tile lists: rays (24 B), vertices
-    (32 B), bounds and intensities, pair counters, image."""
+    (32 B), bounds and intensities, pair rectangles, image."""
     r = project.render
     P = len(project.flare.lens.ghost_paths)
     W, G = len(render_wavelengths(r)), r.grid_count
     rays = P * W * G * G
     prims = P * (G - 1) ** 2
-    return rays * (24 + 32) + prims * (16 + 4 * W + 4 * max(W - 1, 1)) + r.resolution.width() * r.resolution.height() * 16
+    return rays * (24 + 32) + prims * (16 + 4 * W + 8 * max(W - 1, 1)) + r.resolution.width() * r.resolution.height() * 16
 
 
 class BatchRenderer:

@@ -25,7 +25,7 @@ constexpr int kThreads = 256;
 constexpr float kSafeSamples = 16383.0f;
 
 struct BinGeometry {
-    int width, height, B, T, bdx, bdy, ntx, nty, S, W, G, maxW;
+    int width, height, B, T, bdx, bdy, ntx, nty, S, W, G, maxW, wide_bits;
     float st;
     bool safe_screen;  // width * S and height * S fit the overflow-free range
 };
@@ -77,15 +77,26 @@ __global__ void __launch_bounds__(kThreads) k_bin_masks(const float4* __restrict
         }
 }
 
+__device__ __forceinline__ void divide(long long a, int b, long long& q, int& r) {
+    if (a >> 32 == 0) {
+        q = (unsigned)a / (unsigned)b;
+        r = (int)((unsigned)a - (unsigned)q * (unsigned)b);
+    } else {
+        q = a / b;
+        r = (int)(a - q * b);
+    }
+}
+
 // Tile rectangle of one (primitive, wavelength pair); false when it contributes nothing.
 __device__ __forceinline__ bool pair_tile_rect(const float4* __restrict__ bounds, const float4* __restrict__ vtx,
-                                               long long prim, int w, const BinGeometry& g, int& tx0, int& tx1,
+                                               long long pair, const BinGeometry& g, int& tx0, int& tx1,
                                                int& ty0, int& ty1) {
-    int bx0, bx1, by0, by1;
+    int bx0, bx1, by0, by1, w, quad;
+    long long prim, path;
+    divide(pair, g.maxW, prim, w);
     if (!ref_bin_rect(__ldg(bounds + prim), g, bx0, bx1, by0, by1)) return false;
     const int Q = (g.G - 1) * (g.G - 1), VC = g.G * g.G;
-    const long long path = prim / Q;
-    const int quad = (int)(prim % Q);
+    divide(prim, Q, path, quad);
     const int row = quad / (g.G - 1), col = quad % (g.G - 1);
     const int c0 = row * g.G + col;
     const int corners[4] = {c0, c0 + 1, c0 + 1 + g.G, c0 + g.G};
@@ -124,52 +135,124 @@ __device__ __forceinline__ bool pair_tile_rect(const float4* __restrict__ bounds
     return tx0 <= tx1 && ty0 <= ty1;
 }
 
-__global__ void __launch_bounds__(kThreads) k_pair_count(const float4* __restrict__ bounds,
-                                                         const float4* __restrict__ vtx, long long n_pairs,
-                                                         BinGeometry g, uint32_t* __restrict__ counts,
-                                                         unsigned long long* __restrict__ total) {
-    const long long j = (long long)blockIdx.x * kThreads + threadIdx.x;
+// A pair's tile rectangle in 64 bits, so that it is found once, when it is counted, and not again
+// when its entries are written: its first tile (31 bits), width - 1 (wide_bits, those of the largest
+// there is) and height - 1; all ones: empty.
+constexpr unsigned long long kNoTiles = ~0ull;
+__device__ __forceinline__ unsigned long long pack_rect(int tx0, int tx1, int ty0, int ty1, const BinGeometry& g) {
+    return (unsigned long long)((unsigned)ty0 * (unsigned)g.ntx + (unsigned)tx0) |
+           (unsigned long long)(tx1 - tx0) << 31 | (unsigned long long)(ty1 - ty0) << (31 + g.wide_bits);
+}
+
+// Rectangle of a thread's pair into *rect, and the block's number of entries.
+__device__ __forceinline__ void count_pair(const float4* __restrict__ bounds, const float4* __restrict__ vtx,
+                                           long long pair, bool valid, const BinGeometry& g,
+                                           unsigned long long* rect, uint32_t* __restrict__ sums,
+                                           unsigned long long* __restrict__ total) {
+    __shared__ unsigned long long warp_sums[kThreads / 32];
     unsigned long long c = 0;
-    if (j < n_pairs) {
+    if (valid) {
         int tx0, tx1, ty0, ty1;
-        if (pair_tile_rect(bounds, vtx, j / g.maxW, (int)(j % g.maxW), g, tx0, tx1, ty0, ty1))
+        unsigned long long packed = kNoTiles;
+        if (pair_tile_rect(bounds, vtx, pair, g, tx0, tx1, ty0, ty1)) {
             c = (unsigned long long)(tx1 - tx0 + 1) * (unsigned long long)(ty1 - ty0 + 1);
-        counts[j] = (uint32_t)min(c, 0xffffffffull);
+            packed = pack_rect(tx0, tx1, ty0, ty1, g);
+        }
+        *rect = packed;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(total, c);
+    if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 1; k < kThreads / 32; k++) c += warp_sums[k];
+        sums[blockIdx.x] = (uint32_t)c;  // (a total beyond 32 bits is reported or refused by it)
+        if (c) atomicAdd(total, c);
+    }
 }
 
-__global__ void __launch_bounds__(kThreads) k_pair_emit(const float4* __restrict__ bounds,
-                                                        const float4* __restrict__ vtx, long long n_pairs,
-                                                        BinGeometry g, const uint32_t* __restrict__ offsets,
-                                                        uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+__global__ void __launch_bounds__(kThreads) k_pair_count(const float4* __restrict__ bounds,
+                                                         const float4* __restrict__ vtx, long long n_pairs,
+                                                         BinGeometry g, unsigned long long* __restrict__ rects,
+                                                         uint32_t* __restrict__ sums,
+                                                         unsigned long long* __restrict__ total) {
     const long long j = (long long)blockIdx.x * kThreads + threadIdx.x;
-    if (j >= n_pairs) return;
-    int tx0, tx1, ty0, ty1;
-    if (!pair_tile_rect(bounds, vtx, j / g.maxW, (int)(j % g.maxW), g, tx0, tx1, ty0, ty1)) return;
-    uint32_t o = offsets[j];
-    for (int ty = ty0; ty <= ty1; ty++)
-        for (int tx = tx0; tx <= tx1; tx++) {
-            keys[o] = (uint32_t)(ty * g.ntx + tx);
-            vals[o] = (uint32_t)j;
-            o++;
-        }
+    count_pair(bounds, vtx, j, j < n_pairs, g, rects + j, sums, total);
 }
 
-// tile_offsets[t] = first position of key >= t in the sorted keys
-__global__ void k_tile_offsets(const uint32_t* __restrict__ keys, long long n, int ntiles,
-                               uint32_t* __restrict__ tile_offsets) {
-    const int t = blockIdx.x * kThreads + threadIdx.x;
+// Writes the entries of a block's pairs (rects[0, n), the first one's number first_pair): the block's place in
+// the lists is base, its pairs' places follow from a scan of their counts. Threads take places, not
+// pairs (a pair covers one tile or thousands), and find a place's pair by bisection, so the stores
+// are coalesced. 92 M entries of 67 M pairs: 0.92 -> 0.48 ms (a thread per pair, its rectangle found
+// anew); 62 k of 27 k: 14.8 -> 5.3 us.
+__device__ __forceinline__ void emit_pairs(const unsigned long long* rects, int n, uint32_t base, long long capacity,
+                                           int ntx, int wide_bits, uint32_t first_tile, uint32_t first_pair,
+                                           uint32_t* keys, uint32_t* vals) {
+    __shared__ uint32_t start[kThreads], corner[kThreads], width[kThreads], warp_sums[kThreads / 32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const unsigned long long r = t < n ? rects[t] : kNoTiles;
+    const uint32_t w = (uint32_t)(r >> 31 & ((1ull << wide_bits) - 1)) + 1, h = (uint32_t)(r >> (31 + wide_bits)) + 1;
+    const uint32_t count = r == kNoTiles ? 0 : w * h;
+    uint32_t x = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_sums[warp] = x;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+#pragma unroll
+    for (int k = 0; k < kThreads / 32; k++) {
+        if (k == warp) before = total;
+        total += warp_sums[k];
+    }
+    start[t] = before + x - count;
+    corner[t] = (uint32_t)r & 0x7fffffffu;
+    width[t] = w;
+    __syncthreads();
+    for (uint32_t k = t; k < total; k += kThreads) {
+        int i = 0;  // the last pair that starts at or before place k (those without entries start where the next does)
+#pragma unroll
+        for (int step = kThreads / 2; step > 0; step >>= 1)
+            if (start[i + step] <= k) i += step;
+        const uint32_t d = k - start[i], dy = d / width[i], pos = base + k;
+        if (pos < capacity) {  // an overflowing batch is reported through the entry total
+            keys[pos] = first_tile + corner[i] + dy * (uint32_t)ntx + (d - dy * width[i]);
+            vals[pos] = first_pair + (uint32_t)i;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_pair_emit(const unsigned long long* rects, long long n_pairs, int ntx,
+                                                        int wide_bits, const uint32_t* offsets, long long capacity,
+                                                        uint32_t* keys, uint32_t* vals) {
+    chain_wait();
+    const long long first = (long long)blockIdx.x * kThreads;
+    emit_pairs(rects + first, (int)min((long long)kThreads, n_pairs - first), offsets[blockIdx.x], capacity, ntx, wide_bits,
+               0, (uint32_t)first, keys, vals);
+}
+
+// tile_offsets[t] = first position of key >= t in the sorted keys. A warp per tile: each step looks at 32
+// places of the interval at once, 6 dependent loads in 92 M keys instead of 27 (15.7 -> 8.3 us).
+__global__ void __launch_bounds__(kThreads) k_tile_offsets(const uint32_t* keys, long long n, int ntiles,
+                                                           uint32_t* tile_offsets) {
+    chain_wait();
+    const int lane = threadIdx.x & 31;
+    const long long t = ((long long)blockIdx.x * kThreads + threadIdx.x) >> 5;
     if (t > ntiles) return;
     long long lo = 0, hi = n;
-    while (lo < hi) {
-        long long mid = (lo + hi) >> 1;
-        if (keys[mid] < (uint32_t)t) lo = mid + 1;
-        else hi = mid;
+    while (hi > lo) {  // the answer lies in [lo, hi]
+        const long long len = hi - lo, step = (len + 31) / 32;
+        const long long at = lo + lane * step;  // the first of this lane's step places
+        const bool less = at < hi && keys[at] < (uint32_t)t;
+        const int k = __popc(__ballot_sync(0xffffffffu, less));  // lanes whose first place lies before the answer
+        if (k == 0) break;
+        hi = min(hi, lo + k * step);
+        lo += (k - 1) * step + 1;
     }
-    tile_offsets[t] = (uint32_t)lo;
+    if (lane == 0) tile_offsets[t] = (uint32_t)lo;
 }
 
 // Raster tiles are 32 x 32 or 16 x 16 pixels (rf_raster.cu); bins must be multiples of the tile.
@@ -198,6 +281,8 @@ __host__ __device__ inline bool make_geometry(const rf_raster_args& a, BinGeomet
     g.bdy = (a.height + g.B - 1) / g.B;
     g.ntx = (a.width + g.T - 1) / g.T;
     g.nty = (a.height + g.T - 1) / g.T;
+    g.wide_bits = 0;
+    while ((1LL << g.wide_bits) < g.ntx) g.wide_bits++;
     g.S = a.sub_steps;
     g.W = a.wavelength_count;
     g.G = a.grid_count;
@@ -213,82 +298,55 @@ __host__ __device__ inline bool make_geometry(const rf_raster_args& a, BinGeomet
 // numbered from tile_offset in the batch's tile numbering.
 struct FramePairs {
     BinGeometry g;
-    long long n_pairs, first;  // the frame's pair count and this thread's first local pair
-    const float4* bounds;
-    const float4* vtx;
-    long long pair_offset;
-    int tile_offset;
+    long long n_pairs;  // the frame's pair count; 0 for a geometry that is not valid
+    int frame;
 };
 
-__device__ __forceinline__ bool frame_pairs(const rf_frame* __restrict__ frames, int F, const float4* bounds_all,
-                                            const float4* vtx_all, int* frame_index, FramePairs& fp) {
-    if (threadIdx.x == 0)
-        *frame_index = find_frame(frames, F, blockIdx.x, [](const rf_frame& fr) { return fr.pair_block; });
+__device__ __forceinline__ void frame_pairs(const rf_frame* __restrict__ frames, int F, FramePairs* fp) {
+    if (threadIdx.x == 0) {
+        fp->frame = find_frame(frames, F, blockIdx.x, [](const rf_frame& fr) { return fr.pair_block; });
+        const rf_raster_args& a = frames[fp->frame].raster;
+        fp->n_pairs = make_geometry(a, fp->g) ? (long long)a.path_count * (fp->g.G - 1) * (fp->g.G - 1) * fp->g.maxW : 0;
+    }
     __syncthreads();
-    const rf_frame& fr = frames[*frame_index];
-    if (!make_geometry(fr.raster, fp.g)) return false;
-    fp.n_pairs = (long long)fr.raster.path_count * (fp.g.G - 1) * (fp.g.G - 1) * fp.g.maxW;
-    fp.first = (long long)(blockIdx.x - fr.pair_block) * kThreads + threadIdx.x;
-    fp.bounds = bounds_all + fr.prim_offset;
-    fp.vtx = vtx_all + 2 * fr.vertex_offset;
-    fp.pair_offset = fr.pair_offset;
-    fp.tile_offset = fr.tile_offset;
-    return true;
 }
 
 __global__ void __launch_bounds__(kThreads) k_pair_count_batch(const rf_frame* __restrict__ frames, int F,
                                                                const float4* __restrict__ bounds_all,
                                                                const float4* __restrict__ vtx_all,
-                                                               uint32_t* __restrict__ counts,
+                                                               unsigned long long* __restrict__ rects,
+                                                               uint32_t* __restrict__ sums,
                                                                unsigned long long* __restrict__ total) {
-    __shared__ int frame_index;
-    FramePairs fp;
-    const bool ok = frame_pairs(frames, F, bounds_all, vtx_all, &frame_index, fp);
-    const long long j = fp.first;
-    unsigned long long c = 0;
-    if (ok && j < fp.n_pairs) {
-        int tx0, tx1, ty0, ty1;
-        if (pair_tile_rect(fp.bounds, fp.vtx, j / fp.g.maxW, (int)(j % fp.g.maxW), fp.g, tx0, tx1, ty0, ty1))
-            c = (unsigned long long)(tx1 - tx0 + 1) * (unsigned long long)(ty1 - ty0 + 1);
-        counts[fp.pair_offset + j] = (uint32_t)min(c, 0xffffffffull);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(total, c);
+    __shared__ FramePairs fp;
+    frame_pairs(frames, F, &fp);
+    const rf_frame& fr = frames[fp.frame];
+    const long long j = (blockIdx.x - fr.pair_block) * kThreads + threadIdx.x;
+    count_pair(bounds_all + fr.prim_offset, vtx_all + 2 * fr.vertex_offset, j, j < fp.n_pairs, fp.g,
+               rects + fr.pair_offset + j, sums, total);
 }
 
-__global__ void __launch_bounds__(kThreads) k_pair_emit_batch(const rf_frame* __restrict__ frames, int F,
-                                                              const float4* __restrict__ bounds_all,
-                                                              const float4* __restrict__ vtx_all,
-                                                              const uint32_t* __restrict__ offsets,
-                                                              long long capacity, uint32_t* __restrict__ keys,
-                                                              uint32_t* __restrict__ vals) {
-    __shared__ int frame_index;
-    FramePairs fp;
-    if (!frame_pairs(frames, F, bounds_all, vtx_all, &frame_index, fp)) return;
-    const long long j = fp.first;
-    if (j >= fp.n_pairs) return;
-    int tx0, tx1, ty0, ty1;
-    if (!pair_tile_rect(fp.bounds, fp.vtx, j / fp.g.maxW, (int)(j % fp.g.maxW), fp.g, tx0, tx1, ty0, ty1)) return;
-    long long o = offsets[fp.pair_offset + j];
-    for (int ty = ty0; ty <= ty1; ty++)
-        for (int tx = tx0; tx <= tx1; tx++) {
-            if (o < capacity) {  // an overflowing batch is reported through the entry total
-                keys[o] = (uint32_t)(fp.tile_offset + ty * fp.g.ntx + tx);
-                vals[o] = (uint32_t)j;
-            }
-            o++;
-        }
+__global__ void __launch_bounds__(kThreads) k_pair_emit_batch(const rf_frame* frames, int F,
+                                                              const unsigned long long* rects, const uint32_t* offsets,
+                                                              long long capacity, uint32_t* keys, uint32_t* vals) {
+    __shared__ FramePairs fp;
+    chain_wait();
+    frame_pairs(frames, F, &fp);
+    const rf_frame& fr = frames[fp.frame];
+    const long long first = (blockIdx.x - fr.pair_block) * kThreads, rest = fp.n_pairs - first;
+    emit_pairs(rects + fr.pair_offset + first, (int)(rest < kThreads ? rest : kThreads), offsets[blockIdx.x], capacity,
+               fp.g.ntx, fp.g.wide_bits, (uint32_t)fr.tile_offset, (uint32_t)first, keys, vals);
 }
 
 // Entries [total, capacity) get the key `pad` (one past the last tile), so the sort over the
 // whole capacity leaves them at the end.
-__global__ void k_pad_entries(const unsigned long long* __restrict__ total, long long capacity, uint32_t pad,
-                              uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-    const long long i = (long long)blockIdx.x * kThreads + threadIdx.x;
-    if (i >= capacity || (unsigned long long)i < *total) return;
-    keys[i] = pad;
-    vals[i] = 0;
+__global__ void k_pad_entries(const unsigned long long* total, long long capacity, uint32_t pad, uint32_t* keys,
+                              uint32_t* vals) {
+    chain_wait();
+    for (unsigned long long i = *total + (unsigned long long)blockIdx.x * kThreads + threadIdx.x;
+         i < (unsigned long long)capacity; i += (unsigned long long)gridDim.x * kThreads) {
+        keys[i] = pad;
+        vals[i] = 0;
+    }
 }
 
 // Sort keys for the raster's tile order: 255 minus the tile's entry count as a tiny float
@@ -296,23 +354,79 @@ __global__ void k_pad_entries(const unsigned long long* __restrict__ total, long
 // stable sort puts the heaviest tiles first, within 12.5 %, and ties in tile order; empty
 // tiles, which still write their pixels, come last.
 constexpr int kOrderKeyBits = 8;
-__global__ void k_tile_order_keys(const uint32_t* __restrict__ tile_offsets, int tiles, uint32_t* __restrict__ keys,
-                                  uint32_t* __restrict__ vals) {
+__device__ __forceinline__ uint32_t order_key(uint32_t n) {
+    if (n == 0) return 255;
+    const int lz = __clz((int)n);
+    const uint32_t e = 31 - lz, m = (n << lz) << 1 >> 29;  // the 3 bits after the leading one
+    return 255 - (e * 8 + m);
+}
+__global__ void k_tile_order_keys(const uint32_t* tile_offsets, int tiles, uint32_t* keys, uint32_t* vals) {
+    chain_wait();
     const int t = blockIdx.x * kThreads + threadIdx.x;
     if (t >= tiles) return;
-    const uint32_t n = tile_offsets[t + 1] - tile_offsets[t];
-    uint32_t key = 255;
-    if (n > 0) {
-        const int lz = __clz((int)n);
-        const uint32_t e = 31 - lz, m = (n << lz) << 1 >> 29;  // the 3 bits after the leading one
-        key = 255 - (e * 8 + m);
-    }
-    keys[t] = key;
+    keys[t] = order_key(tile_offsets[t + 1] - tile_offsets[t]);
     vals[t] = (uint32_t)t;
+}
+// The whole order by one block, for up to kOrderBlockTiles tiles: a warp takes consecutive tiles, 32 at a
+// time, counts their keys and, once all counts are prefixed in (key, warp) order, places them. 1024
+// tiles: 4.2 us instead of the 16 us of four launches (keys, histogram, scan, scatter).
+constexpr int kOrderThreads = 1024, kOrderWarps = kOrderThreads / 32;
+constexpr int kOrderBlockTiles = 16384;
+__global__ void __launch_bounds__(kOrderThreads) k_tile_order(const uint32_t* tile_offsets, int tiles,
+                                                              uint32_t* order) {
+    __shared__ uint32_t counts[kOrderWarps][257];
+    __shared__ uint32_t warp_sums[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < kOrderWarps * 257; i += kOrderThreads) (&counts[0][0])[i] = 0;
+    chain_wait();
+    __syncthreads();
+    const int per_warp = ((tiles + kOrderThreads - 1) / kOrderThreads) * 32, first = warp * per_warp;
+    const int end = min(first + per_warp, tiles);
+    for (int pass = 0; pass < 2; pass++) {
+        for (int base = first; base < end; base += 32) {
+            const int t = base + lane;
+            const uint32_t key = t < end ? order_key(tile_offsets[t + 1] - tile_offsets[t]) : 256;
+            const unsigned peers = __match_any_sync(0xffffffffu, key);
+            const int leader = __ffs(peers) - 1;
+            uint32_t at = 0;
+            if (lane == leader) {
+                at = counts[warp][key];
+                counts[warp][key] = at + __popc(peers);
+            }
+            at = __shfl_sync(0xffffffffu, at, leader) + __popc(peers & ((1u << lane) - 1u));
+            if (pass == 1 && t < end) order[at] = (uint32_t)t;
+            __syncwarp();
+        }
+        if (pass == 1) break;
+        __syncthreads();
+        uint32_t total = 0, x = 0;
+        if (threadIdx.x < 256) {
+            for (int w = 0; w < kOrderWarps; w++) total += counts[w][threadIdx.x];
+            x = total;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) warp_sums[warp] = x;
+        }
+        __syncthreads();
+        if (threadIdx.x < 256) {
+            uint32_t run = x - total;
+            for (int w = 0; w < warp; w++) run += warp_sums[w];
+            for (int w = 0; w < kOrderWarps; w++) {
+                const uint32_t c = counts[w][threadIdx.x];
+                counts[w][threadIdx.x] = run;
+                run += c;
+            }
+        }
+        __syncthreads();
+    }
 }
 
 struct BinWorkspace {
-    uint32_t *counts, *scan_scratch, *keys_a, *keys_b, *vals_tmp, *radix_scratch;
+    unsigned long long* rects;
+    uint32_t *sums, *scan_scratch, *keys_a, *keys_b, *vals_tmp, *radix_scratch;
     unsigned long long* total;
     size_t bytes;
 };
@@ -326,8 +440,10 @@ BinWorkspace layout(char* base, long long n_pairs, long long capacity) {
         return p;
     };
     w.total = (unsigned long long*)take(sizeof(unsigned long long));
-    w.counts = (uint32_t*)take(sizeof(uint32_t) * (size_t)(n_pairs + 1));
-    w.scan_scratch = (uint32_t*)take(sizeof(uint32_t) * scan_scratch_words(n_pairs));
+    const long long blocks = (n_pairs + kThreads - 1) / kThreads;
+    w.rects = (unsigned long long*)take(sizeof(unsigned long long) * (size_t)n_pairs);
+    w.sums = (uint32_t*)take(sizeof(uint32_t) * (size_t)blocks);
+    w.scan_scratch = (uint32_t*)take(sizeof(uint32_t) * scan_scratch_words(blocks));
     w.keys_a = (uint32_t*)take(sizeof(uint32_t) * (size_t)capacity);
     w.keys_b = (uint32_t*)take(sizeof(uint32_t) * (size_t)capacity);
     w.vals_tmp = (uint32_t*)take(sizeof(uint32_t) * (size_t)capacity);
@@ -349,8 +465,9 @@ BatchWorkspace batch_layout(char* base, const rf_batch_sizes& z, long long capac
         return p;
     };
     const long long sort_n = capacity > z.tiles ? capacity : z.tiles;
-    w.counts = (uint32_t*)take(sizeof(uint32_t) * (size_t)(z.pairs + 1));
-    w.scan_scratch = (uint32_t*)take(sizeof(uint32_t) * scan_scratch_words(z.pairs));
+    w.rects = (unsigned long long*)take(sizeof(unsigned long long) * (size_t)z.pairs);
+    w.sums = (uint32_t*)take(sizeof(uint32_t) * (size_t)z.pair_blocks);
+    w.scan_scratch = (uint32_t*)take(sizeof(uint32_t) * scan_scratch_words(z.pair_blocks));
     w.keys_a = (uint32_t*)take(sizeof(uint32_t) * (size_t)capacity);
     w.keys_b = (uint32_t*)take(sizeof(uint32_t) * (size_t)capacity);
     w.vals_tmp = (uint32_t*)take(sizeof(uint32_t) * (size_t)capacity);
@@ -429,11 +546,12 @@ extern "C" int rf_bin_tiles(const float* bounds, const float* vertexes, const rf
     const int ntiles = g.ntx * g.nty;
     *entry_count = 0;
     RF_TRY(cuda_status(cudaMemsetAsync(w.total, 0, sizeof(unsigned long long), s)));
+    const unsigned pair_blocks = blocks_for(n_pairs, kThreads);
     if (n_pairs > 0) {
-        k_pair_count<<<blocks_for(n_pairs, kThreads), kThreads, 0, s>>>((const float4*)bounds,
-                                                                         (const float4*)vertexes, n_pairs, g,
-                                                                         w.counts, w.total);
+        k_pair_count<<<pair_blocks, kThreads, 0, s>>>((const float4*)bounds, (const float4*)vertexes, n_pairs, g,
+                                                      w.rects, w.sums, w.total);
         RF_TRY(launch_status());
+        RF_TRY(exclusive_scan_u32(w.sums, w.sums, pair_blocks, w.scan_scratch, s));
     }
     unsigned long long total = 0;
     RF_TRY(cuda_status(cudaMemcpyAsync(&total, w.total, sizeof(total), cudaMemcpyDeviceToHost, s)));
@@ -442,23 +560,20 @@ extern "C" int rf_bin_tiles(const float* bounds, const float* vertexes, const rf
     if (total > 0xfffffff0ull) return RF_ERR_NOT_SUPPORTED;
     if ((long long)total > entry_capacity || (total > 0 && !tile_entries)) return RF_ERR_WORKSPACE;
     if (total == 0) return cuda_status(cudaMemsetAsync(tile_offsets, 0, sizeof(uint32_t) * (ntiles + 1), s));
-    RF_TRY(exclusive_scan_u32(w.counts, w.counts, n_pairs, w.scan_scratch, s));
     int bits = 0;
     while ((1LL << bits) < ntiles) bits++;
     const int passes = (bits + 7) / 8;
     // arrange the ping-pong buffers so that the sorted values land in tile_entries
     uint32_t* vals_first = (passes % 2 == 0) ? tile_entries : w.vals_tmp;
     uint32_t* vals_alt = (passes % 2 == 0) ? w.vals_tmp : tile_entries;
-    k_pair_emit<<<blocks_for(n_pairs, kThreads), kThreads, 0, s>>>((const float4*)bounds, (const float4*)vertexes,
-                                                                    n_pairs, g, w.counts, w.keys_a, vals_first);
-    RF_TRY(launch_status());
+    RF_TRY(launch_chained(k_pair_emit, pair_blocks, kThreads, 0, s, w.rects, n_pairs, g.ntx, g.wide_bits, w.sums,
+                          entry_capacity, w.keys_a, vals_first));
     bool in_alt = false;
     RF_TRY(radix_sort_pairs(w.keys_a, vals_first, w.keys_b, vals_alt, (long long)total, bits, w.radix_scratch,
                             &in_alt, s));
     const uint32_t* sorted_keys = in_alt ? w.keys_b : w.keys_a;
-    k_tile_offsets<<<blocks_for(ntiles + 1, kThreads), kThreads, 0, s>>>(sorted_keys, (long long)total, ntiles,
-                                                                          tile_offsets);
-    return launch_status();
+    return launch_chained(k_tile_offsets, blocks_for(32 * (long long)(ntiles + 1), kThreads), kThreads, 0, s, sorted_keys,
+                          (long long)total, ntiles, tile_offsets);
 }
 
 namespace rf {
@@ -499,10 +614,10 @@ extern "C" int rf_tile_order(const uint32_t* tile_offsets, int32_t tile_count, v
     OrderWorkspace w = order_layout((char*)workspace, tile_count);
     if (w.bytes > workspace_bytes) return RF_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    k_tile_order_keys<<<blocks_for(tile_count, kThreads), kThreads, 0, s>>>(tile_offsets, tile_count, w.keys_b,
-                                                                           w.vals_b);
-    RF_TRY(launch_status());
-    if (tile_count == 1) return cuda_status(cudaMemsetAsync(tile_order, 0, sizeof(uint32_t), s));
+    if (tile_count <= kOrderBlockTiles)
+        return launch_chained(k_tile_order, 1, kOrderThreads, 0, s, tile_offsets, tile_count, tile_order);
+    RF_TRY(launch_chained(k_tile_order_keys, blocks_for(tile_count, kThreads), kThreads, 0, s, tile_offsets, tile_count,
+                          w.keys_b, w.vals_b));
     // two or more tiles and 8 key bits: exactly one pass, so the sorted pairs land in the
     // alternate buffers (keys, tile_order)
     bool in_alt = false;
@@ -535,10 +650,10 @@ extern "C" int rf_bin_tiles_batch(const rf_frame* frames, const rf_batch_sizes* 
     RF_TRY(cuda_status(cudaMemsetAsync(entry_total, 0, sizeof(uint64_t), s)));
     if (z.pair_blocks > 0) {
         k_pair_count_batch<<<(unsigned)z.pair_blocks, kThreads, 0, s>>>(
-            frames, z.frame_count, (const float4*)bounds, (const float4*)vertexes, w.counts,
+            frames, z.frame_count, (const float4*)bounds, (const float4*)vertexes, w.rects, w.sums,
             (unsigned long long*)entry_total);
         RF_TRY(launch_status());
-        RF_TRY(exclusive_scan_u32(w.counts, w.counts, z.pairs, w.scan_scratch, s));
+        RF_TRY(exclusive_scan_u32(w.sums, w.sums, z.pair_blocks, w.scan_scratch, s));
     }
     int bits = 0;
     while ((1LL << bits) <= z.tiles) bits++;  // keys 0 .. tiles (tiles = padding)
@@ -546,25 +661,24 @@ extern "C" int rf_bin_tiles_batch(const rf_frame* frames, const rf_batch_sizes* 
     uint32_t* vals_first = (passes % 2 == 0) ? tile_entries : w.vals_tmp;
     uint32_t* vals_alt = (passes % 2 == 0) ? w.vals_tmp : tile_entries;
     if (z.pair_blocks > 0) {
-        k_pair_emit_batch<<<(unsigned)z.pair_blocks, kThreads, 0, s>>>(
-            frames, z.frame_count, (const float4*)bounds, (const float4*)vertexes, w.counts, entry_capacity,
-            w.keys_a, vals_first);
-        RF_TRY(launch_status());
+        RF_TRY(launch_chained(k_pair_emit_batch, (unsigned)z.pair_blocks, kThreads, 0, s, frames, z.frame_count, w.rects,
+                              w.sums, entry_capacity, w.keys_a, vals_first));
     }
-    k_pad_entries<<<blocks_for(entry_capacity, kThreads), kThreads, 0, s>>>(
-        (const unsigned long long*)entry_total, entry_capacity, (uint32_t)z.tiles, w.keys_a, vals_first);
-    RF_TRY(launch_status());
+    RF_TRY(launch_chained(k_pad_entries, std::min(blocks_for(entry_capacity, kThreads), 2048u), kThreads, 0, s,
+                          (const unsigned long long*)entry_total, entry_capacity, (uint32_t)z.tiles, w.keys_a,
+                          vals_first));
     bool in_alt = false;
     RF_TRY(radix_sort_pairs(w.keys_a, vals_first, w.keys_b, vals_alt, entry_capacity, bits, w.radix_scratch,
                             &in_alt, s));
     const uint32_t* sorted_keys = in_alt ? w.keys_b : w.keys_a;
-    k_tile_offsets<<<blocks_for(z.tiles + 1, kThreads), kThreads, 0, s>>>(sorted_keys, entry_capacity, z.tiles,
-                                                                          tile_offsets);
-    RF_TRY(launch_status());
+    RF_TRY(launch_chained(k_tile_offsets, blocks_for(32 * (long long)(z.tiles + 1), kThreads), kThreads, 0, s, sorted_keys,
+                          entry_capacity, z.tiles, tile_offsets));
     // the raster's work queue: tiles by decreasing entry count
-    k_tile_order_keys<<<blocks_for(z.tiles, kThreads), kThreads, 0, s>>>(tile_offsets, z.tiles, w.order_keys_b,
-                                                                         w.order_vals_b);
-    RF_TRY(launch_status());
+    if (z.tiles <= kOrderBlockTiles)
+        return launch_chained(k_tile_order, 1, kOrderThreads, 0, s, tile_offsets, z.tiles,
+                              (uint32_t*)batch_tile_order(w, z));
+    RF_TRY(launch_chained(k_tile_order_keys, blocks_for(z.tiles, kThreads), kThreads, 0, s, tile_offsets, z.tiles,
+                          w.order_keys_b, w.order_vals_b));
     RF_TRY(radix_sort_pairs(w.order_keys_b, w.order_vals_b, w.order_keys, w.order_vals, z.tiles, kOrderKeyBits,
                             w.radix_scratch, &in_alt, s));
     return RF_OK;

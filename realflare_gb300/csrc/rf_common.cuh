@@ -38,6 +38,35 @@ inline int cuda_status(cudaError_t e) {
     } while (0)
 
 inline unsigned blocks_for(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
+
+// A chain of small kernels is launched so that a kernel may start while the one before it in the
+// stream still runs (programmatic dependent launch): its launch latency is then hidden. Every kernel
+// of such a chain calls chain_wait() first, before it touches memory, so each waits for all before it.
+template <class... Params, class... Args>
+int launch_chained(void (*kernel)(Params...), unsigned grid, int block, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchAttribute overlap = {};
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &overlap;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return cuda_status(e);
+    }
+    return launch_status();
+}
+__device__ __forceinline__ void chain_wait() {
+#if __CUDA_ARCH__ >= 900
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+#endif
+}
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 // The traces: threads of a block, ghost paths a thread may trace at once (rf_trace_core.cuh), and the
@@ -170,10 +199,11 @@ __device__ __forceinline__ float4 xyz_to_ap1(float x, float y, float z) {
 __device__ __constant__ static const unsigned char SUB_OFFSETS[15] = {0, 1, 0, 1, 2, 0, 3, 4, 1, 6, 2, 5, 0, 3, 7};
 
 // ---------------------------------------------------------------- batch workspace
-// Scratch of rf_bin_tiles_batch and rf_raster_batch (rf_bin.cu): pair counters and their
-// scan, the entry sort's buffers, the raster's tile order and its queue head.
+// Scratch of rf_bin_tiles_batch and rf_raster_batch (rf_bin.cu): pair rectangles, their blocks'
+// entry counts and scan, the entry sort's buffers, the raster's tile order and its queue head.
 struct BatchWorkspace {
-    uint32_t *counts, *scan_scratch, *keys_a, *keys_b, *vals_tmp, *radix_scratch;
+    unsigned long long* rects;
+    uint32_t *sums, *scan_scratch, *keys_a, *keys_b, *vals_tmp, *radix_scratch;
     uint32_t *order_keys, *order_vals, *order_keys_b, *order_vals_b, *queue;
     size_t bytes;
 };
