@@ -75,15 +75,10 @@ QPoint = QPointF
 def _hashable(cls):
     """Dataclass whose hash is computed from its field values (lists become tuples)."""
     cls = dataclass(eq=True)(cls)
+    names = tuple(f.name for f in dataclasses.fields(cls))
 
     def __hash__(self):
-        values = []
-        for f in dataclasses.fields(self):
-            v = getattr(self, f.name)
-            if isinstance(v, list):
-                v = tuple(v)
-            values.append(v)
-        return hash(tuple(values))
+        return hash(tuple([tuple(v) if isinstance(v, list) else v for v in [getattr(self, n) for n in names]]))
 
     cls.__hash__ = __hash__
     return cls

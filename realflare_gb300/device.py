@@ -17,7 +17,7 @@ from .data import RealflareError
 
 
 def require_cuda() -> torch.device:
-    if not torch.cuda.is_available():
+    if not (torch.cuda.is_initialized() or torch.cuda.is_available()):  # (the second asks the environment)
         raise RealflareError('no CUDA device: the render path runs on the GPU only')
     return torch.device('cuda', torch.cuda.current_device())
 
@@ -40,6 +40,23 @@ def to_device(array: np.ndarray, dtype=None) -> torch.Tensor:
     if dtype is not None:
         t = t.to(dtype)
     return t.to(require_cuda(), non_blocking=False)
+
+
+def upload(arrays: list, stream: int) -> tuple:
+    """Copies host arrays to the device in one transfer, for kernels on ``stream``: the device
+    buffer that holds them and each array's address (16-byte aligned). The copy is asynchronous,
+    from page-locked memory, where ``stream`` is the current stream, and so ordered before them."""
+    starts, size = [], 0
+    for a in arrays:
+        starts.append(size)
+        size += (a.nbytes + 15) & ~15
+    ordered = stream == stream_handle()
+    staging = torch.empty((max(size, 16),), dtype=torch.uint8, pin_memory=ordered)
+    host = staging.numpy()
+    for a, start in zip(arrays, starts):
+        host[start:start + a.nbytes] = np.ascontiguousarray(a).reshape(-1).view(np.uint8)
+    buffer = staging.to(require_cuda(), non_blocking=ordered)
+    return buffer, [buffer.data_ptr() + start for start in starts]
 
 
 class MemoryObject:

@@ -83,30 +83,34 @@ def elements(
     lens_elements.append(LensElement(height=sensor_length))
     glasses = _catalogue(glasses_path)
 
-    array = np.zeros(len(lens_elements), lens_element_dtype)
+    count = len(lens_elements)
+    array = np.zeros(count, lens_element_dtype)
     if not glasses:
         array[0]['coefficients'][0] = np.nan
-    offset = 0.0
-    for i, element in enumerate(lens_elements):
-        array[i]['radius'] = element.radius
-        array[i]['ior'] = element.refractive_index
-        array[i]['height'] = element.height
-        array[i]['center'] = offset + element.radius
-        if i < len(coating):
-            array[i]['coating'] = coating[i]
-        if i < len(coating_thickness) and coating_thickness[i] is not None:
-            t = coating_thickness[i]
-            if np.ndim(t) == 0:
-                array[i]['coating_layers'] = 1
-                array[i]['coating_thickness'][0] = t
-            else:
-                array[i]['coating_layers'] = 2
-                array[i]['coating_thickness'][:] = t[:2]
-        coefficients = _closest_coefficients(glasses_path, element.refractive_index, element.abbe_nr,
-                                             abbe_nr_adjustment)
-        if coefficients:
-            array[i]['coefficients'][:6] = coefficients
+    centers, offset = [], 0.0
+    for element in lens_elements:
+        centers.append(offset + element.radius)
         offset += element.distance
+    # (a whole column at a time: writing single records takes several us each)
+    array['radius'] = [e.radius for e in lens_elements]
+    array['ior'] = [e.refractive_index for e in lens_elements]
+    array['height'] = [e.height for e in lens_elements]
+    array['center'] = centers
+    coated = min(count, len(coating))
+    if coated:
+        array['coating'][:coated] = coating[:coated]
+    layers, thickness = [0] * count, [(0.0, 0.0)] * count
+    for i, t in enumerate(coating_thickness[:count]):
+        if t is not None:
+            single = isinstance(t, (int, float)) or np.ndim(t) == 0
+            layers[i], thickness[i] = (1, (t, 0.0)) if single else (2, tuple(np.broadcast_to(t[:2], 2)))
+    array['coating_layers'] = layers
+    array['coating_thickness'] = thickness
+    rows = [_closest_coefficients(glasses_path, e.refractive_index, e.abbe_nr, abbe_nr_adjustment)
+            for e in lens_elements]
+    known = [i for i, row in enumerate(rows) if row]
+    if known:
+        array['coefficients'][known, :6] = [rows[i] for i in known]
     return array
 
 

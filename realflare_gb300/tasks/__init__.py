@@ -32,7 +32,7 @@ from .._abi import (
 )
 from ..constants import LAMBDA_MID, light_spectrum
 from ..data import Project, QPointF, QSize, RealflareError
-from ..device import Image, MemoryObject, Rays, empty, ptr, require_cuda, stream_handle, to_device
+from ..device import Image, MemoryObject, Rays, empty, ptr, require_cuda, stream_handle, to_device, upload
 
 
 class Task:
@@ -70,13 +70,12 @@ class RaytracingTask(Task):
         if self.use_cache and self._cache is not None and self._cache[0] == key:
             return self._cache[1]
         a = inputs.args
-        elements = to_device(inputs.elements.view(np.uint8))
-        paths_t = to_device(inputs.paths)
-        wl = to_device(inputs.wavelengths)
         rays = empty((6, inputs.ray_count))
         if inputs.ray_count:
+            stream = self.stream
+            uploaded, (elements, paths_t, wl) = upload([inputs.elements, inputs.paths, inputs.wavelengths], stream)
             trace = self.lib.rf_trace_accurate if self.accurate else self.lib.rf_trace
-            check(trace(ptr(elements), ptr(paths_t), ptr(wl), ctypes.byref(a), ptr(rays), self.stream),
+            check(trace(elements, paths_t, wl, ctypes.byref(a), ptr(rays), stream),
                   'rf_trace_accurate' if self.accurate else 'rf_trace')
         shape = (a.path_count, a.wavelength_count, a.grid_count**2)
         result = Rays(rays, shape, args=key)
@@ -171,8 +170,9 @@ class RasterizingTask(Task):
             self._spectrum = to_device(light_spectrum())
         return self._spectrum
 
-    def setup(self, project: Project, rays: Rays):
-        """Quad setup and vertex setup: (bounds, intensities, vertexes) on the device."""
+    def setup(self, project: Project, rays: Rays, args=None):
+        """Quad setup and vertex setup: (bounds, intensities, vertexes) on the device. ``args``: the
+        project's raster arguments, where they are at hand."""
         P, W, R = rays.shape
         G = project.render.grid_count
         Q = (G - 1) ** 2
@@ -181,7 +181,7 @@ class RasterizingTask(Task):
         inten = self._buffer('intensities', P * Q * W)
         check(self.lib.rf_quad_setup(ptr(rays.tensor), P, W, G, area, min_area, ptr(bounds), ptr(inten), self.stream),
               'rf_quad_setup')
-        a = prepare.raster_args(project, P, W, (1, 1))
+        a = args or prepare.raster_args(project, P, W, (1, 1))
         vertexes = self._buffer('vertexes', (P * R * W + 1) * 8)
         check(self.lib.rf_vertex(ptr(rays.tensor), ptr(inten), P, W, G, a.screen_transform, a.width, a.height,
                                  ptr(vertexes), self.stream), 'rf_vertex')
@@ -235,7 +235,7 @@ class RasterizingTask(Task):
         P, W, R = rays.shape
         gt = ghost.tensor
         a = prepare.raster_args(project, P, W, tuple(gt.shape[:2]))
-        bounds, inten, vertexes = self.setup(project, rays)
+        bounds, inten, vertexes = self.setup(project, rays, a)
         offsets, entries = self.bin(a, bounds, vertexes)
         order = self.order(offsets)
         check(self.lib.rf_raster_ordered(ptr(vertexes), ptr(offsets), ptr(entries), ptr(order), ptr(gt),
