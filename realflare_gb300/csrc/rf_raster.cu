@@ -672,7 +672,7 @@ constexpr size_t raster_smem_bytes(int maxW, int WS) {
 
 // Tile (tx, ty), whose entries are tile_entries[begin, end). smem4 holds the dynamic shared
 // memory (raster_smem_bytes), next_block four shared counters. kS: the anti-aliasing sample
-// count when known at compile time (1), else 0 (p.S). kTex: sample the ghost texture through
+// count when known at compile time, else 0 (p.S). kTex: sample the ghost texture through
 // p.ghost_tex.
 template <int T, int kS, bool kTex, int kPix>
 __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint32_t begin, uint32_t end,
@@ -896,24 +896,55 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
                     }
                 }
             }
+            if constexpr (kS != 1) {
+                // Several samples per pixel: the same two steps, with each pixel's number of covered samples
+                // less one in bit planes. Zoom lens, 1920 x 1080, 4 samples: 21.3 -> 19.0 ms (lanes that
+                // missed a record waited for the others: 71 % shaded); 601 x 403, 2 samples 0.296 -> 0.240.
+                const float cx = rx0 + (float)((lane & 7) * S + S / 2), cy = ry0 + (float)((lane >> 3) * S + S / 2);
+                const f2 cx2 = pk(cx, cx), cy2 = pk(cy, cy);
+                unsigned cov[2], h0[2], h1[2], h2[2];
 #pragma unroll
-            for (int m = 0; m < kBatchRecords / 32 && in_image && kS != 1; m++) {
-                unsigned bits = sel[m];
-                while (bits) {  // in increasing record order: the reference's summation order
-                    const int b = __ffs(bits) - 1;
-                    const int j = m * 32 + b;
-                    const bool is_whole = (whole[m] >> b) & 1u;
-                    bits &= bits - 1;
-                    const Rec& r = recs[j];
-                    RF_STAT(if (lane == 0) { st_iter++; st_whole += is_whole; })
-                    int hits = S;
-                    if (!is_whole) hits = sample_hits<T>(r, S, (wild[m] >> b) & 1u, rx0, ry0, sx0, sy0, lane);
-                    if (hits == 0) continue;
-                    RF_STAT(st_frag++; st_frag_whole += is_whole;)
+                for (int m = 0; m < 2; m++) {
+                    const Rec* half = recs + 32 * m;
+                    const unsigned far = __brev(wild[m]), all = __brev(whole[m]);
+                    unsigned c = all, a0 = all, a1 = all, a2 = all;
+#pragma unroll 1
+                    for (unsigned part = __brev(sel[m] & ~whole[m]); part;) {
+                        const int b = __clz(part);
+                        const unsigned bit = 0x80000000u >> b;
+                        part ^= bit;
+                        const int hits = sample_hits<T>(half[b], S, (far & bit) != 0, rx0, ry0, sx0, sy0, lane);
+                        if (hits > 0) {
+                            c |= bit;
+                            if ((hits - 1) & 1) a0 |= bit;
+                            if (kS != 2 && ((hits - 1) & 2)) a1 |= bit;
+                            if (kS != 2 && kS != 4 && ((hits - 1) & 4)) a2 |= bit;
+                        }
+                    }
+                    cov[m] = in_image ? c : 0;
+                    h0[m] = a0, h1[m] = a1, h2[m] = a2;
+                    RF_STAT(if (lane == 0) { st_iter += __popc(sel[m]); st_whole += __popc(whole[m]); })
+                }
+                const int full = S - 1;  // a plane beyond it is not the record's
+                const Rec* half = recs;
+                for (;;) {  // in increasing record order: the reference's summation order
+                    if (cov[0] == 0) {
+                        cov[0] = cov[1], h0[0] = h0[1], h1[0] = h1[1], h2[0] = h2[1];
+                        cov[1] = 0;
+                        half += 32;
+                        if (cov[0] == 0) break;
+                    }
+                    const int j = __clz(cov[0]);
+                    const unsigned bit = 0x80000000u >> j;
+                    cov[0] ^= bit;
+                    const Rec& r = half[j];
+                    const int hits = 1 + (((h0[0] & bit ? 1 : 0) + (kS != 2 && (h1[0] & bit) ? 2 : 0) +
+                                          (kS != 2 && kS != 4 && (h2[0] & bit) ? 4 : 0)) & full);
+                    RF_STAT(st_frag++; const int jj = (int)(&r - recs); st_frag_whole += (whole[jj >> 5] >> (jj & 31)) & 1u;
+                            if (lane == __ffs(__activemask()) - 1) st_steps++;)
                     f2 we, wo;
-                    const float cx = rx0 + (float)((lane & 7) * S + S / 2), cy = ry0 + (float)((lane >> 3) * S + S / 2);
                     float general = 1.0f;
-                    mean_value_weights(r, pk(cx, cx), pk(cy, cy), we, wo, general);
+                    mean_value_weights(r, cx2, cy2, we, wo, general);
                     RF_STAT({
                         const bool z = blend4(we, wo, r.rs) <= 0.0f;
                         st_zero += z;
@@ -1620,7 +1651,10 @@ template <int T>
 int launch_raster(const float* vertexes, const uint32_t* offsets, const uint32_t* entries, const uint32_t* order,
                   const float* ghost, const float* spectrum, RasterParams p, float* image, cudaStream_t s) {
     if (p.S == 1) return launch_raster_s<T, 1>(vertexes, offsets, entries, order, ghost, spectrum, p, image, s);
-    return launch_raster_s<T, 0>(vertexes, offsets, entries, order, ghost, spectrum, p, image, s);
+    // (the sample count known: its tests unroll. Zoom lens, 4 samples: 21.7 ms with a runtime count)
+    if (p.S == 2) return launch_raster_s<T, 2>(vertexes, offsets, entries, order, ghost, spectrum, p, image, s);
+    if (p.S == 4) return launch_raster_s<T, 4>(vertexes, offsets, entries, order, ghost, spectrum, p, image, s);
+    return launch_raster_s<T, 8>(vertexes, offsets, entries, order, ghost, spectrum, p, image, s);
 }
 
 template <int T, int kS, bool kTex>
