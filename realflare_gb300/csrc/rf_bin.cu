@@ -77,16 +77,6 @@ __global__ void __launch_bounds__(kThreads) k_bin_masks(const float4* __restrict
         }
 }
 
-__device__ __forceinline__ void divide(long long a, int b, long long& q, int& r) {
-    if (a >> 32 == 0) {
-        q = (unsigned)a / (unsigned)b;
-        r = (int)((unsigned)a - (unsigned)q * (unsigned)b);
-    } else {
-        q = a / b;
-        r = (int)(a - q * b);
-    }
-}
-
 // Tile rectangle of one (primitive, wavelength pair); false when it contributes nothing.
 __device__ __forceinline__ bool pair_tile_rect(const float4* __restrict__ bounds, const float4* __restrict__ vtx,
                                                long long pair, const BinGeometry& g, int& tx0, int& tx1,

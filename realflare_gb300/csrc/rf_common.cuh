@@ -67,7 +67,7 @@ __device__ __forceinline__ void chain_wait() {
     cudaGridDependencySynchronize();
 #endif
 }
-inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
+__host__ __device__ inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 // The traces: threads of a block, ghost paths a thread may trace at once (rf_trace_core.cuh), and the
 // blocks per SM that a launch should have, below which a block takes fewer paths.
@@ -109,6 +109,18 @@ __device__ __forceinline__ int find_frame(const rf_frame* __restrict__ frames, i
         else hi = mid - 1;
     }
     return lo;
+}
+
+// Quotient and remainder of a >= 0 by b > 0, in 32 bits where a allows (a 64-bit division takes several
+// times as many instructions).
+__device__ __forceinline__ void divide(long long a, int b, long long& q, int& r) {
+    if (a >> 32 == 0) {
+        q = (unsigned)a / (unsigned)b;
+        r = (int)((unsigned)a - (unsigned)q * (unsigned)b);
+    } else {
+        q = a / b;
+        r = (int)(a - q * b);
+    }
 }
 
 // ---------------------------------------------------------------- integer semantics

@@ -23,8 +23,10 @@ __device__ __forceinline__ void quad_setup_one(const float* __restrict__ rays, i
                                                float* __restrict__ inten, long long pq) {
     const int Q = (G - 1) * (G - 1), R = G * G;
     if (pq >= (long long)P * Q) return;
-    const int path = (int)(pq / Q), quad = (int)(pq % Q);
-    const int row = quad / (G - 1), col = quad % (G - 1);
+    long long path;
+    int quad;
+    divide(pq, Q, path, quad);
+    const int row = quad / (G - 1), col = quad - row * (G - 1);
     int v[4];
     v[0] = row * G + col;
     v[1] = v[0] + 1;
@@ -37,10 +39,25 @@ __device__ __forceinline__ void quad_setup_one(const float* __restrict__ rays, i
     float bx0 = INFINITY, by0 = INFINITY, bx1 = -INFINITY, by1 = -INFINITY;
     int invalid_rrel = 0;
     bool culled = false;
-    for (int w = 0; w < W; w++) {
+    // a primitive's intensities are W consecutive floats: four are stored at once where they are aligned
+    // (4.5 M primitives of 16 wavelengths: 0.55 -> 0.43 ms)
+    const bool four = (W & 3) == 0 && aligned16(inten);
+    float held[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    auto put = [&](int w, float v) {
         const size_t prim_index = (size_t)pq * W + w;
+        if (!four) {
+            inten[prim_index] = v;
+            return;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (k == (w & 3)) held[k] = v;
+        if ((w & 3) == 3)
+            *reinterpret_cast<float4*>(inten + prim_index - 3) = make_float4(held[0], held[1], held[2], held[3]);
+    };
+    for (int w = 0; w < W; w++) {
         if (culled) {
-            inten[prim_index] = 0.0f;  // the reference leaves these entries stale
+            put(w, 0.0f);  // the reference leaves these entries stale
             continue;
         }
         const size_t off = ((size_t)path * W + w) * R;
@@ -73,12 +90,12 @@ __device__ __forceinline__ void quad_setup_one(const float* __restrict__ rays, i
             rr[3] = rr[2];
         } else {
             culled = true;
-            inten[prim_index] = 0.0f;
+            put(w, 0.0f);
             continue;
         }
         if (rr[0] > 1.0f && rr[1] > 1.0f && rr[2] > 1.0f && rr[3] > 1.0f) invalid_rrel++;
         float area_actual = fmaxf(area, min_area);
-        inten[prim_index] = area_actual > 0.0f ? area_orig / area_actual : 0.0f;
+        put(w, area_actual > 0.0f ? area_orig / area_actual : 0.0f);
         bx0 = fminf(bx0, fminf(fminf(px[0], px[1]), fminf(px[2], px[3])));
         by0 = fminf(by0, fminf(fminf(py[0], py[1]), fminf(py[2], py[3])));
         bx1 = fmaxf(bx1, fmaxf(fmaxf(px[0], px[1]), fmaxf(px[2], px[3])));
@@ -106,15 +123,15 @@ __device__ __forceinline__ void vertex_one(const float* __restrict__ rays, const
         vertexes[2 * n_rays + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
-    const int ray_id = (int)(i % R);
-    const long long pw = i / R;
-    const int w = (int)(pw % W);
-    const int path = (int)(pw / W);
-    const long long vi = ((long long)path * R + ray_id) * W + w;  // the reference's order
+    long long pw, path;
+    int ray_id, w;
+    divide(i, R, pw, ray_id);
+    divide(pw, W, path, w);
+    const long long vi = (path * R + ray_id) * W + w;  // the reference's order
     const float refl = __ldg(rays + 5 * n_rays + i);
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = make_float4(0.f, refl, 0.f, 0.f);
     if (!isnan(refl)) {
-        const int x = ray_id % G, y = ray_id / G;
+        const int y = ray_id / G, x = ray_id - y * G;
         int nb[4];
         nb[0] = (y - 1) * (G - 1) + (x - 1);
         nb[1] = nb[0] + 1;
