@@ -2,24 +2,28 @@
 //
 // A 2-D transform of a [batch][h][w] complex64 array is a pass over rows and a pass over the
 // rows of the transposed result. A block holds a few rows in shared memory, each thread eight
-// elements of one row in registers: radix-8 steps (the last one 8, 4 or 2) in Stockham's
-// self-sorting order, so data stays in natural order and a row of 512 takes three exchanges
-// instead of nine. What the callers do before, between and after transforms happens in the
-// passes: a pass loads elements through a program, transforms, optionally multiplies and
-// transforms the same rows again, and stores through the program.
+// elements of one row in registers: three radix-2 levels at a time in Stockham's self-sorting
+// order, so data stays in natural order and a row of 512 takes three exchanges instead of nine. The
+// butterflies are those of the plain radix-2 decimation in time, operation for operation, and the
+// passes come in the order of separate 2-D transforms: gradients through the ghost texture can
+// amplify its last bits a thousandfold (the light's are small differences of large terms), so these
+// stay what they were. What the callers do before and after transforms happens in the passes: a
+// pass loads elements through a program, transforms and stores through the program.
 //  * the starburst power spectrum (realflare/api/tasks/starburst.py:45-81): load
 //    A * exp(i pi (x^2 + y^2) / (lambda d)), store |F|^2 at the fftshift position;
 //  * the ghost texture's fractional Fourier transform (realflare/api/tasks/ghost.py:13-36
 //    and realflare/utils/frft.py:20-62, Ozaktas et al. 1996 chirp convolution): three 2-D
-//    transforms of the aperture and one of a chirp in four passes (rf_ghost_frft).
+//    transforms of the aperture and one of a chirp in six passes, or two and one in four
+//    (rf_ghost_frft).
 // Rows whose length is a power of two from 8 on are transformed directly; any other length from
 // 2 to 4096 runs Bluestein's chirp-z form (Bluestein 1970): with w_m = exp(d pi i m^2 / n),
 // X_k = w_k sum_j (x_j w_j) conj(w_{k-j}), a linear convolution evaluated by transforms of a
 // power-of-two length M >= 2n - 1; the filter's transform is evaluated once per block.
 //
 // What bounds it: latency on the small textures (a few microseconds per launch), shared memory and
-// the transposing stores on batches. 512 x 512, 16 spectra 161 -> 70 us (both passes); a 256 x
-// 256 ghost texture 74 -> 34 us in 13 -> 4 launches; 702 x 954 (chirp-z) 757 -> 322 us.
+// the transposing stores on batches. 512 x 512, 16 spectra 161 -> 74 us (both passes); a 256 x 256
+// ghost texture 74 -> 42 us in 13 -> 6 launches; 702 x 954 (chirp-z) 761 -> 384 us. (Radix-8
+// butterflies and merged passes took 34 and 322 us, with other last bits.)
 #include <complex>
 #include <math.h>
 
@@ -32,14 +36,17 @@ namespace {
 
 constexpr int kMaxN = 4096;
 
+// Complex product with one product of each part rounded and the other fused, fixed here so that the
+// results' bits do not depend on how a compiler contracts the expression around: of the imaginary
+// part a.y b.x is rounded (kFlip: a.x b.y).
+template <bool kFlip = false>
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)),
+                       kFlip ? __fmaf_rn(a.y, b.x, __fmul_rn(a.x, b.y)) : __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-// a * (0, s) for s = +-1
-__device__ __forceinline__ float2 rot90(float2 a, float s) { return make_float2(-s * a.y, s * a.x); }
-
+__device__ __forceinline__ float square_sum(float x, float y) { return __fmaf_rn(x, x, __fmul_rn(y, y)); }
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y)); }
 // ---------------------------------------------------------------- row transforms
 // How rows of length n are transformed: M is the power-of-two length, n itself or the convolution's.
 struct RowPlan {
@@ -72,41 +79,11 @@ RowPlan row_plan(int n, long long rows) {
     return p;
 }
 
-// the 4-point transform of v[0], v[q], v[2 q], v[3 q]
-template <int q>
-__device__ __forceinline__ void fft4(float2* v, float s) {
-    const float2 a = cadd(v[0], v[2 * q]), b = csub(v[0], v[2 * q]);
-    const float2 c = cadd(v[q], v[3 * q]), d = rot90(csub(v[q], v[3 * q]), s);
-    v[0] = cadd(a, c);
-    v[q] = cadd(b, d);
-    v[2 * q] = csub(a, c);
-    v[3 * q] = csub(b, d);
-}
-// the 8-point transform, in place, natural order
-__device__ __forceinline__ void fft8(float2 v[8], float s) {
-    const float r = 0.70710678118654752f;
-    float2 e[4], o[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        e[k] = cadd(v[k], v[k + 4]);
-        o[k] = csub(v[k], v[k + 4]);
-    }
-    o[1] = make_float2(r * (o[1].x - s * o[1].y), r * (o[1].y + s * o[1].x));     // exp(s i pi / 4)
-    o[2] = rot90(o[2], s);
-    o[3] = make_float2(-r * (o[3].x + s * o[3].y), r * (s * o[3].x - o[3].y));    // exp(s 3 i pi / 4)
-    fft4<1>(e, s);
-    fft4<1>(o, s);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        v[2 * k] = e[k];
-        v[2 * k + 1] = o[k];
-    }
-}
-
 // Transform of one row of length M by its M / 8 threads: thread t brings elements t + r M / 8 in v;
 // the result lies in x (padded), natural order. s: the exponent's sign. tw[k] = exp(-2 pi i k / M).
 // Every thread of the block takes part (rows share the barriers; rows of at most 32 threads lie
 // within a warp).
+template <bool kFlip>
 __device__ __forceinline__ void fft_row(float2 v[8], float2* x, const float2* tw, int M, int log_m, int t, float s) {
     const int eighth = M >> 3;
     const bool in_warp = eighth <= 32;
@@ -116,59 +93,73 @@ __device__ __forceinline__ void fft_row(float2 v[8], float2* x, const float2* tw
         else
             __syncthreads();
     };
+    auto twiddle = [&](int k) {
+        const float2 w = tw[k];
+        return make_float2(w.x, s < 0.0f ? w.y : -w.y);
+    };
+    auto butterfly = [](float2& a, float2& b, float2 w) {
+        const float2 u = a, c = cmul<kFlip>(b, w);
+        a = cadd(u, c);
+        b = csub(u, c);
+    };
+    // At ns, blocks of ns elements are transformed; a level combines elements M / 2 apart, at place k of
+    // their blocks, with the twiddle exp(s 2 pi i k / (2 ns)) = tw[k M / (2 ns)].
     int log_ns = 0;
     for (int rest = log_m; rest > 0;) {
         if (log_ns > 0) {
 #pragma unroll
             for (int r = 0; r < 8; r++) v[r] = x[padded(t + r * eighth)];
         }
-        const int ns = 1 << log_ns;
+        const int ns = 1 << log_ns, sh = log_m - log_ns;
         if (rest >= 3) {
             const int k = t & (ns - 1);
-            if (log_ns > 0) {
-                const int step = k << (log_m - log_ns - 3);
+            {
+                const float2 w = twiddle(k << (sh - 1));
 #pragma unroll
-                for (int r = 1; r < 8; r++) {
-                    const float2 w = tw[r * step];
-                    v[r] = cmul(v[r], make_float2(w.x, -s * w.y));
-                }
+                for (int r = 0; r < 4; r++) butterfly(v[r], v[r + 4], w);
             }
-            fft8(v, s);
+            {
+                const float2 w0 = twiddle(k << (sh - 2)), w1 = twiddle((k + ns) << (sh - 2));
+                butterfly(v[0], v[2], w0);
+                butterfly(v[1], v[3], w0);
+                butterfly(v[4], v[6], w1);
+                butterfly(v[5], v[7], w1);
+            }
+            butterfly(v[0], v[1], twiddle(k << (sh - 3)));
+            butterfly(v[4], v[5], twiddle((k + ns) << (sh - 3)));
+            butterfly(v[2], v[3], twiddle((k + 2 * ns) << (sh - 3)));
+            butterfly(v[6], v[7], twiddle((k + 3 * ns) << (sh - 3)));
             const int d = ((t - k) << 3) + k;
             sync();  // everything is read
+            const float2 out[8] = {v[0], v[4], v[2], v[6], v[1], v[5], v[3], v[7]};
 #pragma unroll
-            for (int r = 0; r < 8; r++) x[padded(d + (r << log_ns))] = v[r];
+            for (int r = 0; r < 8; r++) x[padded(d + (r << log_ns))] = out[r];
             log_ns += 3;
             rest -= 3;
-        } else if (rest == 2) {  // two 4-point steps: elements t + (q + 2 r) M / 8, r = 0 .. 3
+        } else if (rest == 2) {  // two levels of two groups: elements t + (q + 2 r) M / 8, r = 0 .. 3
 #pragma unroll
             for (int q = 0; q < 2; q++) {
-                const int j = t + q * eighth, k = j & (ns - 1), step = k << (log_m - log_ns - 2);
-#pragma unroll
-                for (int r = 1; r < 4; r++) {
-                    const float2 w = tw[r * step];
-                    v[q + 2 * r] = cmul(v[q + 2 * r], make_float2(w.x, -s * w.y));
-                }
-                fft4<2>(v + q, s);
+                const int k = (t + q * eighth) & (ns - 1);
+                const float2 w = twiddle(k << (sh - 1));
+                butterfly(v[q], v[q + 4], w);
+                butterfly(v[q + 2], v[q + 6], w);
+                butterfly(v[q], v[q + 2], twiddle(k << (sh - 2)));
+                butterfly(v[q + 4], v[q + 6], twiddle((k + ns) << (sh - 2)));
             }
             sync();
 #pragma unroll
             for (int q = 0; q < 2; q++) {
                 const int j = t + q * eighth, k = j & (ns - 1), d = ((j - k) << 2) + k;
+                const float2 out[4] = {v[q], v[q + 4], v[q + 2], v[q + 6]};
 #pragma unroll
-                for (int r = 0; r < 4; r++) x[padded(d + (r << log_ns))] = v[q + 2 * r];
+                for (int r = 0; r < 4; r++) x[padded(d + (r << log_ns))] = out[r];
             }
             log_ns += 2;
             rest = 0;
-        } else {  // four 2-point steps: elements t + (q + 4 r) M / 8, r = 0, 1
+        } else {  // one level of four groups: elements t + (q + 4 r) M / 8, r = 0, 1
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int j = t + q * eighth, k = j & (ns - 1);
-                const float2 w = tw[k << (log_m - log_ns - 1)];
-                const float2 b = cmul(v[q + 4], make_float2(w.x, -s * w.y)), a = v[q];
-                v[q] = cadd(a, b);
-                v[q + 4] = csub(a, b);
-            }
+            for (int q = 0; q < 4; q++)
+                butterfly(v[q], v[q + 4], twiddle(((t + q * eighth) & (ns - 1)) << (sh - 1)));
             sync();
 #pragma unroll
             for (int q = 0; q < 4; q++) {
@@ -191,8 +182,7 @@ __device__ __forceinline__ float2 bluestein_chirp(int m, int n, float d) {
     return make_float2(cs, sn);
 }
 
-// One pass. Program: float2 load(row, i); float sign(row), the first transform's direction (+-1, 0:
-// none); float sign2(row), a second transform's (0: none) of mid(row, i, value); and
+// One pass. Program: float2 load(row, i); float sign(row), the transform's direction (+-1); and
 // store(row, i, value).
 template <class Program>
 __global__ void __launch_bounds__(1024) k_fft_pass(const Program p, int rows, int n, int M, int log_m,
@@ -216,16 +206,17 @@ __global__ void __launch_bounds__(1024) k_fft_pass(const Program p, int rows, in
         tw[k] = make_float2(cs, sn);
     }
     float2 v[8];
+    const float s = p.sign(row0);  // (programs keep directions equal within a block)
     if (chirp_z) {
-        // b_m = conj(w_m) of direction -1 for |m| < n, wrapped; of direction +1 it is the conjugate,
-        // and so is its transform (b is symmetric)
+        // b_m = conj(w_m) for |m| < n, wrapped
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < 8; r++) {
             const int i = t + r * eighth, m = i < n ? i : M - i;
-            v[r] = m < n ? bluestein_chirp(m, n, 1.0f) : make_float2(0.0f, 0.0f);
+            const float2 w = bluestein_chirp(m, n, s);
+            v[r] = m < n ? make_float2(w.x, -w.y) : make_float2(0.0f, 0.0f);
         }
-        fft_row(v, x, tw, M, log_m, t, -1.0f);
+        fft_row<false>(v, x, tw, M, log_m, t, -1.0f);
         if (g == 0)
 #pragma unroll
             for (int r = 0; r < 8; r++) {
@@ -236,57 +227,24 @@ __global__ void __launch_bounds__(1024) k_fft_pass(const Program p, int rows, in
     __syncthreads();
     cudaGridDependencySynchronize();  // the passes before are complete
     const float inv_m = 1.0f / (float)M;
-    // element i of the transformed row
-    auto result = [&](const float2* from, int i, float s) {
-        const float2 c = from[padded(i)];
-        if (!chirp_z) return c;
-        return cmul(bluestein_chirp(i, n, s), make_float2(c.x * inv_m, c.y * inv_m));
-    };
-    // transforms the row whose elements t + r M / 8 are in v
-    auto transform = [&](float s) {
-        if (!chirp_z) {
-            fft_row(v, x, tw, M, log_m, t, s);
-            return;
-        }
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-            const int i = t + r * eighth;
-            if (i < n) v[r] = cmul(v[r], bluestein_chirp(i, n, s));
-        }
-        fft_row(v, x, tw, M, log_m, t, -1.0f);
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-            const int i = padded(t + r * eighth);
-            const float2 f = filter[i];
-            v[r] = cmul(x[i], make_float2(f.x, -s * f.y));
-        }
-        fft_row(v, x, tw, M, log_m, t, 1.0f);
-    };
-    // (directions are those of the block's first row: programs keep them equal within a block)
-    const float s1 = p.sign(row0), s2 = p.sign2(row0);
 #pragma unroll
     for (int r = 0; r < 8; r++) {
         const int i = t + r * eighth;
         v[r] = valid && i < n ? p.load(row, i) : make_float2(0.0f, 0.0f);
+        if (chirp_z && i < n) v[r] = cmul(v[r], bluestein_chirp(i, n, s));
     }
-    if (s1 != 0.0f) transform(s1);
-    if (s2 != 0.0f) {
+    if (chirp_z)
+        fft_row<false>(v, x, tw, M, log_m, t, -1.0f);
+    else
+        fft_row<true>(v, x, tw, M, log_m, t, s);
+    if (chirp_z) {
 #pragma unroll
         for (int r = 0; r < 8; r++) {
-            const int i = t + r * eighth;
-            v[r] = valid && i < n ? p.mid(row, i, s1 != 0.0f ? result(x, i, s1) : v[r]) : make_float2(0.0f, 0.0f);
+            const int i = padded(t + r * eighth);
+            v[r] = cmul<true>(x[i], filter[i]);
         }
-        if (s1 != 0.0f && eighth <= 32) __syncwarp();
-        transform(s2);
-    }
-    const float s = s2 != 0.0f ? s2 : s1;
-    if (s == 0.0f) {  // no transform: the rows pass through
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-            const int i = t + r * eighth;
-            if (valid && i < n) p.store(row, i, v[r]);
-        }
-        return;
+        if (eighth <= 32) __syncwarp();
+        fft_row<false>(v, x, tw, M, log_m, t, 1.0f);
     }
     if (chirp_z) cudaTriggerProgrammaticLaunchCompletion();
     __syncthreads();  // every row of the block is transformed
@@ -295,7 +253,9 @@ __global__ void __launch_bounds__(1024) k_fft_pass(const Program p, int rows, in
     const int log_rows = __ffs(rows_per_block) - 1;
     for (int e = threadIdx.x; e < n << log_rows; e += blockDim.x) {
         const int q = e & (rows_per_block - 1), i = e >> log_rows;
-        if (row0 + q < rows) p.store(row0 + q, i, result(sm + q * row_size, i, s));
+        if (row0 + q >= rows) continue;
+        const float2 c = sm[q * row_size + padded(i)];
+        p.store(row0 + q, i, chirp_z ? cmul<true>(bluestein_chirp(i, n, s), make_float2(c.x * inv_m, c.y * inv_m)) : c);
     }
 }
 
@@ -307,7 +267,7 @@ int launch_pass(const Program& program, long long rows, const RowPlan& plan, cud
         RF_TRY(cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem)));
     const long long blocks = (rows + plan.rows_per_block - 1) / plan.rows_per_block;
     // programmatic dependent launch: the launch latency and the tables overlap the pass before
-    // (256 x 256 ghost texture, four passes: 40.7 -> 34.4 us)
+    // (256 x 256 ghost texture, four passes of radix 8: 40.7 -> 34.4 us)
     cudaLaunchAttribute overlap = {};
     overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     overlap.val.programmaticStreamSerializationAllowed = 1;
@@ -330,9 +290,7 @@ struct TransposePass {
     int n, rows;
     float s, scale;
     __device__ float sign(int) const { return s; }
-    __device__ float sign2(int) const { return 0.0f; }
     __device__ float2 load(int row, int i) const { return in[(size_t)row * n + i]; }
-    __device__ float2 mid(int, int, float2 v) const { return v; }
     __device__ void store(int row, int i, float2 v) const {
         const unsigned b = (unsigned)row / (unsigned)rows, r = (unsigned)row % (unsigned)rows;
         out[((size_t)b * n + i) * rows + r] = make_float2(v.x * scale, v.y * scale);
@@ -354,17 +312,15 @@ struct StarburstRows {  // aperture * chirp, batch = wavelength
     int w, h;
     float phase_scale[256];  // per batch: 1 / (lambda d); the phase is pi * scale * r^2
     __device__ float sign(int) const { return -1.0f; }
-    __device__ float sign2(int) const { return 0.0f; }
     __device__ float2 load(int row, int i) const {
         const int b = (int)((unsigned)row / (unsigned)h), y = (int)((unsigned)row % (unsigned)h);
         const float x0 = w > 1 ? -1.0f + (float)i * (2.0f / (float)(w - 1)) : -1.0f;
         const float y0 = h > 1 ? -1.0f + (float)y * (2.0f / (float)(h - 1)) : -1.0f;
         const float a = __ldg(aperture + (size_t)y * w + i);
         float s, c;
-        sincospif(phase_scale[b] * (x0 * x0 + y0 * y0), &s, &c);
+        sincospif(phase_scale[b] * square_sum(x0, y0), &s, &c);
         return make_float2(a * c, a * s);
     }
-    __device__ float2 mid(int, int, float2 v) const { return v; }
     __device__ void store(int row, int i, float2 v) const {
         const unsigned b = (unsigned)row / (unsigned)h, y = (unsigned)row % (unsigned)h;
         out[((size_t)b * w + i) * h + y] = v;
@@ -375,15 +331,13 @@ struct PowerColumns {  // |v|^2 at the fftshift position of the [batch][h][w] im
     float* out;
     int w, h;
     __device__ float sign(int) const { return -1.0f; }
-    __device__ float sign2(int) const { return 0.0f; }
     __device__ float2 load(int row, int i) const { return in[(size_t)row * h + i]; }
-    __device__ float2 mid(int, int, float2 v) const { return v; }
     __device__ void store(int row, int i, float2 v) const {
         const unsigned b = (unsigned)row / (unsigned)w;
         const int x = (int)((unsigned)row % (unsigned)w);
         int ys = i + h / 2, xs = x + w / 2;
         ys -= ys >= h ? h : 0, xs -= xs >= w ? w : 0;
-        out[((size_t)b * h + ys) * w + xs] = v.x * v.x + v.y * v.y;
+        out[((size_t)b * h + ys) * w + xs] = square_sum(v.x, v.y);
     }
 };
 
@@ -401,28 +355,27 @@ struct FrftArgs {
     int w, h;
     float first;  // the transform before the chirp convolution (normalize() of frft.py): +-1, 0 none
     bool flip;
-    float c1, c2, ortho, first_scale;
+    float c1, c2, ortho;
     float2 scale;
     float norm;
 };
-// Passes 1 and 2 carry two arrays, the aperture's (rows below `split`) and chirp 2's, so that a launch
-// holds the work of both; `split` is a multiple of the rows per block. numpy's fftshift moves
-// element i to (i + n / 2) mod n: output i reads (i + n - n / 2) mod n.
-struct FrftRows1 {  // rows y: the shifted aperture's first transform; chirp 2's
+// The first two passes carry two arrays, the aperture's (rows below `split`) and chirp 2's, so that a
+// launch holds the work of both; `split` is a multiple of the rows per block. numpy's fftshift
+// moves element i to (i + n / 2) mod n: output i reads (i + n - n / 2) mod n.
+struct FrftRows1 {  // rows y: of the shifted aperture, times chirp 1 without a first transform; of chirp 2
     FrftArgs f;
     const float* aperture;
     float2 *a, *b;  // out [w][h]
     int split;
-    __device__ float sign(int row) const { return row < split ? f.first : -1.0f; }
-    __device__ float sign2(int) const { return 0.0f; }
+    __device__ float sign(int row) const { return row < split && f.first != 0.0f ? f.first : -1.0f; }
     __device__ float2 load(int row, int x) const {
         if (row >= split) return chirp_value((int)(row - split), x, f.w, f.h, f.c2);
         if (row >= f.h) return make_float2(0.0f, 0.0f);
-        int y = (int)row;
-        if (f.flip) y = f.h - 1 - y, x = f.w - 1 - x;
-        return make_float2(__ldg(aperture + (size_t)((y + f.h - f.h / 2) % f.h) * f.w + (x + f.w - f.w / 2) % f.w), 0.0f);
+        const int sy = f.flip ? f.h - 1 - row : row, sx = f.flip ? f.w - 1 - x : x;
+        const float2 v = make_float2(
+            __ldg(aperture + (size_t)((sy + f.h - f.h / 2) % f.h) * f.w + (sx + f.w - f.w / 2) % f.w), 0.0f);
+        return f.first != 0.0f ? v : cmul(v, chirp_value(row, x, f.w, f.h, f.c1));
     }
-    __device__ float2 mid(int, int, float2 v) const { return v; }
     __device__ void store(int row, int x, float2 v) const {
         if (row >= split)
             b[(size_t)x * f.h + (row - split)] = v;
@@ -430,54 +383,45 @@ struct FrftRows1 {  // rows y: the shifted aperture's first transform; chirp 2's
             a[(size_t)x * f.h + row] = v;
     }
 };
-struct FrftColumns2 {  // columns x: the first transform's, chirp 1, the forward transform's; chirp 2's
+struct FrftColumns2 {  // columns x of the same; a first transform's result times chirp 1
     FrftArgs f;
     const float2* a;  // [w][h]
     float2* b;        // [w][h], in place
     float2* out;      // [h][w]
     int split;
-    __device__ float sign(int row) const { return row < split ? f.first : -1.0f; }
-    __device__ float sign2(int row) const { return row < split ? -1.0f : 0.0f; }
+    __device__ float sign(int row) const { return row < split && f.first != 0.0f ? f.first : -1.0f; }
     __device__ float2 load(int row, int y) const {
         if (row >= split) return b[(size_t)(row - split) * f.h + y];
         return row < f.w ? a[(size_t)row * f.h + y] : make_float2(0.0f, 0.0f);
     }
-    __device__ float2 mid(int row, int y, float2 v) const {
-        return cmul(make_float2(v.x * f.first_scale, v.y * f.first_scale), chirp_value(y, (int)row, f.w, f.h, f.c1));
-    }
     __device__ void store(int row, int y, float2 v) const {
+        v = make_float2(v.x * f.ortho, v.y * f.ortho);
         if (row >= split)
-            b[(size_t)(row - split) * f.h + y] = make_float2(v.x * f.ortho, v.y * f.ortho);
+            b[(size_t)(row - split) * f.h + y] = v;
         else if (row < f.w)
-            out[(size_t)y * f.w + row] = v;
+            out[(size_t)y * f.w + row] = f.first != 0.0f ? cmul(v, chirp_value(y, row, f.w, f.h, f.c1)) : v;
     }
 };
-struct FrftRows3 {  // rows y: the forward transform's, times chirp 2's transform, the inverse's
+struct FrftRows3 {  // rows y: the product of the two transforms, transformed back
     FrftArgs f;
     const float2 *a, *b;  // [h][w], [w][h]
     float2* out;          // [w][h]
-    __device__ float sign(int) const { return -1.0f; }
-    __device__ float sign2(int) const { return 1.0f; }
-    __device__ float2 load(int row, int x) const { return a[(size_t)row * f.w + x]; }
-    __device__ float2 mid(int row, int x, float2 v) const {
-        return cmul(make_float2(v.x * f.ortho, v.y * f.ortho), b[(size_t)x * f.h + row]);
-    }
+    __device__ float sign(int) const { return 1.0f; }
+    __device__ float2 load(int row, int x) const { return cmul<true>(a[(size_t)row * f.w + x], b[(size_t)x * f.h + row]); }
     __device__ void store(int row, int x, float2 v) const { out[(size_t)x * f.h + row] = v; }
 };
-struct FrftColumns4 {  // columns x: the inverse transform's; |fftshift(scale * chirp 1 * data)| * norm
+struct FrftColumns4 {  // columns x of that; |fftshift(scale * chirp 1 * data)| * norm
     FrftArgs f;
     const float2* a;  // [w][h]
     float* out;
     __device__ float sign(int) const { return 1.0f; }
-    __device__ float sign2(int) const { return 0.0f; }
     __device__ float2 load(int row, int y) const { return a[(size_t)row * f.h + y]; }
-    __device__ float2 mid(int, int, float2 v) const { return v; }
     __device__ void store(int row, int y, float2 v) const {
         v = make_float2(v.x * f.ortho, v.y * f.ortho);
         const float2 r = cmul(cmul(f.scale, chirp_value(y, (int)row, f.w, f.h, f.c1)), v);
         int ys = y + f.h / 2, xs = (int)row + f.w / 2;
         ys -= ys >= f.h ? f.h : 0, xs -= xs >= f.w ? f.w : 0;
-        out[(size_t)ys * f.w + xs] = sqrtf(r.x * r.x + r.y * r.y) * f.norm;
+        out[(size_t)ys * f.w + xs] = sqrtf(square_sum(r.x, r.y)) * f.norm;
     }
 };
 
@@ -549,7 +493,6 @@ extern "C" int rf_ghost_frft(const float* aperture, int32_t width, int32_t heigh
         a = rel - 3;
         f.first = 1.0f;
     }
-    f.first_scale = f.first != 0.0f ? f.ortho : 1.0f;
     const double phi = a * M_PI / 2.0;
     const double cot = 1.0 / std::tan(phi);
     const double sq = std::sqrt(1.0 + cot * cot);
@@ -558,14 +501,16 @@ extern "C" int rf_ghost_frft(const float* aperture, int32_t width, int32_t heigh
     f.c2 = (float)sq;
     f.scale = make_float2((float)scale.real(), (float)scale.imag());
     f.norm = (float)std::sqrt((double)n);  // ghost.py:33-35
-    // fft2 = fftn(chirp1 * A); fft1 = fftn(chirp2); A = ifftn(fft1 * fft2). The first transform's
-    // columns, chirp 1 and the forward transform's columns share a pass, as do the forward
-    // transform's rows, the product with chirp 2's transform and the inverse's rows.
+    // fft2 = fftn(chirp1 * A); fft1 = fftn(chirp2); A = ifftn(fft1 * fft2)
     const RowPlan by_row = row_plan(width, 2LL * height), by_column = row_plan(height, 2LL * width);
     const long long split1 = (height + by_row.rows_per_block - 1) / by_row.rows_per_block * by_row.rows_per_block;
     const long long split2 = (width + by_column.rows_per_block - 1) / by_column.rows_per_block * by_column.rows_per_block;
     RF_TRY(launch_pass(FrftRows1{f, aperture, S0, S1, (int)split1}, split1 + height, by_row, s));
     RF_TRY(launch_pass(FrftColumns2{f, S0, S1, S2, (int)split2}, split2 + width, by_column, s));
+    if (f.first != 0.0f) {  // the first transform is done: the forward one
+        RF_TRY(launch_pass(TransposePass{S2, S0, width, height, -1.0f, 1.0f}, height, row_plan(width, height), s));
+        RF_TRY(launch_pass(TransposePass{S0, S2, height, width, -1.0f, f.ortho}, width, row_plan(height, width), s));
+    }
     RF_TRY(launch_pass(FrftRows3{f, S2, S1, S0}, height, row_plan(width, height), s));
     return launch_pass(FrftColumns4{f, S0, texture}, width, row_plan(height, width), s);
 }
