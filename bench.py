@@ -930,6 +930,7 @@ def main() -> None:
                 'accurate_frame_ms': (elapsed / args.steps * 1e3 - last['trace'] + trace_accurate_ms
                                       if trace_accurate_ms else None),
                 'note': ('interactions: 1 + elements + 2 (b1 - b2) loop steps per ray that reaches the sensor; '
+                         'counted one path at a time, as the reference traces (shared legs are traced once); '
                          'issue_active: ncu smsp__issue_active of k_trace, 1024^2 / 48-ghost case; accurate_ms: '
                          'rf_trace_accurate (double-precision ray geometry) on the same frame'),
             },
