@@ -51,6 +51,32 @@ __device__ __forceinline__ void rot2(float& x, float& y, float angle) {
     y = ny;
 }
 
+// Two FP32 values per register pair: each packed instruction does two lookups' terms in one issue slot,
+// each rounded as the scalar operation.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pk(float lo, float hi) {
+    f2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float lo2(f2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi2(f2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+    f2 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
 // Per-sample terms of k_starburst that do not depend on the pixel, tabulated per CTA in
 // chunks of kStarburstChunk samples: the light's XYZ weight at the sample's spectral position, the
 // spectrum plane's offset, and the texel scale 0.5 * size / (chromatic scale) per axis.
@@ -68,10 +94,11 @@ struct alignas(16) StarburstSample {
 // 1.5 * 2^23 (floors and conversions would go to the unit that also serves the jitter's
 // noise); coordinates too large for that come out as integers outside every texture.
 //
-// What bounds it: instruction issue. 1920 x 1080, 100 samples, 16 spectra, no jitter: 733 -> 310 us
-// (lookups were evaluated with 64-bit indices and divisions); 1000 samples with jitter 16.1 -> 10.6
-// ms (12.3 with the sines' slow path, their quadrant by three selections and a general square root;
-// the two noise hashes are most of what is left); 512 x 512 with jitter and rotation 434 -> 256 us.
+// What bounds it: instruction issue. 1920 x 1080, 100 samples, 16 spectra, no jitter: 733 -> 280 us
+// (310 with scalar coordinates, texel rows and sums instead of packed ones, four samples unrolled instead
+// of two; before that, lookups with 64-bit indices and divisions); 1000 samples with jitter 16.1 ->
+// 10.0 ms (12.3 with the sines' slow path, their quadrant by three selections and a general square root;
+// the two noise hashes are most of what is left); 512 x 512 with jitter and rotation 434 -> 254 us.
 template <bool kJitter, bool kRotate, int kPix>
 __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const float* __restrict__ spectrum,
                                                    const float* __restrict__ light, rf_starburst_args a,
@@ -82,7 +109,7 @@ __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const floa
     const bool inside = x < a.width && y < a.height;  // (every thread takes part in the table fills)
     const int w = a.spectrum_width, h = a.spectrum_height;
     // texel coordinates less a half: see above
-    const float cu = 0.5f * (float)w - 1.0f, cv = 0.5f * (float)h - 1.0f;
+    const f2 centre = pk(0.5f * (float)w - 1.0f, 0.5f * (float)h - 1.0f);
     float nx, ny[kPix], hash0[kPix];
 #pragma unroll
     for (int k = 0; k < kPix; k++) {
@@ -91,9 +118,7 @@ __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const floa
         hash0[k] = (float)x * 112.9898f + (float)(y + 16 * k) * 179.233f;
     }
     nx = (nx - a.offset[0]) / fmaxf(a.scale[0], 1.17549435e-38f);
-    float acc[kPix][3];
-#pragma unroll
-    for (int k = 0; k < kPix; k++) acc[k][0] = acc[k][1] = acc[k][2] = 0.0f;
+    f2 acc[3] = {0, 0, 0};  // of both pixels
     for (int t0 = 0; t0 < a.samples; t0 += kStarburstChunk) {
         const int n = min(kStarburstChunk, a.samples - t0);
         __syncthreads();  // the previous chunk's table is no longer read
@@ -125,12 +150,13 @@ __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const floa
         }
         __syncthreads();
         if (!inside) continue;
-#pragma unroll 2
+#pragma unroll 4
         for (int i = 0; i < n; i++) {
             const float4 e0 = *reinterpret_cast<const float4*>(&tab[i].x);
-            const float2 e1 = *reinterpret_cast<const float2*>(&tab[i].su);
+            const f2 scale = *reinterpret_cast<const f2*>(&tab[i].su);
             const float seed = (float)((t0 + i) * 4);
             const float* plane = spectrum + (size_t)(unsigned)__float_as_int(e0.w) * (unsigned)h * w;
+            float fi[2] = {0.0f, 0.0f};
 #pragma unroll
             for (int k = 0; k < kPix; k++) {
                 float px = nx, py = ny[k];
@@ -147,34 +173,37 @@ __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const floa
                     const float angle = sign * a.rotation * (1.0f - (a.rotation_weight == 1.0f ? r : powf(r, a.rotation_weight)));
                     rot2(px, py, angle);
                 }
-                const float u = fmaf(px, e1.x, cu), v = fmaf(py, e1.y, cv);
-                const float tu = u + 12582912.0f, tv = v + 12582912.0f;
-                const int i0 = __float_as_int(tu) - 0x4b400000, j0 = __float_as_int(tv) - 0x4b400000;
-                const float fa = (u - (tu - 12582912.0f)) + 0.5f, fb = (v - (tv - 12582912.0f)) + 0.5f;
-                const float* q = plane + max(j0, 0) * w;
-                float t00 = 0.0f, t10 = 0.0f, t01 = 0.0f, t11 = 0.0f;
+                const f2 big = pk(12582912.0f, 12582912.0f);
+                const f2 uv = fma2(pk(px, py), scale, centre), near = add2(uv, big);
+                const int i0 = __float_as_int(lo2(near)) - 0x4b400000, j0 = __float_as_int(hi2(near)) - 0x4b400000;
+                const f2 frac = add2(sub2(uv, sub2(near, big)), pk(0.5f, 0.5f));
+                f2 left = 0, right = 0;  // texels (i0, j0), (i0, j0 + 1); (i0 + 1, ...)
                 if ((unsigned)i0 < (unsigned)(w - 1) && (unsigned)j0 < (unsigned)(h - 1)) {
-                    q += i0;
-                    t00 = __ldg(q);
-                    t10 = __ldg(q + 1);
-                    t01 = __ldg(q + w);
-                    t11 = __ldg(q + w + 1);
+                    const float* q = plane + (j0 * w + i0);
+                    left = pk(__ldg(q), __ldg(q + w));
+                    right = pk(__ldg(q + 1), __ldg(q + w + 1));
                 } else {
                     const bool i0_in = (unsigned)i0 < (unsigned)w, i1_in = i0 >= -1 && i0 < w - 1;
                     const bool j0_in = (unsigned)j0 < (unsigned)h, j1_in = j0 >= -1 && j0 < h - 1;
                     if (!((i0_in || i1_in) && (j0_in || j1_in))) continue;  // outside: adds 0
+                    const float* q = plane + max(j0, 0) * w;
                     const float* q1 = j0 < 0 ? q : q + w;
-                    if (i0_in && j0_in) t00 = __ldg(q + i0);
-                    if (i1_in && j0_in) t10 = __ldg(q + i0 + 1);
-                    if (i0_in && j1_in) t01 = __ldg(q1 + i0);
-                    if (i1_in && j1_in) t11 = __ldg(q1 + i0 + 1);
+                    left = pk(i0_in && j0_in ? __ldg(q + i0) : 0.0f, i0_in && j1_in ? __ldg(q1 + i0) : 0.0f);
+                    right = pk(i1_in && j0_in ? __ldg(q + i0 + 1) : 0.0f, i1_in && j1_in ? __ldg(q1 + i0 + 1) : 0.0f);
                 }
-                const float top = fmaf(fa, t10 - t00, t00), bottom = fmaf(fa, t11 - t01, t01);
-                const float fi = fmaf(fb, bottom - top, top);
-                acc[k][0] += e0.x * fi;
-                acc[k][1] += e0.y * fi;
-                acc[k][2] += e0.z * fi;
+                const f2 rows = fma2(pk(lo2(frac), lo2(frac)), sub2(right, left), left);
+                fi[k] = fmaf(hi2(frac), hi2(rows) - lo2(rows), lo2(rows));
             }
+            if (kPix == 1) {
+                acc[0] = pk(fmaf(e0.x, fi[0], lo2(acc[0])), 0.0f);
+                acc[1] = pk(fmaf(e0.y, fi[0], lo2(acc[1])), 0.0f);
+                acc[2] = pk(fmaf(e0.z, fi[0], lo2(acc[2])), 0.0f);
+                continue;
+            }
+            const f2 f = pk(fi[0], fi[1]);
+            acc[0] = fma2(pk(e0.x, e0.x), f, acc[0]);
+            acc[1] = fma2(pk(e0.y, e0.y), f, acc[1]);
+            acc[2] = fma2(pk(e0.z, e0.z), f, acc[2]);
         }
     }
     if (!inside) return;
@@ -183,7 +212,7 @@ __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const floa
         if (y + 16 * k >= a.height) break;
         float v[3];
 #pragma unroll
-        for (int c = 0; c < 3; c++) v[c] = acc[k][c] / (float)a.samples;
+        for (int c = 0; c < 3; c++) v[c] = (k ? hi2(acc[c]) : lo2(acc[c])) / (float)a.samples;
         if (!isnan(a.vignetting[0])) {
             const float sdf = sqrtf(nx * nx + ny[k] * ny[k]) - 0.0f;
             const float f = smoothstepf(a.vignetting[1], a.vignetting[0], sdf);
@@ -365,8 +394,8 @@ extern "C" int rf_starburst(const float* spectrum, const float* light_spectrum, 
     // rotation 0 and a non-negative weight the angle is +-0 * (1 - noise^weight) = +-0: the
     // jitter and the rotation then leave the position unchanged and their noise is skipped.
     const bool jitter = a.blur != 0.0f, rotate = a.rotation != 0.0f || !(a.rotation_weight >= 0.0f);
-    // Plain lookups take two pixels per thread where the image still fills the SMs (2048^2 0.71 ->
-    // 0.59 ms, 640 x 480 0.068 -> 0.061, 300^2 0.035 -> 0.039); with noise one is faster (512^2
+    // Plain lookups take two pixels per thread where the image still fills the SMs (scalar form: 2048^2
+    // 0.71 -> 0.59 ms, 640 x 480 0.068 -> 0.061, 300^2 0.035 -> 0.039); with noise one is faster (512^2
     // 0.32 against 0.39 ms).
     const bool two = !jitter && !rotate && (long long)a.width * a.height >= 200000;
     const dim3 grid((a.width + 15) / 16, (a.height + (two ? 31 : 15)) / (two ? 32 : 16));
