@@ -12,46 +12,7 @@
 namespace rf {
 namespace {
 
-__device__ __forceinline__ float fract1(float x) { return fminf(x - floorf(x), 0x1.fffffep-1f); }
-// sin(x) for the noise hash. The hash's arguments reach 10^6, where sinf takes its slow
-// reduction path; here x is reduced by pi/2 with the Cody-Waite method (W. J. Cody and
-// W. Waite, Software Manual for the Elementary Functions, 1980) using a three-part split of
-// pi/2 (C1 = fl(pi/2), C2 = fl(pi/2 - C1), C3 = fl(pi/2 - C1 - C2), which sum to pi/2 within
-// 1e-23, computed in 200-bit arithmetic) and fused multiply-adds, then sin or cos of the
-// remainder (|r| <= pi/4 + a rounding) by quadrant. Accurate to a few ulps for |x| < 2^22.
-__device__ __forceinline__ float hash_sin(float x) {
-    const float k = rintf(x * 0x1.45f306p-1f);  // x * 2 / pi
-    float r = fmaf(-k, 0x1.921fb6p+0f, x);
-    r = fmaf(-k, -0x1.777a5cp-25f, r);
-    r = fmaf(-k, -0x1.ee59dap-50f, r);
-    // (beyond 2^22 k loses bits and r grows, to less than 10^5 for every sample index there is: no
-    // case for the slow reduction path, which the compiler then leaves out)
-    __builtin_assume(fabsf(r) < 1.0e5f);
-    float sr, cr;
-    sincosf(r, &sr, &cr);
-    const unsigned q = (unsigned)(int)k;
-    return __uint_as_float(__float_as_uint((q & 1) ? cr : sr) ^ (q & 2) << 30);
-}
-// noise(x, y, z) of noise.cl:1-5, with the terms in x and y given
-__device__ __forceinline__ float noise_at(float xy, float z) {
-    return fract1(hash_sin(xy + z * 237.212f) * 43758.5453f);
-}
-__device__ __forceinline__ float noise3(float x, float y, float z) {
-    return noise_at(x * 112.9898f + y * 179.233f, z);
-}
-__device__ __forceinline__ void ndc_of(int px, int py, int w, int h, float& nx, float& ny) {
-    nx = 2.0f * ((float)px / (float)(w - 1)) - 1.0f;
-    ny = 2.0f * ((float)py / (float)(h - 1)) - 1.0f;
-}
-__device__ __forceinline__ void rot2(float& x, float& y, float angle) {
-    float s, c;
-    sincosf(angle, &s, &c);
-    const float nx = x * c + y * s, ny = y * c - x * s;
-    x = nx;
-    y = ny;
-}
-
-// Two FP32 values per register pair: each packed instruction does two lookups' terms in one issue slot,
+// Two FP32 values per register pair: each packed instruction does two terms in one issue slot,
 // each rounded as the scalar operation.
 using f2 = unsigned long long;
 __device__ __forceinline__ f2 pk(float lo, float hi) {
@@ -71,10 +32,62 @@ __device__ __forceinline__ f2 sub2(f2 a, f2 b) {
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
     f2 d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
+}
+
+__device__ __forceinline__ float fract1(float x) { return fminf(x - floorf(x), 0x1.fffffep-1f); }
+// The noise hash's sine. Its arguments x reach 10^6, where sinf takes its slow
+// reduction path; here x is reduced by pi/2 with the Cody-Waite method (W. J. Cody and
+// W. Waite, Software Manual for the Elementary Functions, 1980) using a three-part split of
+// pi/2 (C1 = fl(pi/2), C2 = fl(pi/2 - C1), C3 = fl(pi/2 - C1 - C2), which sum to pi/2 within
+// 1e-23, computed in 200-bit arithmetic) and fused multiply-adds, then sin or cos of the
+// remainder (|r| <= pi/4 + a rounding) by quadrant. Accurate to a few ulps for |x| < 2^22.
+// The sine of a reduced argument r = x - k pi / 2.
+__device__ __forceinline__ float sine_of(float r, float k) {
+    // (beyond 2^22 k loses bits and r grows, to less than 10^5 for every sample index there is: no
+    // case for the slow reduction path, which the compiler then leaves out)
+    __builtin_assume(fabsf(r) < 1.0e5f);
+    float sr, cr;
+    sincosf(r, &sr, &cr);
+    const unsigned q = (unsigned)(int)k;
+    return __uint_as_float(__float_as_uint((q & 1) ? cr : sr) ^ (q & 2) << 30);
+}
+// noise(x, y, z) of noise.cl:1-5 at z and z + 1, with the terms in x and y given
+__device__ __forceinline__ void noise_at(float xy, float z, float& n0, float& n1) {
+    auto both = [](float v) { return pk(v, v); };
+    const f2 x = fma2(pk(z, z + 1.0f), both(237.212f), both(xy)), t = mul2(x, both(0x1.45f306p-1f));  // x * 2 / pi
+    const float k0 = rintf(lo2(t)), k1 = rintf(hi2(t));
+    const f2 k = pk(k0, k1);
+    f2 r = fma2(k, both(-0x1.921fb6p+0f), x);
+    r = fma2(k, both(0x1.777a5cp-25f), r);
+    r = fma2(k, both(0x1.ee59dap-50f), r);
+    const f2 v = mul2(pk(sine_of(lo2(r), k0), sine_of(hi2(r), k1)), both(43758.5453f));
+    n0 = fract1(lo2(v));
+    n1 = fract1(hi2(v));
+}
+__device__ __forceinline__ float noise3(float x, float y, float z) {
+    float n0, n1;
+    noise_at(x * 112.9898f + y * 179.233f, z, n0, n1);
+    return n0;
+}
+__device__ __forceinline__ void ndc_of(int px, int py, int w, int h, float& nx, float& ny) {
+    nx = 2.0f * ((float)px / (float)(w - 1)) - 1.0f;
+    ny = 2.0f * ((float)py / (float)(h - 1)) - 1.0f;
+}
+__device__ __forceinline__ void rot2(float& x, float& y, float angle) {
+    float s, c;
+    sincosf(angle, &s, &c);
+    const float nx = x * c + y * s, ny = y * c - x * s;
+    x = nx;
+    y = ny;
 }
 
 // Per-sample terms of k_starburst that do not depend on the pixel, tabulated per CTA in
@@ -97,8 +110,9 @@ struct alignas(16) StarburstSample {
 // What bounds it: instruction issue. 1920 x 1080, 100 samples, 16 spectra, no jitter: 733 -> 280 us
 // (310 with scalar coordinates, texel rows and sums instead of packed ones, four samples unrolled instead
 // of two; before that, lookups with 64-bit indices and divisions); 1000 samples with jitter 16.1 ->
-// 10.0 ms (12.3 with the sines' slow path, their quadrant by three selections and a general square root;
-// the two noise hashes are most of what is left); 512 x 512 with jitter and rotation 434 -> 254 us.
+// 9.8 ms (12.3 with the sines' slow path, their quadrant by three selections and a general square root;
+// 10.0 with one hash at a time; the two hashes are most of what is left); 512 x 512 with jitter and
+// rotation 434 -> 241 us.
 template <bool kJitter, bool kRotate, int kPix>
 __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const float* __restrict__ spectrum,
                                                    const float* __restrict__ light, rf_starburst_args a,
@@ -161,15 +175,17 @@ __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const floa
             for (int k = 0; k < kPix; k++) {
                 float px = nx, py = ny[k];
                 if (kJitter) {
-                    const float radius = a.blur * sqrt_rn(noise_at(hash0[k], seed));
-                    float sa, ca;
-                    sincospif(2.0f * noise_at(hash0[k], seed + 1.0f), &sa, &ca);
+                    float n0, n1, sa, ca;
+                    noise_at(hash0[k], seed, n0, n1);
+                    const float radius = a.blur * sqrt_rn(n0);
+                    sincospif(2.0f * n1, &sa, &ca);
                     px += ca * radius;
                     py += sa * radius;
                 }
                 if (kRotate) {  // (the chromatic scale is uniform: it can follow the rotation)
-                    const float sign = noise_at(hash0[k], seed + 2.0f) > 0.5f ? 1.0f : -1.0f;
-                    const float r = noise_at(hash0[k], seed + 3.0f);
+                    float n0, r;
+                    noise_at(hash0[k], seed + 2.0f, n0, r);
+                    const float sign = n0 > 0.5f ? 1.0f : -1.0f;
                     const float angle = sign * a.rotation * (1.0f - (a.rotation_weight == 1.0f ? r : powf(r, a.rotation_weight)));
                     rot2(px, py, angle);
                 }
