@@ -217,11 +217,13 @@ __device__ __forceinline__ void load_edges(const Rec& r, Edges& e) {
 }
 // The sample at tile-relative coordinates x = (x, x), y = (y, y), for records with flags & 1: the
 // edge values are exact integers (an exact zero is +0), so their signs are the reference's.
-__device__ __forceinline__ bool inside(const Edges& e, f2 x, f2 y) {
-    const f2 e0 = fma2(e.a0, y, fma2(e.b0, x, e.c0)), e1 = fma2(e.a1, y, fma2(e.b1, x, e.c1));
-    const float e2 = fmaf(e.a20, lo2(y), fmaf(e.b20, lo2(x), e.c20));
+__device__ __forceinline__ bool inside_at(f2 e0, f2 e1, float e2) {
     return (int)outside_sign((unsigned)e0, (unsigned)(e0 >> 32), (unsigned)e1, (unsigned)(e1 >> 32),
                              __float_as_uint(e2)) >= 0;
+}
+__device__ __forceinline__ bool inside(const Edges& e, f2 x, f2 y) {
+    return inside_at(fma2(e.a0, y, fma2(e.b0, x, e.c0)), fma2(e.a1, y, fma2(e.b1, x, e.c1)),
+                     fmaf(e.a20, lo2(y), fmaf(e.b20, lo2(x), e.c20)));
 }
 
 // Coverage of a block's samples (centre (xc, yc) as pairs, tile-relative, half extents
@@ -641,7 +643,7 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
 
 // How many of the S n-rook samples of this lane's pixel a record covers. (rx0, ry0): the block's first
 // sample relative to the tile, (sx0, sy0): the pixel's; wild: the record needs the exact test.
-template <int T>
+template <int T, int kS = 0>
 __device__ __forceinline__ int sample_hits(const Rec& r, int S, bool wild, float rx0, float ry0, int sx0, int sy0,
                                            int lane) {
     int hits = 0;
@@ -652,6 +654,30 @@ __device__ __forceinline__ int sample_hits(const Rec& r, int S, bool wild, float
     Edges e;
     load_edges(r, e);
     const float x = rx0 + (float)((lane & 7) * S), y = ry0 + (float)((lane >> 3) * S);
+    if constexpr (kS == 2 || kS == 4) {
+        // From the first sample on the edge values change by b + (the offsets' difference) a per sample:
+        // offsets 1, 0 (two samples) and 1, 2, 0, 3 (four, SUB_OFFSETS). All are integers below 2^24,
+        // exact as in inside(). Zoom lens, 4 samples: raster 19.0 -> 18.3 ms.
+        const f2 x2 = pk(x, x), y2 = pk(y + 1.0f, y + 1.0f);
+        f2 e0 = fma2(e.a0, y2, fma2(e.b0, x2, e.c0)), e1 = fma2(e.a1, y2, fma2(e.b1, x2, e.c1));
+        float e2 = fmaf(e.a20, lo2(y2), fmaf(e.b20, x, e.c20));
+        hits += inside_at(e0, e1, e2) ? 1 : 0;
+        auto next = [&](float offset) {
+            const f2 o = pk(offset, offset);
+            e0 = add2(e0, fma2(o, e.a0, e.b0));
+            e1 = add2(e1, fma2(o, e.a1, e.b1));
+            e2 += fmaf(offset, e.a20, e.b20);
+            hits += inside_at(e0, e1, e2) ? 1 : 0;
+        };
+        if constexpr (kS == 2) {
+            next(-1.0f);
+        } else {
+            next(1.0f);
+            next(-2.0f);
+            next(3.0f);
+        }
+        return hits;
+    }
     for (int s = 0; s < S; s++) {
         const float xs = x + (float)s, ys = y + (float)SUB_OFFSETS[S - 1 + s];
         hits += inside(e, pk(xs, xs), pk(ys, ys)) ? 1 : 0;
@@ -913,7 +939,7 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
                         const int b = __clz(part);
                         const unsigned bit = 0x80000000u >> b;
                         part ^= bit;
-                        const int hits = sample_hits<T>(half[b], S, (far & bit) != 0, rx0, ry0, sx0, sy0, lane);
+                        const int hits = sample_hits<T, kS>(half[b], S, (far & bit) != 0, rx0, ry0, sx0, sy0, lane);
                         if (hits > 0) {
                             c |= bit;
                             if ((hits - 1) & 1) a0 |= bit;
