@@ -194,7 +194,8 @@ class RasterizingTask(Task):
         check(self.lib.rf_raster_tiles(ctypes.byref(args), ctypes.byref(tile_size), ctypes.byref(tile_count)),
               'rf_raster_tiles')
         self.tile_size = tile_size.value
-        offsets = self._buffer('tile_offsets', tile_count.value + 1, torch.int32)
+        # exactly the image's tiles: the buffer itself only grows, and may be an earlier image's, with more of them
+        offsets = self._buffer('tile_offsets', tile_count.value + 1, torch.int32)[:tile_count.value + 1]
         count = ctypes.c_int64()
         for _ in range(3):
             cap = self._entry_capacity
@@ -215,7 +216,8 @@ class RasterizingTask(Task):
         raise RealflareError('rf_bin_tiles: workspace did not converge')
 
     def order(self, offsets):
-        """Tiles by decreasing entry count (rf_tile_order), for rf_raster_ordered."""
+        """Tiles by decreasing entry count (rf_tile_order), for rf_raster_ordered. ``offsets``: one more than the
+        image has tiles, as ``bin`` returns them."""
         tiles = offsets.numel() - 1
         ws_bytes = ctypes.c_size_t()
         check(self.lib.rf_tile_order_workspace_size(tiles, ctypes.byref(ws_bytes)), 'rf_tile_order_workspace_size')
