@@ -552,7 +552,7 @@ extern "C" int rf_bin_tiles(const float* bounds, const float* vertexes, const rf
     if (total == 0) return cuda_status(cudaMemsetAsync(tile_offsets, 0, sizeof(uint32_t) * (ntiles + 1), s));
     int bits = 0;
     while ((1LL << bits) < ntiles) bits++;
-    const int passes = (bits + 7) / 8;
+    const int passes = total > 1 ? (bits + 7) / 8 : 0;  // (the sort moves nothing where there is one entry)
     // arrange the ping-pong buffers so that the sorted values land in tile_entries
     uint32_t* vals_first = (passes % 2 == 0) ? tile_entries : w.vals_tmp;
     uint32_t* vals_alt = (passes % 2 == 0) ? w.vals_tmp : tile_entries;
