@@ -1191,8 +1191,14 @@ constexpr int kRedStride = 36;
 // rows of a warp's transpose buffer: the 5 attribute gradients and the 4 corner weights
 constexpr int kRedRows = kGradAttrs + 4;
 // adds scale * g to a vertex's attributes: floats 2 to 6 of (pos.xy, uv.xy, rrel, reflectance,
-// intensity, pad)
-__device__ __forceinline__ void add_gradients(float* vertex, const float g[kGradAttrs], float scale) {
+// intensity, pad). vectors: the vertexes start on 16-byte boundaries, as the vector additions
+// need (two instead of five; a buffer that starts elsewhere gets scalar ones).
+__device__ __forceinline__ void add_gradients(float* vertex, const float g[kGradAttrs], float scale, bool vectors) {
+    if (!vectors) {
+#pragma unroll
+        for (int a = 0; a < kGradAttrs; a++) atomicAdd(vertex + 2 + a, g[a] * scale);
+        return;
+    }
     asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(vertex + 2), "f"(g[0] * scale), "f"(g[1] * scale)
                  : "memory");
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(vertex + 4), "f"(g[2] * scale),
@@ -1471,8 +1477,9 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? 3 : 2)
             const float t = tbuf[slot * kBatchRecords + j];
             const int offset = corner == 0 ? 0 : (corner == 1 ? 1 : (corner == 2 ? 1 + p.G : p.G));
             float* v = grad_vtx + 8 * (vbase_buf[slot * kBatchRecords + j] + (long long)offset * p.W);
-            add_gradients(v, g, 1.0f - t);
-            if (t != 0.0f) add_gradients(v + 8, g, t);
+            const bool vectors = aligned16(grad_vtx);
+            add_gradients(v, g, 1.0f - t, vectors);
+            if (t != 0.0f) add_gradients(v + 8, g, t, vectors);
         }
     }
 }
@@ -1824,7 +1831,8 @@ extern "C" int rf_raster_backward(const float* vertexes, const uint32_t* tile_of
     using namespace rf;
     if (!vertexes || !tile_offsets || !ghost || !spectrum || !args || !image || !grad_image || !grad_vertexes)
         return RF_ERR_INVALID_ARG;
-    if (!aligned16(vertexes) || !aligned16(image) || !aligned16(grad_image)) return RF_ERR_INVALID_ARG;
+    if (!aligned16(vertexes) || !aligned16(image) || !aligned16(grad_image) || ((uintptr_t)grad_vertexes & 3u) != 0)
+        return RF_ERR_INVALID_ARG;
     RasterParams p;
     if (!make_params(*args, p)) return RF_ERR_INVALID_ARG;
     if (p.WS > kBatchRecords || p.maxW * p.WS > 4096) return RF_ERR_INVALID_ARG;
