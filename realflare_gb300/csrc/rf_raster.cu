@@ -564,16 +564,19 @@ __device__ __forceinline__ bool zero_record(const RasterParams& p, const Rec& r,
     return rl.x <= 0.0f && rl.y <= 0.0f && rl.z <= 0.0f && rl.w <= 0.0f;
 }
 // Whether the housing falloff is 1 and no clamp acts at any covered pixel of a record with one
-// sample per pixel: every corner's rrel <= 0.95 (ramp >= 1), intensity and reflectance >= 0, and
-// the quad strictly convex. Inside it, off its edges, the cross products a_i share one sign, so
+// sample per pixel: every corner's rrel <= 0.95 (ramp >= 1), intensity and reflectance >= 0, all of
+// them finite, and the quad strictly convex. Inside it, off its edges, the cross products a_i share one sign, so
 // the normalised weights are positive up to rounding and the ramp stays >= 1 up to a rounding,
 // where the smoothstep is 1 to second order. On an edge (a_i = 0: the rare path of the weights)
-// a clockwise quad's weights mix signs, and mean_value_weights asks for the general form.
+// a clockwise quad's weights mix signs, and mean_value_weights asks for the general form. A corner
+// that is NaN (infinite at both wavelengths: an element of height 0) makes every fragment of the
+// general form 0, by its clamps.
 __device__ __forceinline__ bool inside_housing(const Rec& r) {
-    const float4 rl = ld4(r.rs), in = ld4(r.inten), rf = ld4(r.refl);
-    const float ramp = fminf(fminf(rl.x, rl.y), fminf(rl.z, rl.w));
-    const float low = fminf(fminf(fminf(in.x, in.y), fminf(in.z, in.w)), fminf(fminf(rf.x, rf.y), fminf(rf.z, rf.w)));
-    return low >= 0.0f && ramp >= 1.0f;
+    auto within = [](float4 v, float low) {  // (false with a NaN)
+        return v.x >= low && v.y >= low && v.z >= low && v.w >= low &&
+               fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)) <= 3.40282347e38f;
+    };
+    return within(ld4(r.rs), 1.0f) && within(ld4(r.inten), 0.0f) && within(ld4(r.refl), 0.0f);
 }
 
 // edges, bounds and flags of a record whose corners are stored; (ox, oy): the tile's first sample;
