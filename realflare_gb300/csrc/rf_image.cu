@@ -92,12 +92,13 @@ __device__ __forceinline__ void rot2(float& x, float& y, float angle) {
 
 // Per-sample terms of k_starburst that do not depend on the pixel, tabulated per CTA in
 // chunks of kStarburstChunk samples: the light's XYZ weight at the sample's spectral position, the
-// spectrum plane's offset, and the texel scale 0.5 * size / (chromatic scale) per axis.
+// spectrum plane's number, the texel scale 0.5 * size / (chromatic scale) per axis, and the
+// reciprocal of the chromatic scale.
 constexpr int kStarburstChunk = 256;
 struct alignas(16) StarburstSample {
     float x, y, z;
     int plane;
-    float su, sv, pad0, pad1;
+    float su, sv, inv_scale, pad;
 };
 
 // The sum over samples of light x bilinear spectrum lookup. A position p (in [-1, 1]) divided by the
@@ -105,7 +106,8 @@ struct alignas(16) StarburstSample {
 // multiply-add per axis instead of a division and four roundings. The first texel of the
 // footprint is the nearest integer of the texel coordinate less a half, read from the sum with
 // 1.5 * 2^23 (floors and conversions would go to the unit that also serves the jitter's
-// noise); coordinates too large for that come out as integers outside every texture.
+// noise); coordinates too large for that come out as integers outside every texture with sides
+// below 2^22. kWide: a spectrum with a longer side or a plane of 2^31 texels or more, by the general lookup.
 //
 // What bounds it: instruction issue. 1920 x 1080, 100 samples, 16 spectra, no jitter: 733 -> 280 us
 // (310 with scalar coordinates, texel rows and sums instead of packed ones, four samples unrolled instead
@@ -113,7 +115,7 @@ struct alignas(16) StarburstSample {
 // 9.8 ms (12.3 with the sines' slow path, their quadrant by three selections and a general square root;
 // 10.0 with one hash at a time; the two hashes are most of what is left); 512 x 512 with jitter and
 // rotation 434 -> 241 us.
-template <bool kJitter, bool kRotate, int kPix>
+template <bool kJitter, bool kRotate, int kPix, bool kWide = false>
 __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const float* __restrict__ spectrum,
                                                    const float* __restrict__ light, rf_starburst_args a,
                                                    float4* __restrict__ image) {
@@ -159,7 +161,8 @@ __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const floa
             e.x = sample_linear(light, RF_SPECTRUM_WIDTH, 1, 4, 0, step, 0.0f, false);
             e.y = sample_linear(light, RF_SPECTRUM_WIDTH, 1, 4, 1, step, 0.0f, false);
             e.z = sample_linear(light, RF_SPECTRUM_WIDTH, 1, 4, 2, step, 0.0f, false);
-            e.pad0 = e.pad1 = 0.0f;
+            e.inv_scale = (float)RF_LAMBDA_MID * inv_scale;
+            e.pad = 0.0f;
             tab[i] = e;
         }
         __syncthreads();
@@ -188,6 +191,11 @@ __global__ void __launch_bounds__(256, kPix == 2 ? 4 : 7) k_starburst(const floa
                     const float sign = n0 > 0.5f ? 1.0f : -1.0f;
                     const float angle = sign * a.rotation * (1.0f - (a.rotation_weight == 1.0f ? r : powf(r, a.rotation_weight)));
                     rot2(px, py, angle);
+                }
+                if (kWide) {
+                    const float k_inv = tab[i].inv_scale;
+                    fi[k] = sample_linear(plane, w, h, 1, 0, px * k_inv * 0.5f + 0.5f, py * k_inv * 0.5f + 0.5f, false);
+                    continue;
                 }
                 const f2 big = pk(12582912.0f, 12582912.0f);
                 const f2 uv = fma2(pk(px, py), scale, centre), near = add2(uv, big);
@@ -410,12 +418,16 @@ extern "C" int rf_starburst(const float* spectrum, const float* light_spectrum, 
     // rotation 0 and a non-negative weight the angle is +-0 * (1 - noise^weight) = +-0: the
     // jitter and the rotation then leave the position unchanged and their noise is skipped.
     const bool jitter = a.blur != 0.0f, rotate = a.rotation != 0.0f || !(a.rotation_weight >= 0.0f);
+    // Lookups by 32-bit offsets and texel coordinates to 2^22 (k_starburst); beyond, one kernel for all
+    // settings (the noise then multiplies a radius or an angle of 0).
+    const int longest = a.spectrum_width > a.spectrum_height ? a.spectrum_width : a.spectrum_height;
+    const bool wide = longest >= (1 << 22) || (long long)a.spectrum_width * a.spectrum_height > 0x7fffffffLL;
     // Plain lookups take two pixels per thread where the image still fills the SMs (scalar form: 2048^2
     // 0.71 -> 0.59 ms, 640 x 480 0.068 -> 0.061, 300^2 0.035 -> 0.039); with noise one is faster (512^2
     // 0.32 against 0.39 ms).
-    const bool two = !jitter && !rotate && (long long)a.width * a.height >= 200000;
+    const bool two = !wide && !jitter && !rotate && (long long)a.width * a.height >= 200000;
     const dim3 grid((a.width + 15) / 16, (a.height + (two ? 31 : 15)) / (two ? 32 : 16));
-    const auto kernel = two ? k_starburst<false, false, 2>
+    const auto kernel = wide ? k_starburst<true, true, 1, true> : two ? k_starburst<false, false, 2>
                             : (jitter ? (rotate ? k_starburst<true, true, 1> : k_starburst<true, false, 1>)
                                       : (rotate ? k_starburst<false, true, 1> : k_starburst<false, false, 1>));
     kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(spectrum, light_spectrum, a, (float4*)image);
