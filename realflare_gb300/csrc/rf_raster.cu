@@ -156,6 +156,7 @@ struct RasterParams {
     float intensity, ghost_scale;
     int ghost_w, ghost_h;
     bool safe_screen;
+    bool ghost_large;  // the ghost texture has a side of 2^22 texels or more, or 2^31 texels (ghost_sample)
     unsigned long long ghost_tex;  // texture object over the ghost texture (the kTex kernels)
 };
 
@@ -382,7 +383,7 @@ __device__ __forceinline__ float blend4(f2 we, f2 wo, const float* v) {
 // be taken, with a fraction of 1: the same value), found by adding and subtracting 1.5 * 2^23,
 // in packed operations (a floor would go to the same unit as the reciprocals). Returns the
 // footprint's centre (i0 + 1, j0 + 1) and the fractions (a, b). Coordinates beyond 2^22 do not
-// round to integers, but their texels are all outside.
+// round to integers, but their texels are all outside a texture with sides below 2^22.
 __device__ __forceinline__ void ghost_footprint(f2 uv, f2& centre, f2& frac) {
     const f2 big = pk(12582912.0f, 12582912.0f), big1 = pk(12582911.0f, 12582911.0f), half3 = pk(1.5f, 1.5f);
     centre = sub2(add2(uv, big), big1);
@@ -395,11 +396,11 @@ __device__ __forceinline__ float ghost_blend(float t00, float t10, float t01, fl
     const float top = fmaf(a, t10 - t00, t00), bottom = fmaf(a, t11 - t01, t01);
     return fmaf(b, bottom - top, top);
 }
-// The footprint's texels by loads.
-__device__ __forceinline__ void ghost_texels(const float* __restrict__ tex, int w, int h, f2 centre, float& t00,
-                                             float& t10, float& t01, float& t11) {
-    const int i1 = cvt_rz_sat(lo2(centre)), j1 = cvt_rz_sat(hi2(centre)), i0 = wsub(i1, 1), j0 = wsub(j1, 1);
-    if ((unsigned)i0 < (unsigned)(w - 1) && (unsigned)j0 < (unsigned)(h - 1)) {
+// The footprint's texels, the first one (i0, j0), by loads; large: past 32-bit offsets.
+__device__ __forceinline__ void ghost_texels(const float* __restrict__ tex, int w, int h, bool large, int i0, int j0,
+                                             float& t00, float& t10, float& t01, float& t11) {
+    const int i1 = wadd(i0, 1), j1 = wadd(j0, 1);
+    if (!large && (unsigned)i0 < (unsigned)(w - 1) && (unsigned)j0 < (unsigned)(h - 1)) {
         // all four texels inside (the common case)
         const float* q = tex + (j0 * w + i0);
         t00 = __ldg(q);
@@ -435,7 +436,13 @@ __device__ __forceinline__ float ghost_sample(const float* __restrict__ tex, con
         const float4 g = tex2Dgather<float4>((cudaTextureObject_t)p.ghost_tex, lo2(centre), hi2(centre), 0);
         t00 = g.w, t10 = g.z, t01 = g.x, t11 = g.y;
     } else {
-        ghost_texels(tex, p.ghost_w, p.ghost_h, centre, t00, t10, t01, t11);
+        int i0 = wsub(cvt_rz_sat(lo2(centre)), 1), j0 = wsub(cvt_rz_sat(hi2(centre)), 1);
+        if (p.ghost_large) {  // sides past ghost_footprint's range (texture objects have no such sides)
+            const float u = lo2(uv) + 0.5f, v = hi2(uv) + 0.5f, fu = floorf(u), fv = floorf(v);
+            i0 = cvt_rz_sat(fu), j0 = cvt_rz_sat(fv);
+            frac = pk(u - fu, v - fv);
+        }
+        ghost_texels(tex, p.ghost_w, p.ghost_h, p.ghost_large, i0, j0, t00, t10, t01, t11);
     }
     return ghost_blend(t00, t10, t01, t11, frac);
 }
@@ -1175,13 +1182,12 @@ __device__ __forceinline__ float ghost_sample_grad(const float* __restrict__ tex
     if (!(fabsf(u) < 1e9f) || !(fabsf(v) < 1e9f)) return 0.0f;
     const float fu = floorf(u), fv = floorf(v);
     const float a = u - fu, b = v - fv;
-    const f2 centre = pk(fu + 1.0f, fv + 1.0f);
     float t00, t10, t01, t11;
     if (kTex) {
-        const float4 g = tex2Dgather<float4>((cudaTextureObject_t)p.ghost_tex, lo2(centre), hi2(centre), 0);
+        const float4 g = tex2Dgather<float4>((cudaTextureObject_t)p.ghost_tex, fu + 1.0f, fv + 1.0f, 0);
         t00 = g.w, t10 = g.z, t01 = g.x, t11 = g.y;
     } else {
-        ghost_texels(tex, p.ghost_w, p.ghost_h, centre, t00, t10, t01, t11);
+        ghost_texels(tex, p.ghost_w, p.ghost_h, p.ghost_large, cvt_rz_sat(fu), cvt_rz_sat(fv), t00, t10, t01, t11);
     }
     du = (1.0f - b) * (t10 - t00) + b * (t11 - t01);
     dv = (1.0f - a) * (t01 - t00) + a * (t11 - t10);
@@ -1582,6 +1588,8 @@ __host__ __device__ inline bool make_params(const rf_raster_args& a, RasterParam
     p.ghost_w = a.ghost_width;
     p.ghost_h = a.ghost_height;
     p.safe_screen = (float)a.width * a.sub_steps <= 16384.0f && (float)a.height * a.sub_steps <= 16384.0f;
+    p.ghost_large = a.ghost_width >= 1 << 22 || a.ghost_height >= 1 << 22 ||
+                    (long long)a.ghost_width * a.ghost_height > 0x7fffffffLL;
     p.ghost_tex = 0;  // the texels are loaded unless a launcher sets a texture object
     return true;
 }
