@@ -119,6 +119,13 @@ int rf_trace_differentiable(const rf_lens_element* elements, const int32_t* path
 int rf_trace_accurate(const rf_lens_element* elements, const int32_t* paths, const float* wavelengths,
                       const rf_trace_args* args, float* rays, void* stream);
 
+/* rf_trace_accurate with the reflectances of rf_trace_differentiable, from the double incidence angle
+ * rounded to float: the accurate forward trace of a differentiated render. The other outputs are
+ * rf_trace_accurate's bit for bit. */
+int rf_trace_accurate_differentiable(const rf_lens_element* elements, const int32_t* paths,
+                                     const float* wavelengths, const rf_trace_args* args, float* rays,
+                                     void* stream);
+
 /* One surface hit of a traced ray (the reference's Intersection, realflare/api/tasks/
  * opencl.py:18-25, without the float3 padding): position and unit normal at the surface,
  * the incidence angle acos(-dir . normal) (0 on flat elements), hit 1 (0 in an unused

@@ -151,9 +151,10 @@ class DifferentiableRenderer:
     function of ``LensParameters``. ``render(params)`` returns the (h, w, 4) image tensor.
 
     ``accurate=True`` runs the forward trace with the double-precision ray geometry
-    (``rf_trace_accurate``): the image, its coverage and the vertex attributes the gradient
-    is taken at are then those of the double evaluation of the trace, not the reference's
-    FP32 values (the adjoint's re-trace stays FP32: it only evaluates the Jacobians)."""
+    (``rf_trace_accurate_differentiable``): the image, its coverage and the vertex attributes
+    the gradient is taken at are then those of the double evaluation of the trace, not the
+    reference's FP32 values (the adjoint's re-trace stays FP32: it only evaluates the
+    Jacobians, of the same form of the reflectances)."""
 
     def __init__(self, project: Project, ghost: torch.Tensor, paths=None, stream=None,
                  accurate: bool = False) -> None:
@@ -205,7 +206,7 @@ class DifferentiableRenderer:
         s = int(self.stream.cuda_stream)
         self.el = self._element_buffer(radius, center, thickness)
         self.targs = self._trace_args(direction)
-        trace = self.lib.rf_trace_accurate if self.accurate else self.lib.rf_trace_differentiable
+        trace = self.lib.rf_trace_accurate_differentiable if self.accurate else self.lib.rf_trace_differentiable
         check(trace(self.el.data_ptr(), self.paths.data_ptr(), self.wavelengths.data_ptr(),
                     ctypes.byref(self.targs), self.rays.data_ptr(), s), 'rf_trace')
         from .device import Rays
@@ -252,7 +253,7 @@ class DifferentiableRenderer:
         el = self._element_buffer(radius, center, thickness)
         targs = self._trace_args(direction)
         rays = empty((6, max(self.n_rays, 1)))
-        trace = self.lib.rf_trace_accurate if self.accurate else self.lib.rf_trace_differentiable
+        trace = self.lib.rf_trace_accurate_differentiable if self.accurate else self.lib.rf_trace_differentiable
         check(trace(el.data_ptr(), self.paths.data_ptr(), self.wavelengths.data_ptr(), ctypes.byref(targs),
                     rays.data_ptr(), s), 'rf_trace')
         return rays, el, targs

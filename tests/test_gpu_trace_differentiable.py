@@ -1,0 +1,67 @@
+"""The forward traces of a differentiated render, in FP32 and with the geometry in double: the reflectances of both have
+the form that the adjoint differentiates. Where the geometry is exact in FP32 (flat elements, light along the axis, no
+dispersion) the two therefore agree bit for bit."""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip('torch')
+
+from helpers import reduced  # noqa: E402
+from test_gpu_trace_paths import same_bits  # noqa: E402
+
+from realflare_gb300 import prepare  # noqa: E402
+from realflare_gb300._abi import check, lib  # noqa: E402
+from realflare_gb300.device import empty, ptr, stream_handle, to_device  # noqa: E402
+
+
+def trace(name, elements, ti):
+    el, pa, wl = to_device(elements.view(np.uint8)), to_device(ti.paths), to_device(ti.wavelengths)
+    rays = empty((6, ti.ray_count))
+    check(getattr(lib(), name)(ptr(el), ptr(pa), ptr(wl), ctypes.byref(ti.args), ptr(rays), stream_handle()), name)
+    torch.cuda.synchronize()
+    return rays
+
+
+def coated(ti, two_layers):
+    """The elements with every kind of coating among them."""
+    el = ti.elements.copy()
+    for i in range(len(el)):
+        kind = i % (4 if two_layers else 3)
+        el[i]['coating'] = 550 if kind == 1 else 0
+        el[i]['coating_layers'] = (0, 0, 1, 2)[kind]
+        el[i]['coating_thickness'] = (100.0, 80.0)
+    ti.args.coating_layer_ior[0], ti.args.coating_layer_ior[1] = 1.38, 2.1
+    return el
+
+
+@pytest.mark.parametrize('two_layers', [False, True])
+def test_accurate_has_the_adjoints_reflectances(two_layers):
+    ti = prepare.trace_inputs(reduced('spectral-16', grid=5, wavelengths=4).project)
+    el = coated(ti, two_layers)
+    el['center'] -= el['radius']
+    el['radius'] = 0.0
+    el[0]['coefficients'][0] = np.nan
+    ti.args.direction[0], ti.args.direction[1], ti.args.direction[2] = 0.0, 0.0, 1.0
+    a, b = trace('rf_trace_differentiable', el, ti), trace('rf_trace_accurate_differentiable', el, ti)
+    assert not torch.isnan(a[5]).any() and (a[5] > 0).any()
+    assert torch.equal(a[5], b[5])
+
+
+def test_renderer_traces_with_it():
+    from realflare_gb300.diff import DifferentiableRenderer
+
+    w = reduced('differentiable-16', grid=12, resolution=64, paths=20, wavelengths=2)
+    p = w.project
+    p.flare.lens.coating_thickness = (100.0,) * (len(p.flare.lens.lens_model.lens_elements) + 1)
+    r = DifferentiableRenderer(p, torch.ones((64, 64), device='cuda'), w.paths, accurate=True)
+    rays, el, targs = r.trace_kernels(*r.params.elements(*r.params.tensors(), r.E))
+    want = torch.empty_like(rays)
+    check(lib().rf_trace_accurate_differentiable(el.data_ptr(), r.paths.data_ptr(), r.wavelengths.data_ptr(),
+                                                 ctypes.byref(targs), want.data_ptr(), stream_handle()), 'trace')
+    assert same_bits(rays, want)
