@@ -118,7 +118,30 @@ __device__ __forceinline__ void interface_r(float ni, float ci, float nj, float 
     rp = (nj * ci - ni * cj) * rcp_rn(nj * ci + ni * cj);
 }
 
+// theta = incident + 1e-9 (a double sum there); only angles below 0.02 rad are close enough to 1e-9 for
+// the double sum to differ from `incident`
+__device__ __forceinline__ float angle_of(float incident) {
+    return incident < 0.02f ? (float)((double)incident + 1e-9) : incident;
+}
+// The reference's form of the uncoated reflectance (see fresnel_ar_angle).
+__device__ RF_CORE_COLD float fresnel_angle(float theta0, float n1, float n2) {
+    float theta1 = asinf(sinf(theta0) * n1 / n2);
+    float cosi = cosf(theta0);
+    float cost = cosf(theta1);
+    float rs = ((n1 * cosi) - (n2 * cost)) / ((n1 * cosi) + (n2 * cost));
+    float rp = ((n1 * cost) - (n2 * cosi)) / ((n1 * cost) + (n2 * cosi));
+    return (rs * rs + rp * rp) / 2.0f;
+}
+
+// Between equal indices (in every lens: back from the stop at the element before it) the reflectance is
+// 0, which the trace does not multiply by (the reference's rule), or a rounding residue, which it
+// does: a whole ghost lit or dark by last bits. There the reference's form decides.
 __device__ RF_CORE_COLD float fresnel(float c0, float s0, float n1, float n2) {
+    if (n1 == n2) {
+        const float theta = angle_of(acosf(c0));
+        __builtin_assume(fabsf(theta) < 8.0f);  // (sinf and cosf without their slow path)
+        return fresnel_angle(theta, n1, n2);
+    }
     float rs, rp;
     interface_r(n1, c0, n2, refracted_cos(s0 * (n1 / n2)), rs, rp);
     return (rs * rs + rp * rp) / 2.0f;
@@ -174,15 +197,6 @@ __device__ RF_CORE_COLD float fresnel_two_layer(float c0, float s0, float lambda
 // writes them and as the adjoint's duals differentiate them. The adjoint's re-trace and the
 // forward trace of a differentiated render use these: where a gradient is a small difference of
 // large terms (the light's), the reflectances' last bits show in it.
-__device__ RF_CORE_COLD float fresnel_angle(float theta0, float n1, float n2) {
-    float theta1 = asinf(sinf(theta0) * n1 / n2);
-    float cosi = cosf(theta0);
-    float cost = cosf(theta1);
-    float rs = ((n1 * cosi) - (n2 * cost)) / ((n1 * cosi) + (n2 * cost));
-    float rp = ((n1 * cost) - (n2 * cosi)) / ((n1 * cost) + (n2 * cosi));
-    return (rs * rs + rp * rp) / 2.0f;
-}
-
 __device__ RF_CORE_COLD float fresnel_ar_angle(float theta0, float lambda, float d1, float n0, float n1, float n2) {
     float s0 = sinf(theta0);
     float theta1 = asinf(s0 * n0 / n1);
@@ -280,27 +294,33 @@ struct TraceFrame {
     float dir[3];  // normalize(-direction.xyz), host-computed in FP32
 };
 
+// The reflectance of element e from the angle theta0 at which a ray hits it from a medium of index n1, the
+// element's own index being n2.
+__device__ __forceinline__ float reflectance_angle(float theta0, const SmemElement& e, float n1, float n2,
+                                                   float wavelength, const TraceFrame& f) {
+    const float nc = fmaxf(sqrtf(n1 * n2), f.cmin);
+    const float d1 = e.layers == 1 ? e.d0 : (float)e.coating / (4.0f * nc);
+    if (e.layers == 2) return fresnel_two_layer_angle(theta0, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
+    if (e.layers == 1 || e.coating > 0) return fresnel_ar_angle(theta0, wavelength, d1, n1, nc, n2);
+    return fresnel_angle(theta0, n1, n2);
+}
+// The same from the cosine and sine of the angle.
+__device__ __forceinline__ float reflectance_cos(float c0, float s0, const SmemElement& e, float n1, float n2,
+                                                 float wavelength, const TraceFrame& f) {
+    const float nc = fmaxf(sqrtf(n1 * n2), f.cmin);
+    const float d1 = e.layers == 1 ? e.d0 : (float)e.coating / (4.0f * nc);
+    if (e.layers == 2) return fresnel_two_layer(c0, s0, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
+    if (e.layers == 1 || e.coating > 0) return fresnel_ar(c0, s0, wavelength, d1, n1, nc, n2);
+    return fresnel(c0, s0, n1, n2);
+}
 // The reflectance of element e for a ray (dx, dy, dz) that hits it from a medium of index n1, the
 // element's own index being n2. kAngles: from the incidence angle.
 template <bool kAngles>
 __device__ __forceinline__ float surface_reflectance(float dx, float dy, float dz, const Hit& h, const SmemElement& e,
                                                      float n1, float n2, float wavelength, const TraceFrame& f) {
-    const float nc = fmaxf(sqrtf(n1 * n2), f.cmin);
-    const float d1 = e.layers == 1 ? e.d0 : (float)e.coating / (4.0f * nc);
-    if (kAngles) {
-        const float incident = incident_angle(dx, dy, dz, h);
-        // theta = incident + 1e-9 (a double sum there); only angles below 0.02 rad
-        // are close enough to 1e-9 for the double sum to differ from `incident`
-        const float theta = incident < 0.02f ? (float)((double)incident + 1e-9) : incident;
-        if (e.layers == 2)
-            return fresnel_two_layer_angle(theta, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
-        if (e.layers == 1 || e.coating > 0) return fresnel_ar_angle(theta, wavelength, d1, n1, nc, n2);
-        return fresnel_angle(theta, n1, n2);
-    }
-    const float c0 = incident_cos(dx, dy, dz, h), s0 = sqrt_rn((1.0f - c0) * (1.0f + c0));
-    if (e.layers == 2) return fresnel_two_layer(c0, s0, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
-    if (e.layers == 1 || e.coating > 0) return fresnel_ar(c0, s0, wavelength, d1, n1, nc, n2);
-    return fresnel(c0, s0, n1, n2);
+    if (kAngles) return reflectance_angle(angle_of(incident_angle(dx, dy, dz, h)), e, n1, n2, wavelength, f);
+    const float c0 = incident_cos(dx, dy, dz, h);
+    return reflectance_cos(c0, sqrt_rn((1.0f - c0) * (1.0f + c0)), e, n1, n2, wavelength, f);
 }
 
 // Observer of a traced ray: step() sees the ray entering each element (element index,

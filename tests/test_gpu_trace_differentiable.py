@@ -1,6 +1,6 @@
-"""The forward traces of a differentiated render, in FP32 and with the geometry in double: the reflectances of both have
-the form that the adjoint differentiates. Where the geometry is exact in FP32 (flat elements, light along the axis, no
-dispersion) the two therefore agree bit for bit."""
+"""The forward traces of a differentiated render: everything but the reflectance is that of rf_trace and
+rf_trace_accurate bit for bit, and the reflectances have the form that the adjoint differentiates, in both. Where the
+geometry is exact in FP32 (flat elements, light along the axis, no dispersion) the two therefore agree bit for bit."""
 from __future__ import annotations
 
 import ctypes
@@ -38,6 +38,20 @@ def coated(ti, two_layers):
         el[i]['coating_thickness'] = (100.0, 80.0)
     ti.args.coating_layer_ior[0], ti.args.coating_layer_ior[1] = 1.38, 2.1
     return el
+
+
+@pytest.mark.parametrize('two_layers', [False, True])
+@pytest.mark.parametrize('workload,grid', [('plain-8', 33), ('spectral-16', 24)])
+@pytest.mark.parametrize('plain,differentiable', [('rf_trace', 'rf_trace_differentiable'),
+                                                  ('rf_trace_accurate', 'rf_trace_accurate_differentiable')])
+def test_other_outputs(plain, differentiable, workload, grid, two_layers):
+    ti = prepare.trace_inputs(reduced(workload, grid=grid, wavelengths=3).project)
+    el = coated(ti, two_layers)
+    a, b = trace(plain, el, ti), trace(differentiable, el, ti)
+    assert same_bits(a[:5], b[:5])
+    assert torch.equal(torch.isnan(a[5]), torch.isnan(b[5]))
+    ok = ~torch.isnan(a[5])
+    assert ok.any() and (a[5] - b[5])[ok].norm() <= 1e-4 * a[5][ok].norm()
 
 
 @pytest.mark.parametrize('two_layers', [False, True])
