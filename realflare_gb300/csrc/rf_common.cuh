@@ -179,14 +179,17 @@ __device__ __forceinline__ float sample_linear(const float* __restrict__ tex, in
 
 // xyz_to_ap1 (realflare/api/tasks/cl/color.cl:3-10): the matrix literals are double in OpenCL C, so
 // the products and sums are evaluated in double there. Double precision runs at 1/64 of FP32's
-// rate here (15 double operations per pixel were 14 % of a starburst's time), so each output is an
-// unevaluated sum of two floats instead, by error-free products (fused multiply-add) and sums (D.
-// Knuth's two-sum): about 46 bits, rounded to float at the end.
-__device__ __forceinline__ float dot_two_float(float x, float y, float z, double cx, double cy, double cz) {
+// rate here (15 double operations per pixel were 14 % of a starburst's time), so each output is first
+// an unevaluated sum of two floats, by error-free products (fused multiply-add) and sums (D. Knuth's
+// two-sum), within 2^-44 of the terms' magnitudes. Where every value within 2^-42 of it rounds to the
+// same float, that is what the double form rounds to as well; the others (one in some
+// 100,000; sums that cancel; magnitudes whose errors could underflow; infinities and NaN) take the
+// double form.
+__device__ __forceinline__ bool dot_rounded(float x, float y, float z, double cx, double cy, double cz, float& out) {
     const float c[3] = {(float)cx, (float)cy, (float)cz};
     const float l[3] = {(float)(cx - c[0]), (float)(cy - c[1]), (float)(cz - c[2])};
     const float v[3] = {x, y, z};
-    float hi = 0.0f, lo = 0.0f;
+    float hi = 0.0f, lo = 0.0f, magnitude = 0.0f;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const float p = __fmul_rn(v[k], c[k]);
@@ -194,16 +197,24 @@ __device__ __forceinline__ float dot_two_float(float x, float y, float z, double
         const float s = __fadd_rn(hi, p), b = __fsub_rn(s, hi);
         lo = __fadd_rn(lo, __fadd_rn(e, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(p, b))));
         hi = s;
+        magnitude += fabsf(p);
     }
-    const float s = __fadd_rn(hi, lo);
-    return isfinite(s) ? s : __fadd_rn(__fadd_rn(__fmul_rn(x, c[0]), __fmul_rn(y, c[1])), __fmul_rn(z, c[2]));
+    const float d = magnitude * 0x1p-42f;
+    out = __fadd_rn(hi, __fsub_rn(lo, d));
+    return out == __fadd_rn(hi, __fadd_rn(lo, d)) && (magnitude >= 0x1p-80f || magnitude == 0.0f);
 }
 __device__ __forceinline__ float4 xyz_to_ap1(float x, float y, float z) {
     float4 o;
-    o.x = dot_two_float(x, y, z, 1.6410233797, -0.3248032942, -0.2364246952);
-    o.y = dot_two_float(x, y, z, -0.6636628587, 1.6153315917, 0.0167563477);
-    o.z = dot_two_float(x, y, z, 0.0117218943, -0.0082844420, 0.9883948585);
     o.w = 0.0f;
+    bool ok = dot_rounded(x, y, z, 1.6410233797, -0.3248032942, -0.2364246952, o.x);
+    ok = dot_rounded(x, y, z, -0.6636628587, 1.6153315917, 0.0167563477, o.y) && ok;
+    ok = dot_rounded(x, y, z, 0.0117218943, -0.0082844420, 0.9883948585, o.z) && ok;
+    if (!ok) {
+        const double dx = x, dy = y, dz = z;
+        o.x = (float)(1.6410233797 * dx + -0.3248032942 * dy + -0.2364246952 * dz);
+        o.y = (float)(-0.6636628587 * dx + 1.6153315917 * dy + 0.0167563477 * dz);
+        o.z = (float)(0.0117218943 * dx + -0.0082844420 * dy + 0.9883948585 * dz);
+    }
     return o;
 }
 
