@@ -343,8 +343,10 @@ typedef struct rf_frame {
     int64_t prim_offset;      /* the frame's bounds (float4) */
     int64_t inten_offset;     /* the frame's intensities (float) */
     int64_t vertex_offset;    /* the frame's vertices (n_rays + 1 of them) */
-    int64_t pair_offset;      /* the frame's (primitive, wavelength pair) counters */
-    int64_t trace_block, quad_block, vertex_block, pair_block;  /* first block of each stage */
+    int64_t pair_offset;      /* the frame's (primitive, wavelength pair) rectangles */
+    /* first block of each stage (trace_block: of 256 * rays_per_thread rays, which bounds the plan; the trace
+     * itself finds its work by trace_item) */
+    int64_t trace_block, quad_block, vertex_block, pair_block;
     int32_t tile_offset, tile_count;  /* the frame's raster tiles in the batch's tile numbering */
     float direction_n[3];     /* normalize(-direction.xyz) in FP32, as rf_trace computes it */
     int32_t trace_item;       /* the frame's first work item in the batch's trace */

@@ -111,6 +111,17 @@ __device__ __forceinline__ int find_frame(const rf_frame* __restrict__ frames, i
     return lo;
 }
 
+// Two FP32 values in one 64-bit register pair, for the packed FP32 instructions of sm_100 and later (two
+// operations per instruction, each rounded as the scalar one).
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pk(float lo, float hi) {
+    f2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float lo2(f2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi2(f2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+
 // Quotient and remainder of a >= 0 by b > 0, in 32 bits where a allows (a 64-bit division takes several
 // times as many instructions).
 __device__ __forceinline__ void divide(long long a, int b, long long& q, int& r) {

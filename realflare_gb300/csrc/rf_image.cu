@@ -12,16 +12,7 @@
 namespace rf {
 namespace {
 
-// Two FP32 values per register pair: each packed instruction does two terms in one issue slot,
-// each rounded as the scalar operation.
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 pk(float lo, float hi) {
-    f2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ float lo2(f2 v) { return __uint_as_float((unsigned)v); }
-__device__ __forceinline__ float hi2(f2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+// Packed FP32 (f2, rf_common.cuh): two terms in one issue slot.
 __device__ __forceinline__ f2 add2(f2 a, f2 b) {
     f2 d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));

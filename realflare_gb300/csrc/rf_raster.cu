@@ -46,9 +46,6 @@ namespace {
 #ifndef RF_RASTER_MIN_BLOCKS_S1  // the one-sample kernel needs fewer registers
 #define RF_RASTER_MIN_BLOCKS_S1 4
 #endif
-#ifndef RF_RASTER_CLASSIFY
-#define RF_RASTER_CLASSIFY 1
-#endif
 constexpr int kBatchRecords = RF_RASTER_BATCH;
 // Pixels of a column a lane of the one-sample kernels shades: two where a tile has enough blocks
 // of 8 x 8 pixels for the CTA's 8 warps (32-pixel tiles: 16; production frame 102.0 ms with one
@@ -73,17 +70,8 @@ __device__ unsigned long long g_raster_stats[kRasterStats];
 #define RF_STAT(stmt)
 #endif
 
-// Two FP32 values in one 64-bit register pair, for the packed FP32 instructions of sm_100 and
-// later (two lanes per instruction, each rounded as the scalar operation): shading is bound by
+// Packed FP32 (f2, rf_common.cuh) with denormals flushed as in the rest of this unit: shading is bound by
 // instruction issue, and a packed instruction does two corners' work in one issue slot.
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 pk(float lo, float hi) {
-    f2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ float lo2(f2 v) { return __uint_as_float((unsigned)v); }
-__device__ __forceinline__ float hi2(f2 v) { return __uint_as_float((unsigned)(v >> 32)); }
 __device__ __forceinline__ f2 add2(f2 a, f2 b) {
     f2 d;
     asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
