@@ -155,6 +155,7 @@ class RasterizingTask(Task):
         self._spectrum = None
         self._entry_capacity = 0
         self._buffers: dict = {}
+        self._offsets = None, None  # the tile offsets' buffer and its part for the last image
         self.last_entry_count = 0
         self.tile_size = 0
 
@@ -195,7 +196,11 @@ class RasterizingTask(Task):
               'rf_raster_tiles')
         self.tile_size = tile_size.value
         # exactly the image's tiles: the buffer itself only grows, and may be an earlier image's, with more of them
-        offsets = self._buffer('tile_offsets', tile_count.value + 1, torch.int32)[:tile_count.value + 1]
+        # (the view is kept while it fits: making one takes 3 us)
+        whole = self._buffer('tile_offsets', tile_count.value + 1, torch.int32)
+        if self._offsets[0] is not whole or self._offsets[1].numel() != tile_count.value + 1:
+            self._offsets = whole, whole[:tile_count.value + 1]
+        offsets = self._offsets[1]
         count = ctypes.c_int64()
         for _ in range(3):
             cap = self._entry_capacity
