@@ -413,6 +413,9 @@ __device__ __forceinline__ void ghost_texels(const float* __restrict__ tex, int 
         t11 = (i1_in && j1_in) ? __ldg(row1 + ib) : 0.0f;
     }
 }
+// How a kernel looks the ghost texture up: by loads; by gathers from a texture object; by loads from a texture of any
+// size (RasterParams.ghost_large; the test per fragment costs 1.5 % of the kernel).
+constexpr int kLoads = 0, kGather = 1, kAnyLoads = 2;
 // The same texels through a texture object over them (float, pitch-linear, border address
 // mode): tex2Dgather at the footprint's centre, exactly half a texel from every footprint
 // boundary, returns texels (i0, j0 + 1), (i0 + 1, j0 + 1), (i0 + 1, j0), (i0, j0) in x, y, z, w, and
@@ -420,22 +423,23 @@ __device__ __forceinline__ void ghost_texels(const float* __restrict__ tex, int 
 // address arithmetic and four loads. The values, and so the interpolation, are the loads'. u and v
 // are finite: the weights are, and records with a texel coordinate that is not are left out
 // (zero_record).
-template <bool kTex>
+template <int kTex>
 __device__ __forceinline__ float ghost_sample(const float* __restrict__ tex, const RasterParams& p, f2 uv) {
     f2 centre, frac;
     ghost_footprint(uv, centre, frac);
     float t00, t10, t01, t11;
-    if (kTex) {
+    if (kTex == kGather) {
         const float4 g = tex2Dgather<float4>((cudaTextureObject_t)p.ghost_tex, lo2(centre), hi2(centre), 0);
         t00 = g.w, t10 = g.z, t01 = g.x, t11 = g.y;
     } else {
         int i0 = wsub(cvt_rz_sat(lo2(centre)), 1), j0 = wsub(cvt_rz_sat(hi2(centre)), 1);
-        if (p.ghost_large) {  // sides past ghost_footprint's range (texture objects have no such sides)
+        const bool large = kTex == kAnyLoads && p.ghost_large;
+        if (large) {  // sides past ghost_footprint's range (texture objects have no such sides)
             const float u = lo2(uv) + 0.5f, v = hi2(uv) + 0.5f, fu = floorf(u), fv = floorf(v);
             i0 = cvt_rz_sat(fu), j0 = cvt_rz_sat(fv);
             frac = pk(u - fu, v - fv);
         }
-        ghost_texels(tex, p.ghost_w, p.ghost_h, p.ghost_large, i0, j0, t00, t10, t01, t11);
+        ghost_texels(tex, p.ghost_w, p.ghost_h, large, i0, j0, t00, t10, t01, t11);
     }
     return ghost_blend(t00, t10, t01, t11, frac);
 }
@@ -446,7 +450,7 @@ __device__ __forceinline__ float ghost_sample(const float* __restrict__ tex, con
 struct FragmentConsts {
     float tsx, tox, tsy, toy;  // texel coordinate scale and offset per axis
 };
-template <bool kTex, int kN>
+template <int kTex, int kN>
 __device__ __forceinline__ void fragment_fast(const Rec& r, const f2 (&we)[kN], const f2 (&wo)[kN],
                                               const float* __restrict__ ghost, const RasterParams& p, float general,
                                               float (&f)[kN]) {
@@ -472,7 +476,7 @@ __device__ __forceinline__ void fragment_fast(const Rec& r, const f2 (&we)[kN], 
 #pragma unroll
     for (int i = 0; i < kN; i++) f[i] = gi[i] * ai[i] * ci[i];
 }
-template <bool kTex = false>
+template <int kTex = kAnyLoads>
 __device__ __forceinline__ float fragment_fast(const Rec& r, f2 we, f2 wo, const float* __restrict__ ghost,
                                                const RasterParams& p, float general) {
     const f2 e1[1] = {we}, o1[1] = {wo};
@@ -701,9 +705,9 @@ constexpr size_t raster_smem_bytes(int maxW, int WS) {
 
 // Tile (tx, ty), whose entries are tile_entries[begin, end). smem4 holds the dynamic shared
 // memory (raster_smem_bytes), next_block four shared counters. kS: the anti-aliasing sample
-// count when known at compile time, else 0 (p.S). kTex: sample the ghost texture through
-// p.ghost_tex.
-template <int T, int kS, bool kTex, int kPix>
+// count when known at compile time, else 0 (p.S). kTex: how the ghost texture is looked
+// up (kLoads, kGather through p.ghost_tex, kAnyLoads).
+template <int T, int kS, int kTex, int kPix>
 __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint32_t begin, uint32_t end,
                                             const uint32_t* __restrict__ tile_entries,
                                             const float* __restrict__ ghost, const float* __restrict__ spectrum,
@@ -1039,7 +1043,7 @@ constexpr int kPixels = kS != 1 ? 1 : (T == 32 ? RF_RASTER_PIX32 : RF_RASTER_PIX
 // One CTA per tile of a frame: CTA k shades tile order[k], or tile k without an order.
 // CTAs start in index order as slots free up, so an order by decreasing work starts the
 // heaviest tiles first and ends the launch with light ones.
-template <int T, int kS, bool kTex>
+template <int T, int kS, int kTex>
 __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : RF_RASTER_MIN_BLOCKS)
     k_raster(const float4* __restrict__ vtx, const uint32_t* __restrict__ tile_offsets,
              const uint32_t* __restrict__ tile_entries, const uint32_t* __restrict__ order,
@@ -1055,9 +1059,9 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : 
 __host__ __device__ inline bool make_params(const rf_raster_args& a, RasterParams& p);
 
 // Every frame of a batch in one persistent launch: each CTA takes the next tile from the
-// queue (tiles ordered by decreasing entry count) until none are left. kTex: every frame's
+// queue (tiles ordered by decreasing entry count) until none are left. kTex kGather: every frame's
 // ghost lookups go through its rf_frame.ghost_texture.
-template <int T, int kS, bool kTex>
+template <int T, int kS, int kTex>
 __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : RF_RASTER_MIN_BLOCKS)
     k_raster_batch(const rf_frame* __restrict__ frames, int F, int tiles, const uint32_t* __restrict__ order,
                    unsigned* __restrict__ queue, const unsigned long long* __restrict__ entry_total,
@@ -1081,7 +1085,7 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : 
                 const rf_frame& fr = frames[f];
                 RasterParams q;
                 make_params(fr.raster, q);
-                if (kTex) q.ghost_tex = fr.ghost_texture;
+                if (kTex == kGather) q.ghost_tex = fr.ghost_texture;
                 q.T = T;
                 q.ntx = (q.width + T - 1) / T;
                 sp = q;
@@ -1660,28 +1664,28 @@ unsigned long long ghost_texture_object(const float* ghost, int w, int h) {
     return obj;
 }
 
+template <int T, int kS, int kTex>
+int launch_raster_k(const float* vertexes, const uint32_t* offsets, const uint32_t* entries, const uint32_t* order,
+                    const float* ghost, const float* spectrum, const RasterParams& p, float* image, cudaStream_t s) {
+    static std::atomic<size_t> allowed[kMaxDevices];
+    const size_t smem = raster_smem_bytes<T>(p.maxW, p.WS);
+    RF_TRY(allow_smem(k_raster<T, kS, kTex>, smem, allowed));
+    k_raster<T, kS, kTex><<<p.ntx * ((p.height + T - 1) / T), kThreads, smem, s>>>(
+        (const float4*)vertexes, offsets, entries, order, ghost, spectrum, p, fragment_consts(p), (float4*)image);
+    return launch_status();
+}
+
 template <int T, int kS>
 int launch_raster_s(const float* vertexes, const uint32_t* offsets, const uint32_t* entries, const uint32_t* order,
                     const float* ghost, const float* spectrum, RasterParams p, float* image, cudaStream_t s) {
-    static std::atomic<size_t> allowed[kMaxDevices];
-    static std::atomic<size_t> allowed_tex[kMaxDevices];
     p.T = T;
     p.ntx = (p.width + T - 1) / T;
-    const int nty = (p.height + T - 1) / T;
-    const size_t smem = raster_smem_bytes<T>(p.maxW, p.WS);
     p.ghost_tex = ghost_texture_object(ghost, p.ghost_w, p.ghost_h);
-    if (p.ghost_tex) {
-        RF_TRY(allow_smem(k_raster<T, kS, true>, smem, allowed_tex));
-        k_raster<T, kS, true><<<p.ntx * nty, kThreads, smem, s>>>((const float4*)vertexes, offsets, entries, order,
-                                                                 ghost, spectrum, p, fragment_consts(p),
-                                                                 (float4*)image);
-    } else {
-        RF_TRY(allow_smem(k_raster<T, kS, false>, smem, allowed));
-        k_raster<T, kS, false><<<p.ntx * nty, kThreads, smem, s>>>((const float4*)vertexes, offsets, entries, order,
-                                                                  ghost, spectrum, p, fragment_consts(p),
-                                                                  (float4*)image);
-    }
-    return launch_status();
+    if (p.ghost_tex)
+        return launch_raster_k<T, kS, kGather>(vertexes, offsets, entries, order, ghost, spectrum, p, image, s);
+    if (p.ghost_large)  // one kernel for all sample counts
+        return launch_raster_k<T, 0, kAnyLoads>(vertexes, offsets, entries, order, ghost, spectrum, p, image, s);
+    return launch_raster_k<T, kS, kLoads>(vertexes, offsets, entries, order, ghost, spectrum, p, image, s);
 }
 
 template <int T>
@@ -1694,7 +1698,7 @@ int launch_raster(const float* vertexes, const uint32_t* offsets, const uint32_t
     return launch_raster_s<T, 8>(vertexes, offsets, entries, order, ghost, spectrum, p, image, s);
 }
 
-template <int T, int kS, bool kTex>
+template <int T, int kS, int kTex>
 int launch_raster_batch(const rf_frame* frames, const rf_batch_sizes& z, const float* vertexes,
                         const uint32_t* tile_offsets, const uint32_t* tile_entries, const float* ghosts,
                         const float* spectrum, const BatchWorkspace& w, long long capacity,
@@ -1748,11 +1752,11 @@ extern "C" int rf_raster_batch(const rf_frame* frames, const rf_batch_sizes* siz
     const bool tex = z.ghost_textures != 0;
     switch (z.tile_size) {
         case 32:
-            return one ? (tex ? RF_BATCH_LAUNCH(32, 1, true) : RF_BATCH_LAUNCH(32, 1, false))
-                       : (tex ? RF_BATCH_LAUNCH(32, 0, true) : RF_BATCH_LAUNCH(32, 0, false));
+            return one ? (tex ? RF_BATCH_LAUNCH(32, 1, kGather) : RF_BATCH_LAUNCH(32, 1, kAnyLoads))
+                       : (tex ? RF_BATCH_LAUNCH(32, 0, kGather) : RF_BATCH_LAUNCH(32, 0, kAnyLoads));
         case 16:
-            return one ? (tex ? RF_BATCH_LAUNCH(16, 1, true) : RF_BATCH_LAUNCH(16, 1, false))
-                       : (tex ? RF_BATCH_LAUNCH(16, 0, true) : RF_BATCH_LAUNCH(16, 0, false));
+            return one ? (tex ? RF_BATCH_LAUNCH(16, 1, kGather) : RF_BATCH_LAUNCH(16, 1, kAnyLoads))
+                       : (tex ? RF_BATCH_LAUNCH(16, 0, kGather) : RF_BATCH_LAUNCH(16, 0, kAnyLoads));
 #undef RF_BATCH_LAUNCH
         default:
             return RF_ERR_NOT_SUPPORTED;
