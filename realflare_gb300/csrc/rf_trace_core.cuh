@@ -304,11 +304,34 @@ __device__ __forceinline__ float reflectance_angle(float theta0, const SmemEleme
     if (e.layers == 1 || e.coating > 0) return fresnel_ar_angle(theta0, wavelength, d1, n1, nc, n2);
     return fresnel_angle(theta0, n1, n2);
 }
+// Two layers without thickness between equal indices, which is no coating either (see fresnel): the reference's form
+// of the stack (fresnel_two_layer_angle) with the phases' sines 0 and cosines 1.
+__device__ __forceinline__ float bare_layers_r2(float r01, float r12, float r23) {
+    const float nre = r12 + r23, dre = 1.0f + r12 * r23;
+    const float ere = (nre * dre) / (dre * dre);
+    const float tre = r01 + ere, bre = 1.0f + r01 * ere;
+    return (tre * tre) / (bre * bre);
+}
+__device__ RF_CORE_COLD float bare_layers(float c, float n, float na, float nb) {
+    const float theta = angle_of(acosf(c));
+    __builtin_assume(fabsf(theta) < 8.0f);
+    float s0, c0;
+    sincosf(theta, &s0, &c0);
+    const float sa = n * s0 / na, sb = n * s0 / nb, s2 = n * s0 / n;
+    const float ca = sqrtf(1.0f - sa * sa), cb = sqrtf(1.0f - sb * sb), c2 = sqrtf(1.0f - s2 * s2);
+    float rs01, rp01, rs12, rp12, rs23, rp23;
+    interface_r_div(n, c0, na, ca, rs01, rp01);
+    interface_r_div(na, ca, nb, cb, rs12, rp12);
+    interface_r_div(nb, cb, n, c2, rs23, rp23);
+    return (bare_layers_r2(rs01, rs12, rs23) + bare_layers_r2(rp01, rp12, rp23)) / 2.0f;
+}
+
 // The same from the cosine and sine of the angle.
 __device__ __forceinline__ float reflectance_cos(float c0, float s0, const SmemElement& e, float n1, float n2,
                                                  float wavelength, const TraceFrame& f) {
     const float nc = fmaxf(sqrtf(n1 * n2), f.cmin);
     const float d1 = e.layers == 1 ? e.d0 : (float)e.coating / (4.0f * nc);
+    if (e.layers == 2 && n1 == n2 && e.d0 == 0.0f && e.d1 == 0.0f) return bare_layers(c0, n1, f.layer_n0, f.layer_n1);
     if (e.layers == 2) return fresnel_two_layer(c0, s0, wavelength, n1, f.layer_n0, e.d0, f.layer_n1, e.d1, n2);
     if (e.layers == 1 || e.coating > 0) return fresnel_ar(c0, s0, wavelength, d1, n1, nc, n2);
     return fresnel(c0, s0, n1, n2);

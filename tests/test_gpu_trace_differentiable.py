@@ -54,6 +54,24 @@ def test_other_outputs(plain, differentiable, workload, grid, two_layers):
     assert ok.any() and (a[5] - b[5])[ok].norm() <= 1e-4 * a[5][ok].norm()
 
 
+@pytest.mark.parametrize('layers', [0, 2])
+@pytest.mark.parametrize('plain,differentiable', [('rf_trace', 'rf_trace_differentiable'),
+                                                  ('rf_trace_accurate', 'rf_trace_accurate_differentiable')])
+def test_no_coating(plain, differentiable, layers):
+    """Uncoated, and two layers without thickness: between equal indices (at the element before the stop) the reflectance
+    is 0, which the trace does not multiply by, or a rounding residue, which it does; alike in both forms."""
+    ti = prepare.trace_inputs(reduced('spectral-16', grid=24, wavelengths=3).project)
+    el = ti.elements.copy()
+    el['coating'] = 0
+    el['coating_layers'] = layers
+    el['coating_thickness'] = 0.0
+    ti.args.coating_layer_ior[0], ti.args.coating_layer_ior[1] = 1.38, 2.1
+    a, b = trace(plain, el, ti), trace(differentiable, el, ti)
+    ok = ~torch.isnan(a[5])
+    assert ((a[5] < 1e-9) & ok).any()
+    assert (a[5] - b[5])[ok].norm() <= 1e-4 * a[5][ok].norm()
+
+
 @pytest.mark.parametrize('two_layers', [False, True])
 def test_accurate_has_the_adjoints_reflectances(two_layers):
     ti = prepare.trace_inputs(reduced('spectral-16', grid=5, wavelengths=4).project)
