@@ -103,7 +103,7 @@ int rf_trace(const rf_lens_element* elements, const int32_t* paths, const float*
 /* rf_trace with the reflectances evaluated from the incidence angle, operation by operation as the
  * reference writes them (raytracing.cl:1-59) and as rf_trace_adjoint differentiates them:
  * the forward trace of a differentiated render. The other outputs are rf_trace's bit for bit,
- * the reflectance differs in its last bits. */
+ * the reflectance differs in its last bits (not at all between equal indices without a coating). */
 int rf_trace_differentiable(const rf_lens_element* elements, const int32_t* paths, const float* wavelengths,
                             const rf_trace_args* args, float* rays, void* stream);
 

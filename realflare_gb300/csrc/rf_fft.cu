@@ -21,8 +21,8 @@
 // power-of-two length M >= 2n - 1; the filter's transform is evaluated once per block.
 //
 // What bounds it: latency on the small textures (a few microseconds per launch), shared memory and
-// the transposing stores on batches. 512 x 512, 16 spectra 161 -> 74 us (both passes); a 256 x 256
-// ghost texture 74 -> 42 us in 13 -> 6 launches; 702 x 954 (chirp-z) 761 -> 384 us. (Radix-8
+// the transposing stores on batches. 512 x 512, 16 spectra 161 -> 76 us (both passes); a 256 x 256
+// ghost texture 74 -> 45 us in 13 -> 6 launches; 702 x 954 (chirp-z) 761 -> 386 us. (Radix-8
 // butterflies and merged passes took 34 and 322 us, with other last bits.)
 #include <complex>
 #include <math.h>

@@ -14,7 +14,7 @@
 //    ratios of every (wavelength, element) pair are staged in shared memory once per block; the
 //    tables replace the per-interaction Sellmeier evaluation and division with lookups of the
 //    same FP32 values (dispersion() depends only on the wavelength and the element);
-//  * what bounds it is instruction issue (84 % of active cycles). Square roots and reciprocals take
+//  * what bounds it is instruction issue (89 % of active cycles). Square roots and reciprocals take
 //    short correctly rounded forms (sqrt_rn, rcp_rn), rrel is evaluated only where it can be the
 //    largest, reflectances go without trigonometric functions: 72.4 M rays 18.36 -> 12.42 ms one
 //    path at a time;
