@@ -1247,6 +1247,17 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? 3 : 2)
     const int tile = blockIdx.x;
     const int tx = tile % p.ntx, ty = tile / p.ntx;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // this CTA's part of the tile's batches; without one nothing is set up (1004 x 1434 without entries: 66 ->
+    // 21 us)
+    const int per_batch = kBatchRecords / p.WS;
+    uint32_t begin = tile_offsets[tile], end = tile_offsets[tile + 1];
+    {
+        const unsigned batches = (end - begin + per_batch - 1) / per_batch;
+        const unsigned b0 = batches * blockIdx.y / gridDim.y, b1 = batches * (blockIdx.y + 1) / gridDim.y;
+        end = min(end, begin + b1 * per_batch);
+        begin += b0 * per_batch;
+        if (begin >= end) return;
+    }
     if (threadIdx.x == 0) {
         const float sub_step = 1.0f / (float)p.WS;
         float b = 0.0f;
@@ -1292,16 +1303,6 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? 3 : 2)
     for (int i = threadIdx.x; i < 2 * kBatchRecords * 4 * kGradAttrs; i += kThreads) rgrad_buf[i] = 0.0f;
 
     const int S = kS ? kS : p.S;
-    const int per_batch = kBatchRecords / p.WS;
-    // this CTA's part of the tile's batches
-    uint32_t begin = tile_offsets[tile], end = tile_offsets[tile + 1];
-    {
-        const unsigned batches = (end - begin + per_batch - 1) / per_batch;
-        const unsigned b0 = batches * blockIdx.y / gridDim.y, b1 = batches * (blockIdx.y + 1) / gridDim.y;
-        end = min(end, begin + b1 * per_batch);
-        begin += b0 * per_batch;
-        if (begin >= end) return;
-    }
     const int my_entry = threadIdx.x >> 2, my_corner = threadIdx.x & 3;
     const int Q = (p.G - 1) * (p.G - 1), VC = p.G * p.G;
     // Records of the batch at `first` into buffer `dst`, as k_raster builds them: thread j
