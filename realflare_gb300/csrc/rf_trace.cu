@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const rf_lens_element* 
                                                          const int2* __restrict__ paths,
                                                          const float* __restrict__ wavelengths,
                                                          const __grid_constant__ TraceParams p, bool table,
-                                                         int paths_each, int path_blocks, float* __restrict__ rays) {
+                                                         int path_blocks, float* __restrict__ rays) {
     __shared__ SmemElement se[kMaxElements];
     __shared__ PathList list;
     extern __shared__ float2 ratio_tab[];  // [rows][E], then the indices
@@ -45,8 +45,9 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const rf_lens_element* 
     // this block's paths, and its kTraceThreads consecutive ones of a path's (wavelength, grid point) pairs and
     // the wavelengths they span; counted from the first one's start the pairs fit 32 bits. The
     // paths with the longest shared legs come last in a list of pairs: their blocks go first
-    const int path_first = (path_blocks - 1 - (int)(blockIdx.x % path_blocks)) * paths_each;
-    const int path_count = min(paths_each, p.P - path_first);
+    const int path_block = path_blocks - 1 - (int)(blockIdx.x % path_blocks);
+    const int path_first = first_path(path_block, path_blocks, p.P);
+    const int path_count = first_path(path_block + 1, path_blocks, p.P) - path_first;
     const long long per_path = (long long)p.W * p.R;
     const long long first = (long long)(blockIdx.x / path_blocks) * kTraceThreads;
     const long long last = min(first + kTraceThreads, per_path) - 1;
@@ -121,8 +122,9 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace_batch(const rf_frame* _
         const float* wavelengths = wavelengths_all + fr.wavelength_offset;
         const int path_blocks = (fr.trace.path_count + paths_each - 1) / paths_each;
         const long long block = item - fr.trace_item;
-        const int path_first = (path_blocks - 1 - (int)(block % path_blocks)) * paths_each;
-        const int path_count = min(paths_each, fr.trace.path_count - path_first);
+        const int path_block = path_blocks - 1 - (int)(block % path_blocks);
+        const int path_first = first_path(path_block, path_blocks, fr.trace.path_count);
+        const int path_count = first_path(path_block + 1, path_blocks, fr.trace.path_count) - path_first;
         const long long per_path = (long long)W * R, chunk = kTraceThreads * (long long)rays_per_thread;
         const long long first = block / path_blocks * chunk;
         const long long last = min(first + chunk, per_path) - 1;
@@ -187,7 +189,7 @@ int trace_entry(const rf_lens_element* elements, const int32_t* paths, const flo
     if (blocks > 0x7fffffffLL) return RF_ERR_NOT_SUPPORTED;
     const size_t table = table_bytes(kTraceThreads, p.R, p.W, p.E);
     k_trace<kAngles><<<(unsigned)blocks, kTraceThreads, table, (cudaStream_t)stream>>>(
-        elements, (const int2*)paths, wavelengths, p, table > 0, paths_each, (int)path_blocks, rays);
+        elements, (const int2*)paths, wavelengths, p, table > 0, (int)path_blocks, rays);
     return launch_status();
 }
 }  // namespace
