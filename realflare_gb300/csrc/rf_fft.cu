@@ -22,7 +22,7 @@
 //
 // What bounds it: latency on the small textures (a few microseconds per launch), shared memory and
 // the transposing stores on batches. 512 x 512, 16 spectra 161 -> 76 us (both passes); a 256 x 256
-// ghost texture 74 -> 45 us in 13 -> 6 launches; 702 x 954 (chirp-z) 761 -> 386 us. (Radix-8
+// ghost texture 74 -> 45 us in 13 -> 6 launches; 702 x 954 (chirp-z) 759 -> 381 us. (Radix-8
 // butterflies and merged passes took 34 and 322 us, with other last bits.)
 #include <complex>
 #include <math.h>
@@ -74,6 +74,14 @@ RowPlan row_plan(int n, long long rows) {
            rows / (2 * p.rows_per_block) >= 128)
         p.rows_per_block *= 2;
     p.threads = p.rows_per_block * per_row;
+    // Threads for the filter alone (k_fft_pass) where all blocks fit the SMs at once with them (64 registers a
+    // thread: 1024 threads per SM): what counts there is the way through one block. 128 x 300 40 -> 21 us (24 with
+    // a launch per step), 128 x 777 43 -> 25, 300 x 500 41 -> 39. In more blocks they cost occupancy:
+    // 702 x 954 112 -> 126 us, 2000 x 1500 414 -> 590.
+    const int with_filter = p.threads + per_row;
+    if (!direct && per_row >= 32 && with_filter <= 1024 &&
+        (rows + p.rows_per_block - 1) / p.rows_per_block <= 152LL * (1024 / with_filter))
+        p.threads = with_filter;
     const size_t row = sizeof(float2) * padded(p.M);
     p.smem = row * p.rows_per_block + (direct ? 0 : row) + sizeof(float2) * p.M;
     return p;
@@ -209,15 +217,20 @@ __global__ void __launch_bounds__(1024) k_fft_pass(const Program p, int rows, in
     }
     float2 v[8];
     const float s = p.sign(row0);  // (programs keep directions equal within a block)
-    if (chirp_z) {
+    // chirp_z: the filter's threads are a group of their own behind the rows' where the block has them, and
+    // transform it beside the rows' first transform; elsewhere every group does so before.
+    const bool filter_group = g == rows_per_block, apart = blockDim.x > (unsigned)(rows_per_block * eighth);
+    if (chirp_z && (filter_group || !apart)) {
         // b_m = conj(w_m) for |m| < n, wrapped
-        __syncthreads();
 #pragma unroll
         for (int r = 0; r < 8; r++) {
             const int i = t + r * eighth, m = i < n ? i : M - i;
             const float2 w = bluestein_chirp(m, n, s);
             v[r] = m < n ? make_float2(w.x, -w.y) : make_float2(0.0f, 0.0f);
         }
+    }
+    if (chirp_z && !apart) {
+        __syncthreads();
         fft_row<false>(v, x, tw, M, log_m, t, -1.0f);
         if (g == 0)
 #pragma unroll
@@ -229,24 +242,31 @@ __global__ void __launch_bounds__(1024) k_fft_pass(const Program p, int rows, in
     __syncthreads();
     cudaGridDependencySynchronize();  // the passes before are complete
     const float inv_m = 1.0f / (float)M;
+    if (!filter_group) {
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
-        const int i = t + r * eighth;
-        v[r] = valid && i < n ? p.load(row, i) : make_float2(0.0f, 0.0f);
-        if (chirp_z && i < n) v[r] = cmul(v[r], bluestein_chirp(i, n, s));
+        for (int r = 0; r < 8; r++) {
+            const int i = t + r * eighth;
+            v[r] = valid && i < n ? p.load(row, i) : make_float2(0.0f, 0.0f);
+            if (chirp_z && i < n) v[r] = cmul(v[r], bluestein_chirp(i, n, s));
+        }
     }
     if (chirp_z)
         fft_row<false>(v, x, tw, M, log_m, t, -1.0f);
     else
         fft_row<true>(v, x, tw, M, log_m, t, s);
     if (chirp_z) {
+        if (apart && eighth <= 32) __syncthreads();  // (else fft_row ends with one)
+        if (!filter_group) {
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
-            const int i = padded(t + r * eighth);
-            v[r] = cmul<true>(x[i], filter[i]);
+            for (int r = 0; r < 8; r++) {
+                const int i = padded(t + r * eighth);
+                v[r] = cmul<true>(x[i], filter[i]);
+            }
         }
         if (eighth <= 32) __syncwarp();
-        fft_row<false>(v, x, tw, M, log_m, t, 1.0f);
+        // (the filter's threads take part in the barriers of the others' last transform, and overwrite the filter
+        // behind its first one)
+        if (!filter_group || eighth > 32) fft_row<false>(v, x, tw, M, log_m, t, 1.0f);
     }
     if (chirp_z) cudaTriggerProgrammaticLaunchCompletion();
     __syncthreads();  // every row of the block is transformed
