@@ -17,7 +17,7 @@
 // outside a record's integer bounds skips it (exact: with vertex and sample coordinates
 // below 2^14 the edge functions cannot wrap, and the quad test then never accepts a
 // sample outside the bounds; records beyond that range are tested at every pixel, in wrapping
-// int32).
+// int32, WildEdges).
 //
 // k_raster_masks is the literal per-pixel loop over the reference's bin masks, used for
 // parity checks of the binner and the rasteriser.
@@ -119,8 +119,8 @@ struct alignas(16) Rec {
     float ef[15];
     int flags;       // 1: bounds rejection and ef are exact; 2: adds nothing (collinear, or zero_record)
     float ext[4];    // edges 01 12 23 30: half the edge function's range over a block
-    // mixed vertex positions, sample space (x0, y0, ..., x3, y3): in ef's place while the record is
-    // built, and for good where ef is not exact (flags & 1 clear)
+    // in ef's place: the mixed vertex positions, sample space (x0, y0, ..., x3, y3), while the record is
+    // built, and, where ef is not exact (flags & 1 clear), A B C of the five edges as integers
     __device__ __forceinline__ int* q() { return reinterpret_cast<int*>(ef); }
     __device__ __forceinline__ const int* q() const { return reinterpret_cast<const int*>(ef); }
 };
@@ -190,6 +190,28 @@ __device__ __forceinline__ unsigned outside_sign(unsigned n01, unsigned n12, uns
     const unsigned x1 = (n01 | n12) ^ (n23 & n30), x0 = (n23 | n30) ^ (n01 & n12);
     return (~n20 & x1) | (n20 & x0);
 }
+
+// The integer edge functions of a record with flags & 1 clear, and whether the sample (px, py) is inside by them, in
+// wrapping int32. (Formed anew from the corners at every sample, they took half of the rasters at 8 samples, whose
+// coordinates often pass the exact range: 1920 x 1080, 24 surfaces, 60 paths, 139 -> 65 ms; 16 surfaces,
+// 40 paths, 4.79 -> 3.20 ms.)
+struct WildEdges {
+    int e[16];
+    __device__ __forceinline__ explicit WildEdges(const Rec& r) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int4 v = ld4i(r.q() + 4 * k);
+            e[4 * k] = v.x, e[4 * k + 1] = v.y, e[4 * k + 2] = v.z, e[4 * k + 3] = v.w;
+        }
+    }
+    __device__ __forceinline__ bool inside(int px, int py) const {
+        unsigned w[5];
+#pragma unroll
+        for (int i = 0; i < 5; i++)
+            w[i] = (unsigned)wadd(wadd(wmul(e[3 * i], py), wmul(e[3 * i + 1], px)), e[3 * i + 2]);
+        return (int)outside_sign(w[0], w[1], w[2], w[3], w[4]) >= 0;
+    }
+};
 
 // A record's edge functions in registers.
 struct Edges {
@@ -637,12 +659,23 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
     }
     *reinterpret_cast<float4*>(r.col) = col;
     float4* ef = reinterpret_cast<float4*>(r.ef);
-    if (safe) {  // else q stays
+    if (safe) {
         ef[0] = make_float4(ea[0], ea[1], eb[0], eb[1]);
         ef[1] = make_float4(ecl[0], ecl[1], ea[2], ea[3]);
         ef[2] = make_float4(eb[2], eb[3], ecl[2], ecl[3]);
+        ef[3] = make_float4(ea[4], eb[4], ecl[4], __int_as_float(flags));
+    } else {  // WildEdges
+        int e[16];
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            const int a = k < 4 ? k : 2, b = k < 4 ? (k + 1) & 3 : 0;
+            edge_coeffs(q[2 * a], q[2 * a + 1], q[2 * b], q[2 * b + 1], e + 3 * k);
+        }
+        e[15] = flags;
+        int4* wild = reinterpret_cast<int4*>(r.q());
+#pragma unroll
+        for (int k = 0; k < 4; k++) wild[k] = make_int4(e[4 * k], e[4 * k + 1], e[4 * k + 2], e[4 * k + 3]);
     }
-    ef[3] = make_float4(ea[4], eb[4], ecl[4], __int_as_float(flags));
     *reinterpret_cast<float4*>(r.ext) =
         make_float4(fabsf(ea[0]) * hy + fabsf(eb[0]) * hx, fabsf(ea[1]) * hy + fabsf(eb[1]) * hx,
                     fabsf(ea[2]) * hy + fabsf(eb[2]) * hx, fabsf(ea[3]) * hy + fabsf(eb[3]) * hx);
@@ -655,7 +688,8 @@ __device__ __forceinline__ int sample_hits(const Rec& r, int S, bool wild, float
                                            int lane) {
     int hits = 0;
     if (wild) {
-        for (int s = 0; s < S; s++) hits += inside_exact(r.q(), sx0 + s, sy0 + SUB_OFFSETS[S - 1 + s]) ? 1 : 0;
+        const WildEdges we(r);
+        for (int s = 0; s < S; s++) hits += we.inside(sx0 + s, sy0 + SUB_OFFSETS[S - 1 + s]) ? 1 : 0;
         return hits;
     }
     Edges e;
@@ -875,9 +909,10 @@ __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint
                         const int b = __clz(part);
                         const unsigned bit = 0x80000000u >> b;
                         part ^= bit;
+                        const WildEdges we(recs[m * 32 + b]);
 #pragma unroll
                         for (int i = 0; i < kPix; i++)
-                            if (inside_exact(recs[m * 32 + b].q(), sx0, sy0 + i)) c[i] |= bit;
+                            if (we.inside(sx0, sy0 + i)) c[i] |= bit;
                     }
 #pragma unroll
                     for (int i = 0; i < kPix; i++) cov[m][i] = px < p.width && py + i < p.height ? c[i] : 0;
