@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "rf_common.cuh"
@@ -739,7 +740,7 @@ constexpr size_t raster_smem_bytes(int maxW, int WS) {
 
 // Tile (tx, ty), whose entries are tile_entries[begin, end). smem4 holds the dynamic shared
 // memory (raster_smem_bytes), next_block four shared counters. kS: the anti-aliasing sample
-// count when known at compile time, else 0 (p.S). kTex: how the ghost texture is looked
+// count, or 0 for p.S (large ghost textures). kTex: how the ghost texture is looked
 // up (kLoads, kGather through p.ghost_tex, kAnyLoads).
 template <int T, int kS, int kTex, int kPix>
 __device__ __forceinline__ void raster_tile(const float4* __restrict__ vtx, uint32_t begin, uint32_t end,
@@ -1135,9 +1136,23 @@ __global__ void __launch_bounds__(kThreads, kS == 1 ? RF_RASTER_MIN_BLOCKS_S1 : 
         __syncthreads();
         if (item >= tiles) break;
         const int gt = s_gt, tile = s_tile;
-        raster_tile<T, kS, kTex, kPixels<T, kS>>(vtx_all + 2 * s_vtx, tile_offsets[gt], tile_offsets[gt + 1], tile_entries,
-                           ghosts + s_ghost, spectrum, sp, sfc, images + s_image, tile % sp.ntx, tile / sp.ntx, smem4,
-                           next_block);
+        // (the tile's code for the frame's sample count: with a count known at run time only, 12 frames of 1024 x
+        // 1024 take 18.5 instead of 16.4 ms at 2 samples, 19.7 / 17.3 at 4, 22.6 / 20.5 at 8)
+        auto shade = [&](auto samples) {
+            constexpr int kTile = decltype(samples)::value;
+            raster_tile<T, kTile, kTex, kPixels<T, kTile>>(vtx_all + 2 * s_vtx, tile_offsets[gt], tile_offsets[gt + 1],
+                                                           tile_entries, ghosts + s_ghost, spectrum, sp, sfc,
+                                                           images + s_image, tile % sp.ntx, tile / sp.ntx, smem4,
+                                                           next_block);
+        };
+        if (kS == 1 || sp.S == 1)
+            shade(std::integral_constant<int, 1>());
+        else if (sp.S == 2)
+            shade(std::integral_constant<int, 2>());
+        else if (sp.S == 4)
+            shade(std::integral_constant<int, 4>());
+        else
+            shade(std::integral_constant<int, 8>());
         __syncthreads();  // the tile's accumulators and `item` are free again
     }
 }
