@@ -599,11 +599,12 @@ __device__ __forceinline__ bool zero_record(const RasterParams& p, const Rec& r,
 // that is NaN (infinite at both wavelengths: an element of height 0) makes every fragment of the
 // general form 0, by its clamps.
 __device__ __forceinline__ bool inside_housing(const Rec& r) {
-    auto within = [](float4 v, float low) {  // (false with a NaN)
-        return v.x >= low && v.y >= low && v.z >= low && v.w >= low &&
-               fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)) <= 3.40282347e38f;
-    };
-    return within(ld4(r.rs), 1.0f) && within(ld4(r.inten), 0.0f) && within(ld4(r.refl), 0.0f);
+    // As unsigned bits non-negative finite floats come first, in order; then infinity, NaN, the negative ones.
+    auto bits = [](const float* p) { return *reinterpret_cast<const uint4*>(p); };
+    auto most = [](uint4 v) { return max(max(v.x, v.y), max(v.z, v.w)); };
+    const uint4 ramp = bits(r.rs);
+    return min(min(ramp.x, ramp.y), min(ramp.z, ramp.w)) >= 0x3f800000u /* 1 */ &&
+           max(most(ramp), max(most(bits(r.inten)), most(bits(r.refl)))) <= 0x7f7fffffu /* the largest float */;
 }
 
 // edges, bounds and flags of a record whose corners are stored; (ox, oy): the tile's first sample;
