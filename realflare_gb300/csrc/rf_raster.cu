@@ -121,7 +121,7 @@ struct alignas(16) Rec {
     int flags;       // 1: bounds rejection and ef are exact; 2: adds nothing (collinear, or zero_record)
     float ext[4];    // edges 01 12 23 30: half the edge function's range over a block
     // in ef's place: the mixed vertex positions, sample space (x0, y0, ..., x3, y3), while the record is
-    // built, and, where ef is not exact (flags & 1 clear), A B C of the five edges as integers
+    // built, and, where ef is not exact (flags & 1 clear), the same coefficients as integers
     __device__ __forceinline__ int* q() { return reinterpret_cast<int*>(ef); }
     __device__ __forceinline__ const int* q() const { return reinterpret_cast<const int*>(ef); }
 };
@@ -194,23 +194,16 @@ __device__ __forceinline__ unsigned outside_sign(unsigned n01, unsigned n12, uns
 
 // The integer edge functions of a record with flags & 1 clear, and whether the sample (px, py) is inside by them, in
 // wrapping int32. (Formed anew from the corners at every sample, they took half of the rasters at 8 samples, whose
-// coordinates often pass the exact range: 1920 x 1080, 24 surfaces, 60 paths, 139 -> 65 ms; 16 surfaces,
-// 40 paths, 4.79 -> 3.20 ms.)
+// coordinates often pass the exact range: 1920 x 1080, 24 surfaces, 60 paths, 136 -> 57 ms; 16 surfaces,
+// 40 paths, 4.71 -> 3.13 ms.)
 struct WildEdges {
-    int e[16];
-    __device__ __forceinline__ explicit WildEdges(const Rec& r) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int4 v = ld4i(r.q() + 4 * k);
-            e[4 * k] = v.x, e[4 * k + 1] = v.y, e[4 * k + 2] = v.z, e[4 * k + 3] = v.w;
-        }
-    }
+    int4 v0, v1, v2, v3;  // in ef's order: A of edges 01 12, B 01 12, C 01 12, A 23 30, ...
+    __device__ __forceinline__ explicit WildEdges(const Rec& r)
+        : v0(ld4i(r.q())), v1(ld4i(r.q() + 4)), v2(ld4i(r.q() + 8)), v3(ld4i(r.q() + 12)) {}
     __device__ __forceinline__ bool inside(int px, int py) const {
-        unsigned w[5];
-#pragma unroll
-        for (int i = 0; i < 5; i++)
-            w[i] = (unsigned)wadd(wadd(wmul(e[3 * i], py), wmul(e[3 * i + 1], px)), e[3 * i + 2]);
-        return (int)outside_sign(w[0], w[1], w[2], w[3], w[4]) >= 0;
+        auto value = [&](int a, int b, int c) { return (unsigned)wadd(wadd(wmul(a, py), wmul(b, px)), c); };
+        return (int)outside_sign(value(v0.x, v0.z, v1.x), value(v0.y, v0.w, v1.y), value(v1.z, v2.x, v2.z),
+                                 value(v1.w, v2.y, v2.w), value(v3.x, v3.y, v3.z)) >= 0;
     }
 };
 
@@ -626,6 +619,7 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
     const bool safe = p.safe_screen && bb.x >= -lim && bb.y <= lim && bb.z >= -lim && bb.w <= lim &&
                       (p.S < 8 || (bb.y - bb.x < 16384 && bb.w - bb.z < 16384));
     const float hx = 4.0f * (float)p.S - 0.5f, hy = 0.5f * kRows * (float)p.S - 0.5f;
+    // (beyond, the integer coefficients' bits, for samples relative to the image: WildEdges)
     float ea[5], eb[5], ecl[5];
 #pragma unroll
     for (int k = 0; k < 5; k++) {
@@ -633,9 +627,9 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
         int e[3];
         edge_coeffs(q[2 * a], q[2 * a + 1], q[2 * b], q[2 * b + 1], e);
         const int c = wadd(e[2], wadd(wmul(e[0], oy), wmul(e[1], ox)));
-        ea[k] = (float)e[0];
-        eb[k] = (float)e[1];
-        ecl[k] = (float)min(max(c, -8388608), 8388608);
+        ea[k] = safe ? (float)e[0] : __int_as_float(e[0]);
+        eb[k] = safe ? (float)e[1] : __int_as_float(e[1]);
+        ecl[k] = safe ? (float)min(max(c, -8388608), 8388608) : __int_as_float(e[2]);
     }
     int flags = safe ? 1 : 0;
     const bool collinear = edge_i(q[0], q[1], q[2], q[3], q[4], q[5]) == 0 &&
@@ -661,23 +655,11 @@ __device__ __forceinline__ void finish_record(const RasterParams& p, int w, int 
     }
     *reinterpret_cast<float4*>(r.col) = col;
     float4* ef = reinterpret_cast<float4*>(r.ef);
-    if (safe) {
-        ef[0] = make_float4(ea[0], ea[1], eb[0], eb[1]);
-        ef[1] = make_float4(ecl[0], ecl[1], ea[2], ea[3]);
-        ef[2] = make_float4(eb[2], eb[3], ecl[2], ecl[3]);
-        ef[3] = make_float4(ea[4], eb[4], ecl[4], __int_as_float(flags));
-    } else {  // WildEdges
-        int e[16];
-#pragma unroll
-        for (int k = 0; k < 5; k++) {
-            const int a = k < 4 ? k : 2, b = k < 4 ? (k + 1) & 3 : 0;
-            edge_coeffs(q[2 * a], q[2 * a + 1], q[2 * b], q[2 * b + 1], e + 3 * k);
-        }
-        e[15] = flags;
-        int4* wild = reinterpret_cast<int4*>(r.q());
-#pragma unroll
-        for (int k = 0; k < 4; k++) wild[k] = make_int4(e[4 * k], e[4 * k + 1], e[4 * k + 2], e[4 * k + 3]);
-    }
+    ef[0] = make_float4(ea[0], ea[1], eb[0], eb[1]);
+    ef[1] = make_float4(ecl[0], ecl[1], ea[2], ea[3]);
+    ef[2] = make_float4(eb[2], eb[3], ecl[2], ecl[3]);
+    ef[3] = make_float4(ea[4], eb[4], ecl[4], __int_as_float(flags));
+    // (half ranges over a block, of the exact form only)
     *reinterpret_cast<float4*>(r.ext) =
         make_float4(fabsf(ea[0]) * hy + fabsf(eb[0]) * hx, fabsf(ea[1]) * hy + fabsf(eb[1]) * hx,
                     fabsf(ea[2]) * hy + fabsf(eb[2]) * hx, fabsf(ea[3]) * hy + fabsf(eb[3]) * hx);
